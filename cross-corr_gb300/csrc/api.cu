@@ -223,7 +223,7 @@ xc_status cached_plan(xc_mode mode, xc_dtype dtype, xc_size2 left, uint32_t n_le
     return XC_OK;
   }
   FftPlanImpl* p = nullptr;
-  XC_TRY(fft_plan_create(&p, mode, dtype, left, n_left, right, n_right, xc_size2{0, 0}));
+  XC_TRY(fft_plan_create(&p, mode, dtype, left, n_left, right, n_right, xc_size2{0, 0}, false));
   c.plans.emplace(key, std::unique_ptr<FftPlanImpl, PlanDeleter>(p));
   *plan = p;
   return XC_OK;
@@ -775,7 +775,7 @@ xc_status xc_fft_plan_create(xc_fft_plan* plan, xc_mode mode, xc_dtype dtype, xc
   *plan = nullptr;
   XC_TRY(check_sizes(left, right));
   FftPlanImpl* impl = nullptr;
-  XC_TRY(fft_plan_create(&impl, mode, dtype, left, n_left, right, n_right, pad));
+  XC_TRY(fft_plan_create(&impl, mode, dtype, left, n_left, right, n_right, pad, true));
   *plan = new xc_fft_plan_s{impl};
   return XC_OK;
 }

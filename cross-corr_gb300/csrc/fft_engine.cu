@@ -1,0 +1,305 @@
+// fft_engine.cu -- planning and launches of the fused FFT correlation
+// (kernels in fft_engine.cuh).
+//
+// A problem runs as three kernels per chunk of outputs: row transforms of the
+// inputs, column transforms + product + inverse columns, inverse rows.  The
+// zero padding, the conjugate product, the quadrant swap, the scale and the
+// crop of the separate-kernel path (fft_pipeline.cu's stages) happen inside
+// them, rows of zeros are never transformed or stored, and the intermediate
+// spectra cross memory twice instead of eight times.
+#include "fft_engine.h"
+
+#include <algorithm>
+#include <cmath>
+#include <vector>
+
+namespace xc {
+namespace fe {
+
+namespace {
+
+struct Factors {
+  int n, r1, r2, r3;
+};
+#define XC_FACTORS(N_, A_, B_, C_) {N_, A_, B_, C_},
+constexpr Factors kLengths[] = {XC_FFT_LENGTHS(XC_FACTORS)};
+#undef XC_FACTORS
+
+const Factors* factors(int n) {
+  for (const Factors& f : kLengths)
+    if (f.n == n) return &f;
+  return nullptr;
+}
+
+// exp(-2 pi i k / n): the angle is reduced to the first octant, where sine
+// and cosine are accurate to the last place.
+void root(long long k, long long n, double* re, double* im) {
+  k %= n;
+  const double pi = 3.14159265358979323846264338327950288;
+  const long long e = 8 * k;  // in octants of n
+  const int oct = (int)(e / n);
+  double c, s;
+  const auto angle = [&](long long num) { return 2.0 * pi * ((double)num / (double)n); };  // num / n of a turn
+  switch (oct) {
+    case 0: c = std::cos(angle(k)); s = std::sin(angle(k)); break;
+    case 1: c = std::sin(angle(n - 4 * k) / 4); s = std::cos(angle(n - 4 * k) / 4); break;
+    case 2: c = -std::sin(angle(4 * k - n) / 4); s = std::cos(angle(4 * k - n) / 4); break;
+    case 3: c = -std::cos(angle(n - 2 * k) / 2); s = std::sin(angle(n - 2 * k) / 2); break;
+    case 4: c = -std::cos(angle(2 * k - n) / 2); s = -std::sin(angle(2 * k - n) / 2); break;
+    case 5: c = -std::sin(angle(3 * n - 4 * k) / 4); s = -std::cos(angle(3 * n - 4 * k) / 4); break;
+    case 6: c = std::sin(angle(4 * k - 3 * n) / 4); s = -std::cos(angle(4 * k - 3 * n) / 4); break;
+    default: c = std::cos(angle(n - k)); s = -std::sin(angle(n - k)); break;
+  }
+  *re = c;
+  *im = -s;
+}
+
+template <typename T>
+void fill(int n, T* out) {
+  const Factors* f = factors(n);
+  const int s1 = n / f->r1;
+  size_t at = 0;
+  auto put = [&](long long k, long long m) {
+    double re, im;
+    root(k, m, &re, &im);
+    out[2 * at] = (T)re;
+    out[2 * at + 1] = (T)im;
+    ++at;
+  };
+  for (int q = 1; q < f->r1; ++q)
+    for (int o = 0; o < s1; ++o) put((long long)o * q, n);
+  if (f->r2 > 1)
+    for (int q = 1; q < f->r2; ++q)
+      for (int o = 0; o < f->r3; ++o) put((long long)o * q, s1);
+}
+
+size_t align256(size_t x) { return (x + 255) & ~size_t(255); }
+
+xc_status raise_limit(const void* fn, int bytes) {
+  if (bytes > 48 * 1024) XC_CUDA_TRY(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes));
+  return XC_OK;
+}
+
+template <typename Args>
+xc_status launch(const void* fn, long long blocks, int threads, int smem, Args& args, cudaStream_t stream) {
+  if (blocks > 0x7fffffffLL) return fail(XC_ERR_INVALID_ARGUMENT, "problem too large for one launch");
+  void* a[] = {&args};
+  XC_CUDA_TRY(cudaLaunchKernel(fn, dim3((unsigned)blocks), dim3((unsigned)threads), a, (size_t)smem, stream));
+  return XC_OK;
+}
+
+template <typename T>
+xc_status run(const Engine& e, const void* left, const void* right, void* out, char* ws, cudaStream_t stream) {
+  using C = Cx<T>;
+  const Geometry& g = e.g;
+  const C* twx = reinterpret_cast<const C*>(e.tw);
+  const C* twy = reinterpret_cast<const C*>(static_cast<const char*>(e.tw) + e.tw_col);
+  C* al = reinterpret_cast<C*>(ws + e.off_al);
+  C* ar = reinterpret_cast<C*>(ws + e.off_ar);
+  C* fl = reinterpret_cast<C*>(ws + e.off_fl);
+  C* fr = reinterpret_cast<C*>(ws + e.off_fr);
+  C* b = reinterpret_cast<C*>(ws + e.off_b);
+  const int lgcb = e.ck.lgcb, nblk = e.nblk;
+  const int q = e.rk.q;
+
+  // rows of `nr` rights from the r0-th on, and (first) of all lefts
+  const auto rows = [&](bool lefts, long long r0, long long nr) {
+    RowFwdArgs<T> a{};
+    a.a = RowSide<T>{static_cast<const T*>(left), al, g.Hl, g.Wl, div_up(div_up(g.Hl, 2), q)};
+    a.b = RowSide<T>{static_cast<const T*>(right) + r0 * g.Hr * g.Wr, ar, g.Hr, g.Wr, div_up(div_up(g.Hr, 2), q)};
+    a.a_blocks = lefts ? (unsigned)(e.pm.n_left * a.a.groups) : 0u;
+    a.nblk = nblk;
+    a.lgcb = lgcb;
+    a.tw = twx;
+    return launch(e.rk.forward, a.a_blocks + nr * a.b.groups, e.rk.threads, e.rk.smem, a, stream);
+  };
+  const auto columns = [&](const C* src, C* dst, int H, long long mats) {
+    ColFwdArgs<T> a{src, dst, H, nblk, mats * nblk, twy};
+    return launch(e.ck.forward, div_up(a.units, e.ck.pu), e.ck.threads, e.ck.unit_smem, a, stream);
+  };
+
+  if (e.shared) XC_TRY(rows(true, 0, e.n_right));
+  if (e.shared) {
+    XC_TRY(columns(al, fl, g.Hl, e.pm.n_left));
+    XC_TRY(columns(ar, fr, g.Hr, e.n_right));
+  }
+  const double scale = 1.0 / ((double)e.nx * (double)e.ny);
+  for (int k0 = 0; k0 < e.pm.K; k0 += e.k_chunk) {
+    const int k1 = std::min(e.pm.K, k0 + e.k_chunk), nk = k1 - k0;
+    if (!e.shared) {
+      XC_TRY(rows(k0 == 0, k0 * e.pm.r_k, nk * e.pm.r_k));
+      if (e.lpre && k0 == 0) XC_TRY(columns(al, fl, g.Hl, e.pm.n_left));
+    }
+    for (int l0 = 0; l0 < e.pm.n_left; l0 += e.l_chunk) {
+      const int nl = std::min(e.pm.n_left - l0, e.l_chunk);
+      {
+        ColArgs<T> a{};
+        a.left = e.shared || e.lpre ? fl : al;
+        a.right = e.shared ? fr : ar;
+        a.out = b;
+        a.Hl = g.Hl;
+        a.Hr = g.Hr;
+        a.Sy = g.Sy;
+        a.nblk = nblk;
+        a.n_left = nl;
+        a.l0 = l0;
+        a.k0 = k0;
+        a.k1 = k1;
+        a.kc = std::min(e.kc, nk);
+        a.n_kg = div_up(nk, a.kc);
+        a.r_l = e.pm.r_l;
+        a.r_k = e.pm.r_k;
+        a.r_off = e.shared ? 0 : k0 * e.pm.r_k;
+        a.tw = twy;
+        const void* fn = e.shared ? e.ck.pairs_pre : e.lpre ? e.ck.pairs_lpre : e.ck.pairs;
+        XC_TRY(launch(fn, div_up((long long)nl * a.n_kg * nblk, e.ck.pu), e.ck.threads,
+                      e.ck.unit_smem * (e.shared || e.lpre ? 1 : 2), a, stream));
+      }
+      {
+        RowInvArgs<T> a{};
+        a.src = b;
+        a.out = static_cast<T*>(out);
+        a.Sy = g.Sy;
+        a.Sx = g.Sx;
+        a.Wr = g.Wr;
+        a.groups = div_up(div_up(g.Sy, 2), q);
+        a.nblk = nblk;
+        a.lgcb = lgcb;
+        a.l0 = l0;
+        a.k0 = k0;
+        a.nk = nk;
+        a.o_l = e.pm.o_l;
+        a.o_k = e.pm.o_k;
+        a.scale_hi = (T)scale;
+        a.scale_lo = (T)(scale - (double)a.scale_hi);
+        a.tw = twx;
+        XC_TRY(launch(e.rk.inverse, (long long)nl * nk * a.groups, e.rk.threads, e.rk.smem, a, stream));
+      }
+    }
+  }
+  return XC_OK;
+}
+
+}  // namespace
+
+int length_for(int n) {
+  for (const Factors& f : kLengths)
+    if (f.n >= n) return f.n;
+  return 0;
+}
+
+size_t twiddle_count(int n) {
+  const Factors* f = factors(n);
+  return (size_t)(f->r1 - 1) * (n / f->r1) + (f->r2 > 1 ? (size_t)(f->r2 - 1) * f->r3 : 0);
+}
+void fill_twiddles_f32(int n, float* out) { fill(n, out); }
+void fill_twiddles_f64(int n, double* out) { fill(n, out); }
+
+xc_status engine_plan(Engine* e, xc_dtype dtype, const Geometry& g, const PairMap& pm, long long n_right,
+                      size_t ws_bytes) {
+  e->ready = false;
+  e->dtype = dtype;
+  e->g = g;
+  e->pm = pm;
+  e->n_right = n_right;
+  e->nx = length_for(g.Sx);
+  e->ny = length_for(g.Sy);
+  if (e->nx == 0 || e->ny == 0) return XC_OK;
+  const bool f32 = dtype == XC_F32;
+  if (!(f32 ? row_kernels_f32(e->nx, &e->rk) : row_kernels_f64(e->nx, &e->rk)) ||
+      !(f32 ? col_kernels_f32(e->ny, &e->ck) : col_kernels_f64(e->ny, &e->ck)))
+    return XC_OK;
+  const size_t ce = f32 ? sizeof(float2) : sizeof(double2);
+  const int cb = 1 << e->ck.lgcb;
+  e->nblk = div_up(e->nx / 2 + 1, cb);
+  const size_t row = (size_t)e->nblk * cb * ce;  // bytes of one spectrum row
+  e->shared = pm.r_l == 0 && pm.n_left > 1;
+  // a left spectrum beside the partner's block in shared memory, while two
+  // CTAs still fit an SM
+  e->lpre = !e->shared && 2 * e->ck.unit_smem > 100 * 1024;
+
+  // Workspace: row spectra of the lefts and of a chunk of rights, full
+  // spectra of shared matrices, column-inverted products of a chunk.  Chunks
+  // keep what one kernel writes and the next one reads within the L2 cache.
+  const size_t budget = (size_t)64 << 20;
+  const size_t ar1 = row * g.Hr, b1 = row * g.Sy;
+  size_t off = 0;
+  const auto take = [&](size_t bytes) {
+    const size_t at = off;
+    off += align256(bytes);
+    return at;
+  };
+  if (e->shared || e->lpre) e->off_fl = take(row * e->ny * pm.n_left);
+  if (e->shared) {
+    e->off_fr = take(row * e->ny * n_right);
+    const size_t at = off;
+    e->off_al = take(row * g.Hl * pm.n_left);
+    e->off_ar = take(ar1 * n_right);
+    const size_t a_end = off;
+    e->off_b = at;  // products replace the row spectra, which are done with by then
+    off = at;
+    if (at + b1 > ws_bytes) return XC_OK;
+    const long long fit = std::max<long long>(1, std::min<long long>((long long)(budget / b1), (long long)((ws_bytes - at) / b1)));
+    e->l_chunk = (int)std::min<long long>(pm.n_left, std::max<long long>(1, fit / pm.K));
+    e->k_chunk = (int)std::min<long long>(pm.K, std::max<long long>(1, fit / e->l_chunk));
+    if ((long long)e->l_chunk * e->k_chunk > fit) e->l_chunk = 1;
+    off = std::max(a_end, at + align256(b1 * e->l_chunk * e->k_chunk));
+    e->kc = 1;
+  } else {
+    e->off_al = take(row * g.Hl * pm.n_left);
+    e->l_chunk = pm.n_left;
+    const size_t per_k = (ar1 + b1) * pm.n_left;  // r_k = n_left rights (one for a single left)
+    if (off + per_k + 512 > ws_bytes) return XC_OK;
+    const long long fit = std::max<long long>(1, std::min<long long>((long long)(budget / per_k),
+                                                                    (long long)((ws_bytes - off - 512) / per_k)));
+    e->k_chunk = (int)std::min<long long>(pm.K, fit);
+    e->off_ar = take(ar1 * pm.n_left * e->k_chunk);
+    e->off_b = take(b1 * pm.n_left * e->k_chunk);
+    // partners per CTA: as many as leave eight CTAs per SM
+    const long long units = div_up((long long)pm.n_left * e->nblk, e->ck.pu);
+    e->kc = 1;
+    while (!e->lpre && e->kc < 8 && 2 * e->kc <= e->k_chunk && units * div_up(e->k_chunk, 2 * e->kc) >= 152 * 8)
+      e->kc *= 2;
+  }
+  e->bytes = off;
+  if (e->bytes > ws_bytes) return XC_OK;
+
+  XC_TRY(raise_limit(e->rk.forward, e->rk.smem));
+  XC_TRY(raise_limit(e->rk.inverse, e->rk.smem));
+  XC_TRY(raise_limit(e->ck.forward, e->ck.unit_smem));
+  XC_TRY(raise_limit(e->ck.pairs_lpre, e->ck.unit_smem));
+  XC_TRY(raise_limit(e->ck.pairs_pre, e->ck.unit_smem));
+  if (2 * e->ck.unit_smem <= 227 * 1024) XC_TRY(raise_limit(e->ck.pairs, 2 * e->ck.unit_smem));
+  const size_t cx = twiddle_count(e->nx), cy = twiddle_count(e->ny);
+  std::vector<char> host((cx + cy) * ce);
+  if (f32) {
+    fill_twiddles_f32(e->nx, reinterpret_cast<float*>(host.data()));
+    fill_twiddles_f32(e->ny, reinterpret_cast<float*>(host.data() + cx * ce));
+  } else {
+    fill_twiddles_f64(e->nx, reinterpret_cast<double*>(host.data()));
+    fill_twiddles_f64(e->ny, reinterpret_cast<double*>(host.data() + cx * ce));
+  }
+  XC_CUDA_TRY(cudaMalloc(&e->tw, host.size()));
+  e->tw_col = cx * ce;
+  const cudaError_t err = cudaMemcpy(e->tw, host.data(), host.size(), cudaMemcpyHostToDevice);
+  if (err != cudaSuccess) {
+    engine_release(e);
+    return from_cuda(err, "upload of the twiddle tables");
+  }
+  e->ready = true;
+  return XC_OK;
+}
+
+xc_status engine_run(const Engine& e, const void* left, const void* right, void* out, char* ws, cudaStream_t stream) {
+  return e.dtype == XC_F32 ? run<float>(e, left, right, out, ws, stream)
+                           : run<double>(e, left, right, out, ws, stream);
+}
+
+void engine_release(Engine* e) {
+  cudaFree(e->tw);
+  e->tw = nullptr;
+  e->ready = false;
+}
+
+}  // namespace fe
+}  // namespace xc

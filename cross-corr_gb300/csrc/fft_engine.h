@@ -1,0 +1,51 @@
+// fft_engine.h -- host side of the fused FFT correlation (fft_engine.cu):
+// what a plan keeps, and how it is made and run.
+#pragma once
+
+#include <cuda_runtime.h>
+
+#include <cstddef>
+#include <cstdint>
+
+#include "fft_engine.cuh"
+#include "xc_internal.h"
+
+namespace xc {
+namespace fe {
+
+// One uniform problem: transform lengths, kernels, twiddle tables and the
+// workspace layout (byte offsets).
+struct Engine {
+  bool ready = false;
+  xc_dtype dtype = XC_F32;
+  Geometry g{};
+  PairMap pm{};
+  long long n_right = 0;
+  int nx = 0, ny = 0, nblk = 0;
+  RowKernels rk{};
+  ColKernels ck{};
+  void* tw = nullptr;      // device: row table, then column table
+  size_t tw_col = 0;       // byte offset of the column table
+  bool shared = false;     // every right serves several lefts: all spectra are made first
+  bool lpre = false;       // left spectra are made first
+  int l_chunk = 1, k_chunk = 1, kc = 1;
+  size_t off_al = 0, off_ar = 0, off_fl = 0, off_fr = 0, off_b = 0, bytes = 0;
+};
+
+// Smallest length >= n that the kernels have; 0 when n is beyond the largest.
+int length_for(int n);
+// Twiddle table of a length (entries of two reals; host memory).
+size_t twiddle_count(int n);
+void fill_twiddles_f32(int n, float* out);
+void fill_twiddles_f64(int n, double* out);
+
+// Plans a problem within `ws_bytes` of workspace.  *e stays not ready (and
+// XC_OK is returned) when the sizes are beyond the kernels' lengths or the
+// workspace is too small; an error only when the device calls fail.
+xc_status engine_plan(Engine* e, xc_dtype dtype, const Geometry& g, const PairMap& pm, long long n_right,
+                      size_t ws_bytes);
+xc_status engine_run(const Engine& e, const void* left, const void* right, void* out, char* ws, cudaStream_t stream);
+void engine_release(Engine* e);
+
+}  // namespace fe
+}  // namespace xc

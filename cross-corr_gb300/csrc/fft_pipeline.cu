@@ -19,6 +19,7 @@
 #include <new>
 #include <string>
 
+#include "fft_engine.h"
 #include "xc_common.cuh"
 #include "xc_internal.h"
 
@@ -37,6 +38,7 @@ struct FftPlanImpl {
   cufftHandle r2c = 0, c2r = 0;
   bool have_r2c = false, have_c2r = false;
   size_t ws_inputs, ws_products;  // bytes
+  fe::Engine engine;  // the fused kernels, where they take the problem (normalised results)
 };
 
 namespace {
@@ -59,7 +61,7 @@ int next_smooth(long long n) {
 }  // namespace
 
 xc_status fft_plan_create(FftPlanImpl** out, xc_mode mode, xc_dtype dtype, xc_size2 left, uint32_t n_left,
-                          xc_size2 right, uint32_t n_right, xc_size2 pad) {
+                          xc_size2 right, uint32_t n_right, xc_size2 pad, bool stages) {
   *out = nullptr;
   FftPlanImpl* p = new (std::nothrow) FftPlanImpl();
   if (p == nullptr) return fail(XC_ERR_CUDA, "host allocation failed");
@@ -95,6 +97,16 @@ xc_status fft_plan_create(FftPlanImpl** out, xc_mode mode, xc_dtype dtype, xc_si
   p->ws_inputs = (size_t)(n_left + n_right) * (size_t)p->bins * ce;
   p->ws_products = (size_t)p->n_out * (size_t)p->bins * ce;
 
+  const xc_status es = fe::engine_plan(&p->engine, dtype, p->g, p->pm, (long long)n_right, p->ws_inputs + p->ws_products);
+  if (es != XC_OK) {
+    delete p;
+    return es;
+  }
+  if (p->engine.ready && !stages) {  // the library transforms would not be used
+    *out = p;
+    return XC_OK;
+  }
+
   int n[2] = {p->py, p->px};
   int rembed[2] = {p->py, 2 * p->cols_c};
   int cembed[2] = {p->py, p->cols_c};
@@ -102,6 +114,7 @@ xc_status fft_plan_create(FftPlanImpl** out, xc_mode mode, xc_dtype dtype, xc_si
   cufftResult r = cufftPlanMany(&p->r2c, 2, n, rembed, 1, rdist, cembed, 1, cdist,
                                 dtype == XC_F32 ? CUFFT_R2C : CUFFT_D2Z, (int)(n_left + n_right));
   if (r != CUFFT_SUCCESS) {
+    fe::engine_release(&p->engine);
     delete p;
     return cufft_fail(r, "cufftPlanMany(R2C)");
   }
@@ -110,6 +123,7 @@ xc_status fft_plan_create(FftPlanImpl** out, xc_mode mode, xc_dtype dtype, xc_si
                     (int)p->n_out);
   if (r != CUFFT_SUCCESS) {
     cufftDestroy(p->r2c);
+    fe::engine_release(&p->engine);
     delete p;
     return cufft_fail(r, "cufftPlanMany(C2R)");
   }
@@ -187,6 +201,11 @@ xc_status fft_plan_inverse(FftPlanImpl* p, void* out, int normalize, void* works
 
 xc_status fft_plan_execute(FftPlanImpl* p, const void* left, const void* right, void* out, int normalize,
                            void* workspace, size_t ws_bytes, cudaStream_t stream) {
+  if (normalize && p->engine.ready) {
+    WsView v;
+    XC_TRY(ws_view(p, workspace, ws_bytes, &v));
+    return fe::engine_run(p->engine, left, right, out, v.inputs, stream);
+  }
   XC_TRY(fft_plan_forward(p, left, right, workspace, ws_bytes, stream));
   XC_TRY(fft_plan_multiply(p, workspace, ws_bytes, stream));
   return fft_plan_inverse(p, out, normalize, workspace, ws_bytes, stream);
@@ -196,6 +215,7 @@ void fft_plan_destroy(FftPlanImpl* p) {
   if (p == nullptr) return;
   if (p->have_r2c) cufftDestroy(p->r2c);
   if (p->have_c2r) cufftDestroy(p->c2r);
+  fe::engine_release(&p->engine);
   delete p;
 }
 

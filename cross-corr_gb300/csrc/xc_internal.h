@@ -113,8 +113,10 @@ xc_status mlp_adam(float* params, const float* grad, float* m, float* v, uint32_
 
 // FFT pipeline (fft_pipeline.cu).
 struct FftPlanImpl;
+// `stages`: the plan will run stage by stage or unnormalised too, which needs
+// the library transforms beside the fused kernels.
 xc_status fft_plan_create(FftPlanImpl** plan, xc_mode mode, xc_dtype dtype, xc_size2 left, uint32_t n_left,
-                          xc_size2 right, uint32_t n_right, xc_size2 pad);
+                          xc_size2 right, uint32_t n_right, xc_size2 pad, bool stages);
 size_t fft_plan_workspace(const FftPlanImpl* plan);
 xc_size2 fft_plan_pad(const FftPlanImpl* plan);
 xc_status fft_plan_execute(FftPlanImpl* plan, const void* left, const void* right, void* out, int normalize,
