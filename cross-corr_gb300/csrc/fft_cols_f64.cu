@@ -5,10 +5,10 @@
 namespace xc {
 namespace fe {
 
-#define XC_FFT_T double
+#define XC_FFT_S double
 bool col_kernels_f64(int n, ColKernels* k) {
   switch (n) {
-    XC_FFT_LENGTHS(XC_COL_CASE)
+    XC_FFT_COLS(XC_COL_CASE)
     default: return false;
   }
 }

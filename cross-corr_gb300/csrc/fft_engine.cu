@@ -19,15 +19,20 @@ namespace fe {
 namespace {
 
 struct Factors {
-  int n, r1, r2, r3;
+  int n, r1, ra, rb, r3;
 };
-#define XC_FACTORS(N_, A_, B_, C_) {N_, A_, B_, C_},
-constexpr Factors kLengths[] = {XC_FFT_LENGTHS(XC_FACTORS)};
+#define XC_FACTORS(N_, A_, B_, C_, D_) {N_, A_, B_, C_, D_},
+constexpr Factors kRows[] = {XC_FFT_ROWS(XC_FACTORS)};
 #undef XC_FACTORS
+#define XC_FACTORS(N_, A_, B_, D_) {N_, A_, B_, 1, D_},
+constexpr Factors kCols[] = {XC_FFT_COLS(XC_FACTORS)};
+#undef XC_FACTORS
+constexpr int kLengths = (int)(sizeof(kRows) / sizeof(kRows[0]));
+static_assert(sizeof(kRows) == sizeof(kCols), "the same lengths on both axes");
 
-const Factors* factors(int n) {
-  for (const Factors& f : kLengths)
-    if (f.n == n) return &f;
+const Factors* factors(int n, bool rows) {
+  for (int i = 0; i < kLengths; ++i)
+    if (kRows[i].n == n) return rows ? &kRows[i] : &kCols[i];
   return nullptr;
 }
 
@@ -54,23 +59,16 @@ void root(long long k, long long n, double* re, double* im) {
   *im = -s;
 }
 
-template <typename T>
-void fill(int n, T* out) {
-  const Factors* f = factors(n);
-  const int s1 = n / f->r1;
-  size_t at = 0;
-  auto put = [&](long long k, long long m) {
-    double re, im;
-    root(k, m, &re, &im);
-    out[2 * at] = (T)re;
-    out[2 * at + 1] = (T)im;
-    ++at;
-  };
-  for (int q = 1; q < f->r1; ++q)
-    for (int o = 0; o < s1; ++o) put((long long)o * q, n);
-  if (f->r2 > 1)
-    for (int q = 1; q < f->r2; ++q)
-      for (int o = 0; o < f->r3; ++o) put((long long)o * q, s1);
+// The table of a pass structure: [q - 1][o] of every pass but the last.
+template <typename Put>
+void each_twiddle(const Factors& f, Put put) {
+  const int s1 = f.n / f.r1, sa = s1 / f.ra;
+  for (int q = 1; q < f.r1; ++q)
+    for (int o = 0; o < s1; ++o) put((long long)o * q, f.n);
+  for (int q = 1; q < f.ra; ++q)
+    for (int o = 0; o < sa; ++o) put((long long)o * q, s1);
+  for (int q = 1; q < f.rb; ++q)
+    for (int o = 0; o < f.r3; ++o) put((long long)o * q, sa);
 }
 
 size_t align256(size_t x) { return (x + 255) & ~size_t(255); }
@@ -84,37 +82,54 @@ template <typename Args>
 xc_status launch(const void* fn, long long blocks, int threads, int smem, Args& args, cudaStream_t stream) {
   if (blocks > 0x7fffffffLL) return fail(XC_ERR_INVALID_ARGUMENT, "problem too large for one launch");
   void* a[] = {&args};
-  XC_CUDA_TRY(cudaLaunchKernel(fn, dim3((unsigned)blocks), dim3((unsigned)threads), a, (size_t)smem, stream));
+  // Programmatic dependent launch: the next kernel's CTAs may become resident
+  // while this one's last ones run; each waits for the whole previous grid
+  // (griddepcontrol.wait) before it touches memory.
+  cudaLaunchAttribute attr{};
+  attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr.val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3((unsigned)blocks);
+  cfg.blockDim = dim3((unsigned)threads);
+  cfg.dynamicSmemBytes = (size_t)smem;
+  cfg.stream = stream;
+  cfg.attrs = &attr;
+  cfg.numAttrs = 1;
+  XC_CUDA_TRY(cudaLaunchKernelExC(&cfg, fn, a));
   return XC_OK;
 }
 
 template <typename T>
 xc_status run(const Engine& e, const void* left, const void* right, void* out, char* ws, cudaStream_t stream) {
-  using C = Cx<T>;
   const Geometry& g = e.g;
-  const C* twx = reinterpret_cast<const C*>(e.tw);
-  const C* twy = reinterpret_cast<const C*>(static_cast<const char*>(e.tw) + e.tw_col);
-  C* al = reinterpret_cast<C*>(ws + e.off_al);
-  C* ar = reinterpret_cast<C*>(ws + e.off_ar);
-  C* fl = reinterpret_cast<C*>(ws + e.off_fl);
-  C* fr = reinterpret_cast<C*>(ws + e.off_fr);
-  C* b = reinterpret_cast<C*>(ws + e.off_b);
+  const char* tw = static_cast<const char*>(e.tw);
+  Cx<T>* al = reinterpret_cast<Cx<T>*>(ws + e.off_al);
+  Cx<T>* ar = reinterpret_cast<Cx<T>*>(ws + e.off_ar);
+  char* fl = ws + e.off_fl;
+  char* fr = ws + e.off_fr;
+  Cx<T>* b = reinterpret_cast<Cx<T>*>(ws + e.off_b);
   const int lgcb = e.ck.lgcb, nblk = e.nblk;
-  const int q = e.rk.q;
+  const int rows_per_cta = 2 * e.rk.nv * e.rk.q;
+  const double scale = 1.0 / ((double)e.nx * (double)e.ny);
 
-  // rows of `nr` rights from the r0-th on, and (first) of all lefts
+  // rows of `nr` rights from the r0-th on, and (first) of all lefts.  FP64
+  // applies the result's scale here, in a product that is there anyway.
   const auto rows = [&](bool lefts, long long r0, long long nr) {
     RowFwdArgs<T> a{};
-    a.a = RowSide<T>{static_cast<const T*>(left), al, g.Hl, g.Wl, div_up(div_up(g.Hl, 2), q)};
-    a.b = RowSide<T>{static_cast<const T*>(right) + r0 * g.Hr * g.Wr, ar, g.Hr, g.Wr, div_up(div_up(g.Hr, 2), q)};
-    a.a_blocks = lefts ? (unsigned)(e.pm.n_left * a.a.groups) : 0u;
+    a.a = RowSide<T>{static_cast<const T*>(left), al, g.Hl, g.Wl, div_up(g.Hl, rows_per_cta), T(1)};
+    a.b = RowSide<T>{static_cast<const T*>(right) + r0 * g.Hr * g.Wr, ar, g.Hr, g.Wr, div_up(g.Hr, rows_per_cta),
+                     (T)scale};
+    const long long ab = lefts ? (long long)e.pm.n_left * a.a.groups : 0;
+    if (ab + nr * a.b.groups > 0x7fffffffLL) return fail(XC_ERR_INVALID_ARGUMENT, "problem too large for one launch");
+    a.a_blocks = (unsigned)ab;
     a.nblk = nblk;
     a.lgcb = lgcb;
-    a.tw = twx;
-    return launch(e.rk.forward, a.a_blocks + nr * a.b.groups, e.rk.threads, e.rk.smem, a, stream);
+    a.tw = tw;
+    a.zeros = reinterpret_cast<const T*>(tw + e.zeros);
+    return launch(e.rk.forward, ab + nr * a.b.groups, e.rk.threads, e.rk.smem, a, stream);
   };
-  const auto columns = [&](const C* src, C* dst, int H, long long mats) {
-    ColFwdArgs<T> a{src, dst, H, nblk, mats * nblk, twy};
+  const auto columns = [&](const Cx<T>* src, void* dst, int H, long long mats) {
+    ColFwdArgs<T> a{src, dst, H, nblk, mats * nblk, tw + e.tw_col};
     return launch(e.ck.forward, div_up(a.units, e.ck.pu), e.ck.threads, e.ck.unit_smem, a, stream);
   };
 
@@ -123,7 +138,6 @@ xc_status run(const Engine& e, const void* left, const void* right, void* out, c
     XC_TRY(columns(al, fl, g.Hl, e.pm.n_left));
     XC_TRY(columns(ar, fr, g.Hr, e.n_right));
   }
-  const double scale = 1.0 / ((double)e.nx * (double)e.ny);
   for (int k0 = 0; k0 < e.pm.K; k0 += e.k_chunk) {
     const int k1 = std::min(e.pm.K, k0 + e.k_chunk), nk = k1 - k0;
     if (!e.shared) {
@@ -134,8 +148,8 @@ xc_status run(const Engine& e, const void* left, const void* right, void* out, c
       const int nl = std::min(e.pm.n_left - l0, e.l_chunk);
       {
         ColArgs<T> a{};
-        a.left = e.shared || e.lpre ? fl : al;
-        a.right = e.shared ? fr : ar;
+        a.left = e.shared || e.lpre ? static_cast<void*>(fl) : al;
+        a.right = e.shared ? static_cast<void*>(fr) : ar;
         a.out = b;
         a.Hl = g.Hl;
         a.Hr = g.Hr;
@@ -150,7 +164,7 @@ xc_status run(const Engine& e, const void* left, const void* right, void* out, c
         a.r_l = e.pm.r_l;
         a.r_k = e.pm.r_k;
         a.r_off = e.shared ? 0 : k0 * e.pm.r_k;
-        a.tw = twy;
+        a.tw = tw + e.tw_col;
         const void* fn = e.shared ? e.ck.pairs_pre : e.lpre ? e.ck.pairs_lpre : e.ck.pairs;
         XC_TRY(launch(fn, div_up((long long)nl * a.n_kg * nblk, e.ck.pu), e.ck.threads,
                       e.ck.unit_smem * (e.shared || e.lpre ? 1 : 2), a, stream));
@@ -162,7 +176,7 @@ xc_status run(const Engine& e, const void* left, const void* right, void* out, c
         a.Sy = g.Sy;
         a.Sx = g.Sx;
         a.Wr = g.Wr;
-        a.groups = div_up(div_up(g.Sy, 2), q);
+        a.groups = div_up(g.Sy, rows_per_cta);
         a.nblk = nblk;
         a.lgcb = lgcb;
         a.l0 = l0;
@@ -172,7 +186,7 @@ xc_status run(const Engine& e, const void* left, const void* right, void* out, c
         a.o_k = e.pm.o_k;
         a.scale_hi = (T)scale;
         a.scale_lo = (T)(scale - (double)a.scale_hi);
-        a.tw = twx;
+        a.tw = tw;
         XC_TRY(launch(e.rk.inverse, (long long)nl * nk * a.groups, e.rk.threads, e.rk.smem, a, stream));
       }
     }
@@ -183,17 +197,34 @@ xc_status run(const Engine& e, const void* left, const void* right, void* out, c
 }  // namespace
 
 int length_for(int n) {
-  for (const Factors& f : kLengths)
+  for (const Factors& f : kRows)
     if (f.n >= n) return f.n;
   return 0;
 }
 
-size_t twiddle_count(int n) {
-  const Factors* f = factors(n);
-  return (size_t)(f->r1 - 1) * (n / f->r1) + (f->r2 > 1 ? (size_t)(f->r2 - 1) * f->r3 : 0);
+size_t twiddle_bytes(int n, bool rows) {
+  size_t count = 0;
+  each_twiddle(*factors(n, rows), [&](long long, long long) { ++count; });
+  return 16 * count;
 }
-void fill_twiddles_f32(int n, float* out) { fill(n, out); }
-void fill_twiddles_f64(int n, double* out) { fill(n, out); }
+
+void fill_twiddles(int n, bool rows, xc_dtype dtype, void* out) {
+  float* of = static_cast<float*>(out);
+  double* od = static_cast<double*>(out);
+  each_twiddle(*factors(n, rows), [&](long long k, long long m) {
+    double re, im;
+    root(k, m, &re, &im);
+    if (dtype == XC_F32) {  // one entry serves the two packed transforms
+      of[0] = of[1] = (float)re;
+      of[2] = of[3] = (float)im;
+      of += 4;
+    } else {
+      od[0] = re;
+      od[1] = im;
+      od += 2;
+    }
+  });
+}
 
 xc_status engine_plan(Engine* e, xc_dtype dtype, const Geometry& g, const PairMap& pm, long long n_right,
                       size_t ws_bytes) {
@@ -214,14 +245,19 @@ xc_status engine_plan(Engine* e, xc_dtype dtype, const Geometry& g, const PairMa
   e->nblk = div_up(e->nx / 2 + 1, cb);
   const size_t row = (size_t)e->nblk * cb * ce;  // bytes of one spectrum row
   e->shared = pm.r_l == 0 && pm.n_left > 1;
-  // a left spectrum beside the partner's block in shared memory, while two
-  // CTAs still fit an SM
-  e->lpre = !e->shared && 2 * e->ck.unit_smem > 100 * 1024;
+  // The left spectra are made first (col_forward) when several partners use
+  // them: transforming the left's columns in every CTA of the column kernel
+  // doubles the serial work before its first product (one_to_many 256x256 x
+  // 64: column kernel 47 us against 32).  One to three partners save the
+  // launch instead, while both blocks' shared memory leaves two CTAs per SM.
+  e->lpre = !e->shared && (pm.K >= 4 || 2 * e->ck.unit_smem > 100 * 1024);
 
   // Workspace: row spectra of the lefts and of a chunk of rights, full
-  // spectra of shared matrices, column-inverted products of a chunk.  Chunks
-  // keep what one kernel writes and the next one reads within the L2 cache.
-  const size_t budget = (size_t)64 << 20;
+  // spectra of shared matrices, column-inverted products of a chunk: all
+  // partners in one chunk unless the workspace is smaller (shorter chunks,
+  // whose spectra stay in the L2 cache, measured slower: the launches' ramps
+  // cost more than the traffic; 2048x2048 x 16: 1.78 ms in one chunk, 2.06 in
+  // sixteen; 256x256 x 64: 86 us in one, 112 in two).
   const size_t ar1 = row * g.Hr, b1 = row * g.Sy;
   size_t off = 0;
   const auto take = [&](size_t bytes) {
@@ -239,10 +275,12 @@ xc_status engine_plan(Engine* e, xc_dtype dtype, const Geometry& g, const PairMa
     e->off_b = at;  // products replace the row spectra, which are done with by then
     off = at;
     if (at + b1 > ws_bytes) return XC_OK;
-    const long long fit = std::max<long long>(1, std::min<long long>((long long)(budget / b1), (long long)((ws_bytes - at) / b1)));
-    e->l_chunk = (int)std::min<long long>(pm.n_left, std::max<long long>(1, fit / pm.K));
-    e->k_chunk = (int)std::min<long long>(pm.K, std::max<long long>(1, fit / e->l_chunk));
-    if ((long long)e->l_chunk * e->k_chunk > fit) e->l_chunk = 1;
+    const long long fit = std::max<long long>(1, (long long)((ws_bytes - at) / b1));
+    // whole lefts while one's products fit, else partners of one left; even chunks
+    const int lfit = (int)std::min<long long>(pm.n_left, std::max<long long>(1, fit / pm.K));
+    e->l_chunk = div_up(pm.n_left, div_up(pm.n_left, lfit));
+    const int kfit = (int)std::min<long long>(pm.K, fit);
+    e->k_chunk = e->l_chunk > 1 ? pm.K : div_up(pm.K, div_up(pm.K, kfit));
     off = std::max(a_end, at + align256(b1 * e->l_chunk * e->k_chunk));
     e->kc = 1;
   } else {
@@ -250,16 +288,11 @@ xc_status engine_plan(Engine* e, xc_dtype dtype, const Geometry& g, const PairMa
     e->l_chunk = pm.n_left;
     const size_t per_k = (ar1 + b1) * pm.n_left;  // r_k = n_left rights (one for a single left)
     if (off + per_k + 512 > ws_bytes) return XC_OK;
-    const long long fit = std::max<long long>(1, std::min<long long>((long long)(budget / per_k),
-                                                                    (long long)((ws_bytes - off - 512) / per_k)));
-    e->k_chunk = (int)std::min<long long>(pm.K, fit);
+    const long long fit = (long long)((ws_bytes - off - 512) / per_k);
+    e->k_chunk = div_up(pm.K, div_up(pm.K, (int)std::min<long long>(pm.K, fit)));  // even chunks
     e->off_ar = take(ar1 * pm.n_left * e->k_chunk);
     e->off_b = take(b1 * pm.n_left * e->k_chunk);
-    // partners per CTA: as many as leave eight CTAs per SM
-    const long long units = div_up((long long)pm.n_left * e->nblk, e->ck.pu);
-    e->kc = 1;
-    while (!e->lpre && e->kc < 8 && 2 * e->kc <= e->k_chunk && units * div_up(e->k_chunk, 2 * e->kc) >= 152 * 8)
-      e->kc *= 2;
+    e->kc = e->lpre ? 1 : e->k_chunk;
   }
   e->bytes = off;
   if (e->bytes > ws_bytes) return XC_OK;
@@ -270,17 +303,12 @@ xc_status engine_plan(Engine* e, xc_dtype dtype, const Geometry& g, const PairMa
   XC_TRY(raise_limit(e->ck.pairs_lpre, e->ck.unit_smem));
   XC_TRY(raise_limit(e->ck.pairs_pre, e->ck.unit_smem));
   if (2 * e->ck.unit_smem <= 227 * 1024) XC_TRY(raise_limit(e->ck.pairs, 2 * e->ck.unit_smem));
-  const size_t cx = twiddle_count(e->nx), cy = twiddle_count(e->ny);
-  std::vector<char> host((cx + cy) * ce);
-  if (f32) {
-    fill_twiddles_f32(e->nx, reinterpret_cast<float*>(host.data()));
-    fill_twiddles_f32(e->ny, reinterpret_cast<float*>(host.data() + cx * ce));
-  } else {
-    fill_twiddles_f64(e->nx, reinterpret_cast<double*>(host.data()));
-    fill_twiddles_f64(e->ny, reinterpret_cast<double*>(host.data() + cx * ce));
-  }
+  e->tw_col = twiddle_bytes(e->nx, true);
+  e->zeros = e->tw_col + twiddle_bytes(e->ny, false);
+  std::vector<char> host(e->zeros + (size_t)e->nx * (f32 ? 4 : 8), 0);
+  fill_twiddles(e->nx, true, dtype, host.data());
+  fill_twiddles(e->ny, false, dtype, host.data() + e->tw_col);
   XC_CUDA_TRY(cudaMalloc(&e->tw, host.size()));
-  e->tw_col = cx * ce;
   const cudaError_t err = cudaMemcpy(e->tw, host.data(), host.size(), cudaMemcpyHostToDevice);
   if (err != cudaSuccess) {
     engine_release(e);

@@ -9,13 +9,24 @@
 // and col_forward, which transforms the columns of matrices whose spectra
 // several outputs share.  fft_engine.cu plans and launches them.
 //
-// Transforms are decimation-in-frequency over two or three radix passes
-// N = R1 [R2] R3.  A pass reads and writes the same places, so a pass costs
-// one shared-memory round trip and one barrier.  The column kernel never
-// leaves digit-reversed order: left and right spectra are in the same order,
-// and the inverse (decimation in time) starts from it, so its innermost
-// forward pass, the product and the first inverse pass happen in registers.
-// The row kernels transform two real rows as one complex row.
+// Transforms are decimation-in-frequency over two to four radix passes
+// N = R1 [Ra [Rb]] R3.  A pass reads and writes the same places, so a pass
+// costs one shared-memory round trip and one barrier.  The column kernel
+// never leaves digit-reversed order: left and right spectra are in the same
+// order, and the inverse (decimation in time) starts from it, so its
+// innermost forward pass, the product and the first inverse pass happen in
+// registers.  The row kernels transform two real rows as one complex row; a
+// thread owns the passes' items k and N - k together, so the two rows'
+// spectra are separated (and joined) in registers too.
+//
+// What bounds it.  FP32: a scalar form took 57-63% of the issue slots at 25-40%
+// of the FMA pipe and under 20% of memory, so a thread works on two transforms
+// in packed pairs (add, mul and fma .f32x2: the same rate per value in half
+// the instructions): two adjacent columns or two row pairs.  With that the
+// instructions fell by a third to two fifths and the kernels wait for their
+// loads and for shared memory (64% of its wavefronts in col_pairs), 16 to 24
+// warps per SM: 64 outputs of 511x511 take 80 us, 113 in the scalar form.
+// FP64 is bound by its pipe (85% busy; 1.0 TFLOP/s measured).
 #pragma once
 
 #include <cstdint>
@@ -25,208 +36,285 @@
 namespace xc {
 namespace fe {
 
-template <typename T>
-struct CxOf;
-template <>
-struct CxOf<float> {
-  using type = float2;
+// ---------------------------------------------------------------------------
+// Scalars of the transforms: f2 (two FP32 values, one of each transform) or
+// double.
+// ---------------------------------------------------------------------------
+struct f2 {
+  unsigned long long v;
 };
-template <>
-struct CxOf<double> {
-  using type = double2;
-};
-template <typename T>
-using Cx = typename CxOf<T>::type;
-
-template <typename T>
-__device__ __forceinline__ Cx<T> mk(T x, T y) {
-  Cx<T> r;
-  r.x = x;
-  r.y = y;
+__device__ __forceinline__ f2 pack(float lo, float hi) {
+  f2 r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r.v) : "f"(lo), "f"(hi));
   return r;
 }
-template <typename C>
-__device__ __forceinline__ C cadd(C a, C b) {
-  a.x += b.x;
-  a.y += b.y;
+__device__ __forceinline__ float lo(f2 a) {
+  float x, y;
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(x), "=f"(y) : "l"(a.v));
+  return x;
+}
+__device__ __forceinline__ float hi(f2 a) {
+  float x, y;
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(x), "=f"(y) : "l"(a.v));
+  return y;
+}
+__device__ __forceinline__ f2 add(f2 a, f2 b) {
+  f2 r;
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r.v) : "l"(a.v), "l"(b.v));
+  return r;
+}
+__device__ __forceinline__ f2 sub(f2 a, f2 b) {
+  f2 r;
+  asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(r.v) : "l"(a.v), "l"(b.v));
+  return r;
+}
+__device__ __forceinline__ f2 mul(f2 a, f2 b) {
+  f2 r;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r.v) : "l"(a.v), "l"(b.v));
+  return r;
+}
+__device__ __forceinline__ f2 fma(f2 a, f2 b, f2 c) {
+  f2 r;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r.v) : "l"(a.v), "l"(b.v), "l"(c.v));
+  return r;
+}
+__device__ __forceinline__ f2 neg(f2 a) {
+  a.v ^= 0x8000000080000000ull;
   return a;
 }
-template <typename C>
-__device__ __forceinline__ C csub(C a, C b) {
-  a.x -= b.x;
-  a.y -= b.y;
-  return a;
+__device__ __forceinline__ double add(double a, double b) { return a + b; }
+__device__ __forceinline__ double sub(double a, double b) { return a - b; }
+__device__ __forceinline__ double mul(double a, double b) { return a * b; }
+__device__ __forceinline__ double fma(double a, double b, double c) { return ::fma(a, b, c); }
+__device__ __forceinline__ double neg(double a) { return -a; }
+
+template <typename S>
+struct Sc;
+template <>
+struct Sc<f2> {
+  using real = float;
+  static constexpr int NV = 2;  // transforms per thread
+  static __device__ __forceinline__ f2 bc(double c) { return pack((float)c, (float)c); }
+};
+template <>
+struct Sc<double> {
+  using real = double;
+  static constexpr int NV = 1;
+  static __device__ __forceinline__ double bc(double c) { return c; }
+};
+
+// A complex value of each transform: 16 bytes for either scalar.
+template <typename S>
+struct alignas(16) Cp {
+  S x, y;
+};
+template <typename S>
+__device__ __forceinline__ Cp<S> cadd(Cp<S> a, Cp<S> b) {
+  return {add(a.x, b.x), add(a.y, b.y)};
+}
+template <typename S>
+__device__ __forceinline__ Cp<S> csub(Cp<S> a, Cp<S> b) {
+  return {sub(a.x, b.x), sub(a.y, b.y)};
+}
+// a + (D i) b, D = +-1
+template <int D, typename S>
+__device__ __forceinline__ Cp<S> cadd_i(Cp<S> a, Cp<S> b) {
+  if (D > 0) return {sub(a.x, b.y), add(a.y, b.x)};
+  return {add(a.x, b.y), sub(a.y, b.x)};
+}
+// a + c b for a real constant
+template <typename S>
+__device__ __forceinline__ Cp<S> cfma(S c, Cp<S> b, Cp<S> a) {
+  return {fma(c, b.x, a.x), fma(c, b.y, a.y)};
+}
+// a + (D i c) b
+template <int D, typename S>
+__device__ __forceinline__ Cp<S> cfma_i(S c, S nc, Cp<S> b, Cp<S> a) {
+  if (D > 0) return {fma(nc, b.y, a.x), fma(c, b.x, a.y)};
+  return {fma(c, b.y, a.x), fma(nc, b.x, a.y)};
 }
 // a * b, or a * conj(b)
-template <bool CONJ, typename C>
-__device__ __forceinline__ C cmul(C a, C b) {
-  C r;
-  if (CONJ) {
-    r.x = a.x * b.x + a.y * b.y;
-    r.y = a.y * b.x - a.x * b.y;
-  } else {
-    r.x = a.x * b.x - a.y * b.y;
-    r.y = a.y * b.x + a.x * b.y;
-  }
-  return r;
+template <bool CONJ, typename S>
+__device__ __forceinline__ Cp<S> cmul(Cp<S> a, Cp<S> b) {
+  const S nby = neg(b.y);
+  if (CONJ) return {fma(a.y, b.y, mul(a.x, b.x)), fma(a.x, nby, mul(a.y, b.x))};
+  return {fma(a.y, nby, mul(a.x, b.x)), fma(a.x, b.y, mul(a.y, b.x))};
 }
-// a * (S i): S = -1 for forward transforms, +1 for inverse ones
-template <int S, typename C>
-__device__ __forceinline__ C mul_i(C a) {
-  C r;
-  r.x = S > 0 ? -a.y : a.y;
-  r.y = S > 0 ? a.x : -a.x;
-  return r;
+template <typename S>
+__device__ __forceinline__ Cp<S> czero() {
+  return {Sc<S>::bc(0.0), Sc<S>::bc(0.0)};
+}
+template <typename S>
+__device__ __forceinline__ Cp<S> csel(bool p, Cp<S> a, Cp<S> b) {
+  return p ? a : b;
 }
 
 // ---------------------------------------------------------------------------
 // In-register transforms of R values, natural order in and out,
-// X[k] = sum_n x[n] exp(S 2 pi i n k / R).
+// X[k] = sum_n x[n] exp(D 2 pi i n k / R), D = -1 forward, +1 inverse.
 // ---------------------------------------------------------------------------
-template <typename T, int S, int R>
+template <typename S, int D, int R>
 struct Dft;
 
-template <typename T, int S>
-struct Dft<T, S, 2> {
-  using C = Cx<T>;
-  static __device__ __forceinline__ void run(C* x) {
-    const C a = x[0], b = x[1];
+template <typename S, int D>
+struct Dft<S, D, 2> {
+  static __device__ __forceinline__ void run(Cp<S>* x) {
+    const Cp<S> a = x[0], b = x[1];
     x[0] = cadd(a, b);
     x[1] = csub(a, b);
   }
 };
 
-template <typename T, int S>
-struct Dft<T, S, 4> {
-  using C = Cx<T>;
-  static __device__ __forceinline__ void run(C* x) {
-    const C a = cadd(x[0], x[2]), b = csub(x[0], x[2]);
-    const C c = cadd(x[1], x[3]), d = mul_i<S>(csub(x[1], x[3]));
+template <typename S, int D>
+struct Dft<S, D, 4> {
+  static __device__ __forceinline__ void run(Cp<S>* x) {
+    const Cp<S> a = cadd(x[0], x[2]), b = csub(x[0], x[2]);
+    const Cp<S> c = cadd(x[1], x[3]), d = csub(x[1], x[3]);
     x[0] = cadd(a, c);
-    x[1] = cadd(b, d);
+    x[1] = cadd_i<D>(b, d);
     x[2] = csub(a, c);
-    x[3] = csub(b, d);
+    x[3] = cadd_i<-D>(b, d);
   }
 };
 
-template <typename T, int S>
-struct Dft<T, S, 3> {
-  using C = Cx<T>;
-  static __device__ __forceinline__ void run(C* x) {
-    constexpr T h = T(0.8660254037844386467637231707529362);  // sin(2 pi / 3)
-    const C s = cadd(x[1], x[2]), d = csub(x[1], x[2]);
-    const C m = mk<T>(x[0].x - T(0.5) * s.x, x[0].y - T(0.5) * s.y);
-    const C r = mul_i<S>(mk<T>(h * d.x, h * d.y));
+template <typename S, int D>
+struct Dft<S, D, 3> {
+  static __device__ __forceinline__ void run(Cp<S>* x) {
+    constexpr double h = 0.8660254037844386467637231707529362;  // sin(2 pi / 3)
+    const S ch = Sc<S>::bc(h), nh = Sc<S>::bc(-h);
+    const Cp<S> s = cadd(x[1], x[2]), d = csub(x[1], x[2]);
+    const Cp<S> m = cfma(Sc<S>::bc(-0.5), s, x[0]);
     x[0] = cadd(x[0], s);
-    x[1] = cadd(m, r);
-    x[2] = csub(m, r);
+    x[1] = cfma_i<D>(ch, nh, d, m);
+    x[2] = cfma_i<-D>(ch, nh, d, m);
   }
 };
 
-// Odd prime R by symmetry: sums and differences of x[n], x[R-n].
-template <typename T, int S>
-struct Dft<T, S, 5> {
-  using C = Cx<T>;
-  static __device__ __forceinline__ void run(C* x) {
-    constexpr T c1 = T(0.3090169943749474241022934171828191), c2 = T(-0.8090169943749474241022934171828191);
-    constexpr T s1 = T(0.9510565162951535721164393333793821), s2 = T(0.5877852522924731291687059546390728);
-    const C a1 = cadd(x[1], x[4]), b1 = csub(x[1], x[4]);
-    const C a2 = cadd(x[2], x[3]), b2 = csub(x[2], x[3]);
-    const C m1 = mk<T>(x[0].x + c1 * a1.x + c2 * a2.x, x[0].y + c1 * a1.y + c2 * a2.y);
-    const C m2 = mk<T>(x[0].x + c2 * a1.x + c1 * a2.x, x[0].y + c2 * a1.y + c1 * a2.y);
-    const C r1 = mul_i<S>(mk<T>(s1 * b1.x + s2 * b2.x, s1 * b1.y + s2 * b2.y));
-    const C r2 = mul_i<S>(mk<T>(s2 * b1.x - s1 * b2.x, s2 * b1.y - s1 * b2.y));
+// Odd primes by symmetry: sums and differences of x[n], x[R-n].
+template <typename S, int D>
+struct Dft<S, D, 5> {
+  static __device__ __forceinline__ void run(Cp<S>* x) {
+    constexpr double k1 = 0.3090169943749474241022934171828191, k2 = -0.8090169943749474241022934171828191;
+    constexpr double l1 = 0.9510565162951535721164393333793821, l2 = 0.5877852522924731291687059546390728;
+    const S c1 = Sc<S>::bc(k1), c2 = Sc<S>::bc(k2), s1 = Sc<S>::bc(l1), s2 = Sc<S>::bc(l2), n1 = Sc<S>::bc(-l1);
+    const Cp<S> a1 = cadd(x[1], x[4]), b1 = csub(x[1], x[4]);
+    const Cp<S> a2 = cadd(x[2], x[3]), b2 = csub(x[2], x[3]);
+    const Cp<S> m1 = cfma(c2, a2, cfma(c1, a1, x[0]));
+    const Cp<S> m2 = cfma(c1, a2, cfma(c2, a1, x[0]));
+    const Cp<S> r1 = {fma(s2, b2.x, mul(s1, b1.x)), fma(s2, b2.y, mul(s1, b1.y))};
+    const Cp<S> r2 = {fma(n1, b2.x, mul(s2, b1.x)), fma(n1, b2.y, mul(s2, b1.y))};
     x[0] = cadd(x[0], cadd(a1, a2));
-    x[1] = cadd(m1, r1);
-    x[4] = csub(m1, r1);
-    x[2] = cadd(m2, r2);
-    x[3] = csub(m2, r2);
+    x[1] = cadd_i<D>(m1, r1);
+    x[4] = cadd_i<-D>(m1, r1);
+    x[2] = cadd_i<D>(m2, r2);
+    x[3] = cadd_i<-D>(m2, r2);
   }
 };
 
-template <typename T, int S>
-struct Dft<T, S, 7> {
-  using C = Cx<T>;
-  static __device__ __forceinline__ void run(C* x) {
-    constexpr T c1 = T(0.6234898018587335305250048840042398), c2 = T(-0.2225209339563144042889025644967948),
-                c3 = T(-0.9009688679024191262361023195074451);
-    constexpr T s1 = T(0.7818314824680298087084445266740578), s2 = T(0.9749279121818236070181316829939312),
-                s3 = T(0.4338837391175581204757683328483587);
-    const C a1 = cadd(x[1], x[6]), b1 = csub(x[1], x[6]);
-    const C a2 = cadd(x[2], x[5]), b2 = csub(x[2], x[5]);
-    const C a3 = cadd(x[3], x[4]), b3 = csub(x[3], x[4]);
-    const C m1 = mk<T>(x[0].x + c1 * a1.x + c2 * a2.x + c3 * a3.x, x[0].y + c1 * a1.y + c2 * a2.y + c3 * a3.y);
-    const C m2 = mk<T>(x[0].x + c2 * a1.x + c3 * a2.x + c1 * a3.x, x[0].y + c2 * a1.y + c3 * a2.y + c1 * a3.y);
-    const C m3 = mk<T>(x[0].x + c3 * a1.x + c1 * a2.x + c2 * a3.x, x[0].y + c3 * a1.y + c1 * a2.y + c2 * a3.y);
-    const C r1 = mul_i<S>(mk<T>(s1 * b1.x + s2 * b2.x + s3 * b3.x, s1 * b1.y + s2 * b2.y + s3 * b3.y));
-    const C r2 = mul_i<S>(mk<T>(s2 * b1.x - s3 * b2.x - s1 * b3.x, s2 * b1.y - s3 * b2.y - s1 * b3.y));
-    const C r3 = mul_i<S>(mk<T>(s3 * b1.x - s1 * b2.x + s2 * b3.x, s3 * b1.y - s1 * b2.y + s2 * b3.y));
+template <typename S, int D>
+struct Dft<S, D, 7> {
+  static __device__ __forceinline__ void run(Cp<S>* x) {
+    constexpr double k1 = 0.6234898018587335305250048840042398, k2 = -0.2225209339563144042889025644967948,
+                     k3 = -0.9009688679024191262361023195074451;
+    constexpr double l1 = 0.7818314824680298087084445266740578, l2 = 0.9749279121818236070181316829939312,
+                     l3 = 0.4338837391175581204757683328483587;
+    const S c1 = Sc<S>::bc(k1), c2 = Sc<S>::bc(k2), c3 = Sc<S>::bc(k3);
+    const S s1 = Sc<S>::bc(l1), s2 = Sc<S>::bc(l2), s3 = Sc<S>::bc(l3), n1 = Sc<S>::bc(-l1), n3 = Sc<S>::bc(-l3);
+    const Cp<S> a1 = cadd(x[1], x[6]), b1 = csub(x[1], x[6]);
+    const Cp<S> a2 = cadd(x[2], x[5]), b2 = csub(x[2], x[5]);
+    const Cp<S> a3 = cadd(x[3], x[4]), b3 = csub(x[3], x[4]);
+    const Cp<S> m1 = cfma(c3, a3, cfma(c2, a2, cfma(c1, a1, x[0])));
+    const Cp<S> m2 = cfma(c1, a3, cfma(c3, a2, cfma(c2, a1, x[0])));
+    const Cp<S> m3 = cfma(c2, a3, cfma(c1, a2, cfma(c3, a1, x[0])));
+    const Cp<S> r1 = {fma(s3, b3.x, fma(s2, b2.x, mul(s1, b1.x))), fma(s3, b3.y, fma(s2, b2.y, mul(s1, b1.y)))};
+    const Cp<S> r2 = {fma(n1, b3.x, fma(n3, b2.x, mul(s2, b1.x))), fma(n1, b3.y, fma(n3, b2.y, mul(s2, b1.y)))};
+    const Cp<S> r3 = {fma(s2, b3.x, fma(n1, b2.x, mul(s3, b1.x))), fma(s2, b3.y, fma(n1, b2.y, mul(s3, b1.y)))};
     x[0] = cadd(x[0], cadd(a1, cadd(a2, a3)));
-    x[1] = cadd(m1, r1);
-    x[6] = csub(m1, r1);
-    x[2] = cadd(m2, r2);
-    x[5] = csub(m2, r2);
-    x[3] = cadd(m3, r3);
-    x[4] = csub(m3, r3);
+    x[1] = cadd_i<D>(m1, r1);
+    x[6] = cadd_i<-D>(m1, r1);
+    x[2] = cadd_i<D>(m2, r2);
+    x[5] = cadd_i<-D>(m2, r2);
+    x[3] = cadd_i<D>(m3, r3);
+    x[4] = cadd_i<-D>(m3, r3);
   }
 };
 
-template <typename T, int S>
-struct Dft<T, S, 8> {
-  using C = Cx<T>;
-  static __device__ __forceinline__ void run(C* x) {
-    constexpr T h = T(0.7071067811865475244008443621048490);
-    C e[4] = {x[0], x[2], x[4], x[6]}, o[4] = {x[1], x[3], x[5], x[7]};
-    Dft<T, S, 4>::run(e);
-    Dft<T, S, 4>::run(o);
-    // o[k] *= exp(S 2 pi i k / 8)
-    const C i1 = mul_i<S>(o[1]), i3 = mul_i<S>(o[3]);
-    o[1] = mk<T>(h * (o[1].x + i1.x), h * (o[1].y + i1.y));
-    o[2] = mul_i<S>(o[2]);
-    o[3] = mk<T>(h * (i3.x - o[3].x), h * (i3.y - o[3].y));
-#pragma unroll
-    for (int k = 0; k < 4; ++k) {
-      x[k] = cadd(e[k], o[k]);
-      x[k + 4] = csub(e[k], o[k]);
-    }
+template <typename S, int D>
+struct Dft<S, D, 8> {
+  static __device__ __forceinline__ void run(Cp<S>* x) {
+    constexpr double k = 0.7071067811865475244008443621048490;
+    const S h = Sc<S>::bc(k), nh = Sc<S>::bc(-k);
+    Cp<S> e[4] = {x[0], x[2], x[4], x[6]}, o[4] = {x[1], x[3], x[5], x[7]};
+    Dft<S, D, 4>::run(e);
+    Dft<S, D, 4>::run(o);
+    // o[n] exp(D 2 pi i n / 8): n = 1: h (1 + D i) o, n = 2: D i o, n = 3: -h (1 - D i) o
+    const Cp<S> u1 = cadd_i<D>(o[1], o[1]), u3 = cadd_i<-D>(o[3], o[3]);
+    x[0] = cadd(e[0], o[0]);
+    x[4] = csub(e[0], o[0]);
+    x[1] = cfma(h, u1, e[1]);
+    x[5] = cfma(nh, u1, e[1]);
+    x[2] = cadd_i<D>(e[2], o[2]);
+    x[6] = cadd_i<-D>(e[2], o[2]);
+    x[3] = cfma(nh, u3, e[3]);
+    x[7] = cfma(h, u3, e[3]);
   }
 };
 
-template <typename T, int S>
-struct Dft<T, S, 16> {
-  using C = Cx<T>;
-  static __device__ __forceinline__ void run(C* x) {
-    constexpr T h = T(0.7071067811865475244008443621048490);
-    constexpr T c = T(0.9238795325112867561281831893967882), s = T(0.3826834323650897717284599840303988);
-    const T sg = S > 0 ? T(1) : T(-1);
-    C y[4][4];  // [n2][k1]
+template <typename S, int D>
+struct Dft<S, D, 16> {
+  static __device__ __forceinline__ void run(Cp<S>* x) {
+    constexpr double kh = 0.7071067811865475244008443621048490;
+    constexpr double kc = 0.9238795325112867561281831893967882, ks = 0.3826834323650897717284599840303988;
+    const S h = Sc<S>::bc(kh), nh = Sc<S>::bc(-kh);
+    Cp<S> y[4][4];  // [n2][k1]
 #pragma unroll
     for (int n2 = 0; n2 < 4; ++n2) {
 #pragma unroll
       for (int n1 = 0; n1 < 4; ++n1) y[n2][n1] = x[4 * n1 + n2];
-      Dft<T, S, 4>::run(y[n2]);
+      Dft<S, D, 4>::run(y[n2]);
     }
-    // y[n2][k1] *= exp(S 2 pi i n2 k1 / 16)
-    const C w1 = mk<T>(c, sg * s), w3 = mk<T>(s, sg * c), w9 = mk<T>(-c, -sg * s);
-    auto eighth = [](C v) {  // exp(S pi i / 4)
-      const C i = mul_i<S>(v);
-      return mk<T>(h * (v.x + i.x), h * (v.y + i.y));
+    // y[n2][k1] *= exp(D 2 pi i n2 k1 / 16)
+    constexpr double sg = D > 0 ? 1.0 : -1.0;
+    const auto rot = [](Cp<S> a, double wx, double wy) {
+      const S cx = Sc<S>::bc(wx), cy = Sc<S>::bc(wy), ny = Sc<S>::bc(-wy);
+      return Cp<S>{fma(a.y, ny, mul(a.x, cx)), fma(a.x, cy, mul(a.y, cx))};
     };
-    y[1][1] = cmul<false>(y[1][1], w1);
-    y[1][2] = eighth(y[1][2]);
-    y[1][3] = cmul<false>(y[1][3], w3);
-    y[2][1] = eighth(y[2][1]);
-    y[2][2] = mul_i<S>(y[2][2]);
-    y[2][3] = eighth(mul_i<S>(y[2][3]));
-    y[3][1] = cmul<false>(y[3][1], w3);
-    y[3][2] = eighth(mul_i<S>(y[3][2]));
-    y[3][3] = cmul<false>(y[3][3], w9);
+    y[1][1] = rot(y[1][1], kc, sg * ks);
+    y[1][3] = rot(y[1][3], ks, sg * kc);
+    y[3][1] = rot(y[3][1], ks, sg * kc);
+    y[3][3] = rot(y[3][3], -kc, -sg * ks);
+    // the eighths, left unscaled: u = (1 + D i) y or (1 - D i) y, times +-h below
+    const Cp<S> u12 = cadd_i<D>(y[1][2], y[1][2]), u32 = cadd_i<-D>(y[3][2], y[3][2]);
+    const Cp<S> u21 = cadd_i<D>(y[2][1], y[2][1]), u23 = cadd_i<-D>(y[2][3], y[2][3]);
+    {  // k1 = 0
+      Cp<S> z[4] = {y[0][0], y[1][0], y[2][0], y[3][0]};
+      Dft<S, D, 4>::run(z);
 #pragma unroll
-    for (int k1 = 0; k1 < 4; ++k1) {
-      C z[4] = {y[0][k1], y[1][k1], y[2][k1], y[3][k1]};
-      Dft<T, S, 4>::run(z);
-#pragma unroll
-      for (int k2 = 0; k2 < 4; ++k2) x[k1 + 4 * k2] = z[k2];
+      for (int k2 = 0; k2 < 4; ++k2) x[4 * k2] = z[k2];
+    }
+    {  // k1 = 1: second input h u21
+      const Cp<S> a = cfma(h, u21, y[0][1]), b = cfma(nh, u21, y[0][1]);
+      const Cp<S> c = cadd(y[1][1], y[3][1]), d = csub(y[1][1], y[3][1]);
+      x[1] = cadd(a, c);
+      x[5] = cadd_i<D>(b, d);
+      x[9] = csub(a, c);
+      x[13] = cadd_i<-D>(b, d);
+    }
+    {  // k1 = 2: inputs y02, h u12, D i y22, -h u32
+      const Cp<S> a = cadd_i<D>(y[0][2], y[2][2]), b = cadd_i<-D>(y[0][2], y[2][2]);
+      const Cp<S> c = csub(u12, u32), d = cadd(u12, u32);
+      x[2] = cfma(h, c, a);
+      x[6] = cfma_i<D>(h, nh, d, b);
+      x[10] = cfma(nh, c, a);
+      x[14] = cfma_i<-D>(h, nh, d, b);
+    }
+    {  // k1 = 3: third input -h u23
+      const Cp<S> a = cfma(nh, u23, y[0][3]), b = cfma(h, u23, y[0][3]);
+      const Cp<S> c = cadd(y[1][3], y[3][3]), d = csub(y[1][3], y[3][3]);
+      x[3] = cadd(a, c);
+      x[7] = cadd_i<D>(b, d);
+      x[11] = csub(a, c);
+      x[15] = cadd_i<-D>(b, d);
     }
   }
 };
@@ -238,441 +326,592 @@ constexpr int crt(int A, int B, int k1, int k2) {
     if (k % A == k1 && k % B == k2) return k;
   return 0;
 }
-template <typename T, int S, int A, int B>
+template <typename S, int D, int A, int B>
 struct DftPfa {
-  using C = Cx<T>;
-  static __device__ __forceinline__ void run(C* x) {
+  static __device__ __forceinline__ void run(Cp<S>* x) {
     constexpr int R = A * B;
-    C y[B][A];
+    Cp<S> y[B][A];
 #pragma unroll
     for (int n2 = 0; n2 < B; ++n2) {
 #pragma unroll
       for (int n1 = 0; n1 < A; ++n1) y[n2][n1] = x[(B * n1 + A * n2) % R];
-      // n k / R = n1 k1 / A + n2 k2 / B (mod 1): B n1 k / R = n1 k / A
-      Dft<T, S, A>::run(y[n2]);
+      Dft<S, D, A>::run(y[n2]);  // n k / R = n1 k / A + n2 k / B (mod 1)
     }
 #pragma unroll
     for (int k1 = 0; k1 < A; ++k1) {
-      C z[B];
+      Cp<S> z[B];
 #pragma unroll
       for (int n2 = 0; n2 < B; ++n2) z[n2] = y[n2][k1];
-      Dft<T, S, B>::run(z);
+      Dft<S, D, B>::run(z);
 #pragma unroll
       for (int k2 = 0; k2 < B; ++k2) x[crt(A, B, k1, k2)] = z[k2];
     }
   }
 };
-template <typename T, int S>
-struct Dft<T, S, 6> : DftPfa<T, S, 2, 3> {};
-template <typename T, int S>
-struct Dft<T, S, 10> : DftPfa<T, S, 2, 5> {};
-template <typename T, int S>
-struct Dft<T, S, 12> : DftPfa<T, S, 4, 3> {};
-template <typename T, int S>
-struct Dft<T, S, 14> : DftPfa<T, S, 2, 7> {};
+template <typename S, int D>
+struct Dft<S, D, 6> : DftPfa<S, D, 2, 3> {};
+template <typename S, int D>
+struct Dft<S, D, 10> : DftPfa<S, D, 2, 5> {};
+template <typename S, int D>
+struct Dft<S, D, 12> : DftPfa<S, D, 4, 3> {};
+template <typename S, int D>
+struct Dft<S, D, 14> : DftPfa<S, D, 2, 7> {};
 
 // ---------------------------------------------------------------------------
-// Lengths and their passes.  R1 >= R2 >= R3 where possible; R2 = 1: two
-// passes.  All lengths are multiples of 16, at most 25% apart (33% below 64).
+// Lengths and their passes.  All lengths are multiples of 16, at most 25%
+// apart (33% below 64).  Columns: X(N, R1, Ra, R3), R1 >= Ra >= R3, as few
+// passes as 16 registers' worth allows.  Rows: X(N, R1, Ra, Rb, R3), with R1
+// and R3 small, because a row thread holds two items of its first (inverse) or
+// last (forward) pass, and alike, so that neither pass leaves threads idle.
 // ---------------------------------------------------------------------------
-#define XC_FFT_LENGTHS(X)                                                                                   \
+#define XC_FFT_COLS(X)                                                                                   \
   X(16, 4, 1, 4) X(32, 8, 1, 4) X(48, 8, 1, 6) X(64, 8, 1, 8) X(80, 10, 1, 8) X(96, 12, 1, 8)              \
   X(112, 14, 1, 8) X(128, 16, 1, 8) X(160, 16, 1, 10) X(192, 16, 1, 12) X(224, 16, 1, 14) X(256, 16, 1, 16) \
   X(320, 8, 8, 5) X(384, 8, 8, 6) X(448, 8, 8, 7) X(512, 8, 8, 8) X(640, 10, 8, 8) X(768, 12, 8, 8)         \
   X(896, 14, 8, 8) X(1024, 16, 8, 8) X(1280, 16, 10, 8) X(1536, 16, 12, 8) X(1792, 16, 14, 8)              \
   X(2048, 16, 16, 8) X(2560, 16, 16, 10) X(3072, 16, 16, 12) X(3584, 16, 16, 14) X(4096, 16, 16, 16)
+#define XC_FFT_ROWS(X)                                                                                     \
+  X(16, 4, 1, 1, 4) X(32, 8, 1, 1, 4) X(48, 8, 1, 1, 6) X(64, 8, 1, 1, 8) X(80, 10, 1, 1, 8)                 \
+  X(96, 12, 1, 1, 8) X(112, 8, 1, 1, 14) X(128, 4, 8, 1, 4) X(160, 4, 10, 1, 4) X(192, 8, 3, 1, 8)           \
+  X(224, 4, 14, 1, 4) X(256, 8, 4, 1, 8) X(320, 8, 5, 1, 8) X(384, 8, 6, 1, 8) X(448, 8, 7, 1, 8)            \
+  X(512, 8, 8, 1, 8) X(640, 8, 10, 1, 8) X(768, 8, 12, 1, 8) X(896, 8, 14, 1, 8) X(1024, 8, 16, 1, 8)         \
+  X(1280, 8, 5, 4, 8) X(1536, 8, 6, 4, 8) X(1792, 8, 7, 4, 8) X(2048, 8, 8, 4, 8) X(2560, 8, 8, 5, 8)         \
+  X(3072, 8, 8, 6, 8) X(3584, 8, 8, 7, 8) X(4096, 8, 8, 8, 8)
 
-template <int N>
-struct Fac;
-#define XC_FAC(N_, A_, B_, C_)                             \
-  template <>                                              \
-  struct Fac<N_> {                                         \
-    static constexpr int R1 = A_, R2 = B_, R3 = C_;        \
-    static_assert(A_ * B_ * C_ == N_, "factors of length"); \
-  };
-XC_FFT_LENGTHS(XC_FAC)
-#undef XC_FAC
-
-// Derived geometry of a length.  Element (q1, q2, m) of the pass structure --
-// index q1 S1 + q2 R3 + m -- lies at q1 P1 + q2 PR + m in shared memory: odd
-// strides, so that the passes that walk q1 or q2 across lanes hit different
+// Geometry of a pass structure.  Element (q1, qa, qb, m) -- index q1 S1 +
+// qa Sa + qb R3 + m -- lies at q1 P1 + qa Pa + qb PR + m in shared memory:
+// odd strides, so that passes that walk a digit across lanes hit different
 // banks.
-template <int N>
-struct Len {
-  static constexpr int R1 = Fac<N>::R1, R2 = Fac<N>::R2, R3 = Fac<N>::R3;
-  static constexpr bool three = R2 > 1;
-  static constexpr int S1 = N / R1;         // stride of the first pass
+template <int N_, int R1_, int Ra_, int Rb_, int R3_>
+struct Passes {
+  static constexpr int N = N_, R1 = R1_, Ra = Ra_, Rb = Rb_, R3 = R3_;
+  static_assert(R1 * Ra * Rb * R3 == N, "factors of the length");
+  static constexpr int S1 = N / R1, Sa = S1 / Ra;
+  static constexpr int TF = N / R3;  // items of the last pass
   static constexpr int PR = R3 | 1;
-  static constexpr int P1 = (R2 * PR) | 1;
-  static constexpr int rows = R1 * P1;      // padded length
-  static constexpr int rmax = R1 > R3 ? R1 : R3;
-  static constexpr int tw1 = 0;             // twiddles of pass 1: (R1 - 1) x S1, [q - 1][o]
-  static constexpr int tw2 = (R1 - 1) * S1;  // of pass 2: (R2 - 1) x R3, [q - 1][o]
-  static constexpr int ntw = tw2 + (three ? (R2 - 1) * R3 : 0);
-  static __device__ __forceinline__ int pos(int i) {  // padded place of index i
-    const int q1 = i / S1, o = i - q1 * S1;
-    if (!three) return q1 * P1 + o;
-    const int q2 = o / R3;
-    return q1 * P1 + q2 * PR + (o - q2 * R3);
+  static constexpr int Pa = Rb > 1 ? (Rb * PR) | 1 : PR;
+  static constexpr int P1 = Ra > 1 ? (Ra * Pa) | 1 : Pa;
+  static constexpr int rows = R1 * P1;        // padded length
+  static constexpr int tw_a = (R1 - 1) * S1;  // twiddles: [q - 1][o] of each pass but the last
+  static constexpr int tw_b = tw_a + (Ra - 1) * Sa;
+  static constexpr int n_tw = tw_b + (Rb - 1) * R3;
+  // place of offset o < S1 within the first digit's block
+  static __device__ __forceinline__ int in_block(int o) {
+    if (Ra == 1) return o;
+    const int qa = o / Sa, r = o - qa * Sa;
+    if (Rb == 1) return qa * Pa + r;
+    const int qb = r / R3;
+    return qa * Pa + qb * PR + (r - qb * R3);
+  }
+  // place of the last pass's item i, whose outputs are k = i + q TF
+  static __device__ __forceinline__ int last_item(int i) {
+    if (Ra == 1) return i * P1;
+    const int q1 = i % R1, r = i / R1;
+    if (Rb == 1) return q1 * P1 + r * Pa;
+    return q1 * P1 + (r % Ra) * Pa + (r / Ra) * PR;
   }
 };
+template <int N>
+struct RowPasses;
+template <int N>
+struct ColPasses;
+#define XC_DEF(N_, A_, B_, C_, D_) \
+  template <>                      \
+  struct RowPasses<N_> : Passes<N_, A_, B_, C_, D_> {};
+XC_FFT_ROWS(XC_DEF)
+#undef XC_DEF
+#define XC_DEF(N_, A_, B_, D_) \
+  template <>                  \
+  struct ColPasses<N_> : Passes<N_, A_, B_, 1, D_> {};
+XC_FFT_COLS(XC_DEF)
+#undef XC_DEF
+
+// A pass between the first and the last, in place: radix R, items of `LEN`
+// elements' blocks with offsets o < ST; block b of the pass starts at
+// place(b), its elements PS apart.  Forward and row-inverse passes are
+// decimation in frequency (twiddles after), column-inverse ones decimation in
+// time (twiddles before).
+template <typename S, int D, bool DIT, int R, int PS, int STEP>
+__device__ __forceinline__ void butterfly(Cp<S>* base, const Cp<S>* __restrict__ tw, int tw_step) {
+  Cp<S> x[R];
+  if (!DIT) {
+#pragma unroll
+    for (int m = 0; m < R; ++m) x[m] = base[m * PS * STEP];
+    Dft<S, D, R>::run(x);
+    base[0] = x[0];
+#pragma unroll
+    for (int q = 1; q < R; ++q) base[q * PS * STEP] = cmul<(D > 0)>(x[q], tw[(q - 1) * tw_step]);
+  } else {
+    x[0] = base[0];
+#pragma unroll
+    for (int q = 1; q < R; ++q) x[q] = cmul<(D > 0)>(base[q * PS * STEP], tw[(q - 1) * tw_step]);
+    Dft<S, D, R>::run(x);
+#pragma unroll
+    for (int m = 0; m < R; ++m) base[m * PS * STEP] = x[m];
+  }
+}
+template <typename S, int D, bool DIT, typename L, int STEP>
+__device__ __forceinline__ void mid_passes(Cp<S>* z, int it0, int step, const Cp<S>* __restrict__ tw) {
+  if constexpr (L::Ra > 1) {
+    for (int it = it0; it < L::N / L::Ra; it += step) {
+      const int b = it / L::Sa, o = it - b * L::Sa;
+      const int at = b * L::P1 + (L::Rb > 1 ? (o / L::R3) * L::PR + o % L::R3 : o);
+      butterfly<S, D, DIT, L::Ra, L::Pa, STEP>(z + at * STEP, tw + L::tw_a + o, L::Sa);
+    }
+    __syncthreads();
+  }
+  if constexpr (L::Rb > 1) {
+    static_assert(!DIT, "four passes: rows only");
+    for (int it = it0; it < L::N / L::Rb; it += step) {
+      const int b = it / L::R3, o = it - b * L::R3;
+      const int at = (b / L::Ra) * L::P1 + (b % L::Ra) * L::Pa + o;
+      butterfly<S, D, DIT, L::Rb, L::PR, STEP>(z + at * STEP, tw + L::tw_b + o, L::R3);
+    }
+    __syncthreads();
+  }
+}
 
 // ---------------------------------------------------------------------------
 // Layout of the half spectra between the kernels: matrix by matrix, blocks of
-// CB = 2^lgcb columns, [block][row][column in block], columns 0..N/2 rounded
-// up to whole blocks.  A row pair's share of a block is contiguous (row
-// kernels), and so is a whole block (column kernels).
+// CB = 2^lgcb columns, [block][row][column in block] of complex values,
+// columns 0..N/2 rounded up to whole blocks (the columns beyond N/2 are never
+// written by the row kernels nor read by them).  A row pair's share of a
+// block is contiguous (row kernels), and so is a whole block (column kernels).
 // ---------------------------------------------------------------------------
+template <typename T>
+struct Cx {
+  T x, y;
+};
 template <typename T>
 struct RowSide {
   const T* src;  // matrices, H x W each
   Cx<T>* dst;    // half spectra of their rows
   int H, W;
   int groups;    // CTAs per matrix
+  T scale;       // of the spectra (times the 1/2 of the separation)
 };
 template <typename T>
 struct RowFwdArgs {
   RowSide<T> a, b;    // blocks [0, a_blocks) on side a, the rest on side b
   unsigned a_blocks;
   int nblk, lgcb;
-  const Cx<T>* tw;
+  const void* tw;     // Cp<S> entries
+  const T* zeros;     // a row of zeros, read in the place of rows past the last
 };
 
 template <typename T>
 struct ColArgs {
-  const Cx<T>* left;   // row spectra of the lefts, or (LPRE) their full spectra
-  const Cx<T>* right;  // the same of the rights (RPRE)
-  Cx<T>* out;          // column-inverted products, Sy rows in output order
+  const void* left;   // row spectra of the lefts, or (LPRE) their full spectra
+  const void* right;  // the same of the rights (RPRE)
+  Cx<T>* out;         // column-inverted products, Sy rows in output order
   int Hl, Hr, Sy;
   int nblk;
-  int n_left;          // lefts l0 .. l0 + n_left - 1 of this launch
-  int l0, k0, k1;      // partners k0 .. k1 - 1 of each
-  int n_kg, kc;        // partner groups of kc partners
+  int n_left;         // lefts l0 .. l0 + n_left - 1 of this launch
+  int l0, k0, k1;     // partners k0 .. k1 - 1 of each
+  int n_kg, kc;       // partner groups of kc partners
   long long r_l, r_k, r_off;  // right(l, k) = l r_l + k r_k - r_off within `right`
-  const Cx<T>* tw;
+  const void* tw;
 };
 template <typename T>
 struct ColFwdArgs {
-  const Cx<T>* src;    // row spectra, H rows
-  Cx<T>* dst;          // full spectra, N rows in pass order
+  const Cx<T>* src;   // row spectra, H rows
+  void* dst;          // full spectra: Cp<S> in pass order
   int H, nblk;
-  long long units;     // matrices x nblk
-  const Cx<T>* tw;
+  long long units;    // matrices x nblk
+  const void* tw;
 };
 template <typename T>
 struct RowInvArgs {
-  const Cx<T>* src;    // [output of this launch][block][Sy][CB]
+  const Cx<T>* src;   // [output of this launch][block][Sy][CB]
   T* out;
   int Sy, Sx, Wr;
-  int groups;          // CTAs per output
+  int groups;         // CTAs per output
   int nblk, lgcb;
-  int l0, k0, nk;      // output index t of the launch: l = l0 + t / nk, k = k0 + t % nk
+  int l0, k0, nk;     // output index t of the launch: l = l0 + t / nk, k = k0 + t % nk
   long long o_l, o_k;
   T scale_hi, scale_lo;
-  const Cx<T>* tw;
+  const void* tw;
 };
 
-// Row kernels: one transform (a row pair) on N / R3 threads, Q of them per CTA.
+// Row kernels: a transform (NV row pairs) on TP threads, Q of them per CTA.
 template <int N>
 struct RowCfg {
-  static constexpr int TF = N / Len<N>::R3;
-  static constexpr int fit(int q) { return 2 * q * TF <= 320 ? fit(2 * q) : q; }
-  static constexpr int Q = fit(1);
-  static constexpr int threads = Q * TF;
-  static constexpr int FS = Len<N>::rows + (21 - Len<N>::rows % 16) % 16;  // = 5 mod 16: transforms on different banks
-  template <typename T>
-  static constexpr int smem() {
-    return Q * FS * (int)sizeof(Cx<T>);
+  using L = RowPasses<N>;
+  static constexpr int TP = L::TF / 2;
+  // 64 to 128 threads, the count that leaves the fewest lanes of the last
+  // warp idle (small CTAs overlap one's loads with another's passes: 64
+  // threads measured 34 us against 47 with 256 at 64 outputs of 511x511)
+  static constexpr int idle(int q) { return ((q * TP + 31) / 32 * 32 - q * TP) * 128 / (q * TP); }
+  static constexpr int pick() {
+    int best = 0;
+    for (int q = 1; q == 1 || q * TP <= 128; ++q)
+      if (best == 0 || best * TP < 64 || idle(q) < idle(best))
+        if (best == 0 || best * TP < 64 || q * TP <= 128) best = q;
+    return best;
   }
+  static constexpr int Q = pick();
+  static constexpr int threads = Q * TP;
+  static constexpr int min_ctas = 512 / threads;  // up to 128 registers a thread
+  static constexpr int FS = L::rows | 1;
+  static constexpr int smem = Q * FS * 16;
 };
 
-template <typename C>
-struct alignas(16) Vec16 {  // 16 bytes of complex values
-  static constexpr int V = 16 / (int)sizeof(C);
-  C v[V];
-};
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void pdl_launch() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
-// The middle pass of a three-pass transform, in place.
-template <typename T, int S, int N, int STEP>
-__device__ __forceinline__ void mid_pass(Cx<T>* z, int it0, int step, const Cx<T>* __restrict__ tw) {
-  using L = Len<N>;
-  using C = Cx<T>;
-  for (int it = it0; it < N / L::R2; it += step) {
-    const int b = it / L::R3, o = it - b * L::R3;
-    C* base = z + (b * L::P1 + o) * STEP;
-    C x[L::R2];
-    if (S < 0) {
-#pragma unroll
-      for (int m = 0; m < L::R2; ++m) x[m] = base[m * L::PR * STEP];
-      Dft<T, S, L::R2>::run(x);
-      base[0] = x[0];
-#pragma unroll
-      for (int q = 1; q < L::R2; ++q)
-        base[q * L::PR * STEP] = cmul<false>(x[q], __ldg(tw + L::tw2 + (q - 1) * L::R3 + o));
-    } else {
-      x[0] = base[0];
-#pragma unroll
-      for (int q = 1; q < L::R2; ++q)
-        x[q] = cmul<true>(base[q * L::PR * STEP], __ldg(tw + L::tw2 + (q - 1) * L::R3 + o));
-      Dft<T, S, L::R2>::run(x);
-#pragma unroll
-      for (int m = 0; m < L::R2; ++m) base[m * L::PR * STEP] = x[m];
-    }
-  }
+// Loads of what an earlier kernel of the chain wrote.  Not __ldg: the compiler
+// may move a non-coherent load above the wait for that kernel; volatile
+// assembly stays below it.
+__device__ __forceinline__ float ld(const float* g) {
+  float v;
+  asm volatile("ld.global.f32 %0, [%1];" : "=f"(v) : "l"(g));
+  return v;
+}
+__device__ __forceinline__ double ld(const double* g) {
+  double v;
+  asm volatile("ld.global.f64 %0, [%1];" : "=d"(v) : "l"(g));
+  return v;
+}
+__device__ __forceinline__ float2 ld(const float2* g) {
+  float2 v;
+  asm volatile("ld.global.v2.f32 {%0, %1}, [%2];" : "=f"(v.x), "=f"(v.y) : "l"(g));
+  return v;
+}
+__device__ __forceinline__ float4 ld(const float4* g) {
+  float4 v;
+  asm volatile("ld.global.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "l"(g));
+  return v;
+}
+__device__ __forceinline__ double2 ld(const double2* g) {
+  double2 v;
+  asm volatile("ld.global.v2.f64 {%0, %1}, [%2];" : "=d"(v.x), "=d"(v.y) : "l"(g));
+  return v;
+}
+__device__ __forceinline__ Cp<f2> ld(const Cp<f2>* g) {
+  Cp<f2> v;
+  asm volatile("ld.global.v2.b64 {%0, %1}, [%2];" : "=l"(v.x.v), "=l"(v.y.v) : "l"(g));
+  return v;
+}
+__device__ __forceinline__ Cp<double> ld(const Cp<double>* g) {
+  const double2 v = ld(reinterpret_cast<const double2*>(g));
+  return {v.x, v.y};
 }
 
-template <typename T, int N>
-__global__ void __launch_bounds__(RowCfg<N>::threads) row_forward(const RowFwdArgs<T> p) {
-  using L = Len<N>;
-  using C = Cx<T>;
-  using V16 = Vec16<C>;
-  constexpr int TF = RowCfg<N>::TF, Q = RowCfg<N>::Q, V = V16::V;
+__device__ __forceinline__ Cp<f2> gather(const float* v) { return {pack(v[0], v[2]), pack(v[1], v[3])}; }
+__device__ __forceinline__ Cp<double> gather(const double* v) { return {v[0], v[1]}; }
+
+template <typename S, int N>
+__global__ void __launch_bounds__(RowCfg<N>::threads, RowCfg<N>::min_ctas) row_forward(const RowFwdArgs<typename Sc<S>::real> p) {
+  using L = RowPasses<N>;
+  using C = Cp<S>;
+  using T = typename Sc<S>::real;
+  constexpr int TP = RowCfg<N>::TP, Q = RowCfg<N>::Q, NV = Sc<S>::NV;
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  C* s = reinterpret_cast<C*>(smem_raw);
+  pdl_launch();
+  const C* __restrict__ tw = static_cast<const C*>(p.tw);
   const bool first = blockIdx.x < p.a_blocks;
   const unsigned b = first ? blockIdx.x : blockIdx.x - p.a_blocks;
   const int H = first ? p.a.H : p.b.H, W = first ? p.a.W : p.b.W;
   const unsigned groups = (unsigned)(first ? p.a.groups : p.b.groups);
-  const T* __restrict__ src = first ? p.a.src : p.b.src;
-  C* __restrict__ dst = first ? p.a.dst : p.b.dst;
-  const long long mat = b / groups;
-  const int rp0 = (int)(b - (unsigned)mat * groups) * Q;
-  const int f = threadIdx.x / TF, i = threadIdx.x - f * TF;
-  C* z = s + f * RowCfg<N>::FS;
-  {
-    const int row = 2 * (rp0 + f);
-    const int w0 = row < H ? W : 0, w1 = row + 1 < H ? W : 0;
-    const T* r0 = src + (mat * H + (row < H ? row : 0)) * (long long)W;
-    const T* r1 = r0 + (row + 1 < H ? W : 0);
-    if (i < L::S1) {
-      C x[L::R1];
+  const unsigned mat = b / groups;
+  const int f = threadIdx.x / TP, i = threadIdx.x - f * TP;
+  const int row0 = (int)((b - mat * groups) * Q + f) * (2 * NV);
+  C* z = reinterpret_cast<C*>(smem_raw) + f * RowCfg<N>::FS;
+  const T* __restrict__ src = (first ? p.a.src : p.b.src) + (long long)mat * H * W;
+  const T* r[2 * NV];
 #pragma unroll
-      for (int m = 0; m < L::R1; ++m) {
-        const int k = i + m * L::S1;
-        x[m] = mk<T>(k < w0 ? __ldg(r0 + k) : T(0), k < w1 ? __ldg(r1 + k) : T(0));
-      }
-      Dft<T, -1, L::R1>::run(x);
-      C* base = z + (L::three ? (i / L::R3) * L::PR + i % L::R3 : i);
-      base[0] = x[0];
+  for (int j = 0; j < 2 * NV; ++j) r[j] = row0 + j < H ? src + (long long)(row0 + j) * W : p.zeros;
+  pdl_wait();
+  for (int o = i; o < L::S1; o += TP) {
+    C x[L::R1];
 #pragma unroll
-      for (int q = 1; q < L::R1; ++q) base[q * L::P1] = cmul<false>(x[q], __ldg(p.tw + (q - 1) * L::S1 + i));
+    for (int m = 0; m < L::R1; ++m) {
+      const int k = o + m * L::S1;
+      T v[2 * NV];
+#pragma unroll
+      for (int j = 0; j < 2 * NV; ++j) v[j] = k < W ? ld(r[j] + k) : T(0);
+      x[m] = gather(v);
     }
+    Dft<S, -1, L::R1>::run(x);
+    C* base = z + L::in_block(o);
+    base[0] = x[0];
+#pragma unroll
+    for (int q = 1; q < L::R1; ++q) base[q * L::P1] = cmul<false>(x[q], tw[(q - 1) * L::S1 + o]);
   }
   __syncthreads();
-  if constexpr (L::three) {
-    mid_pass<T, -1, N, 1>(z, i, TF, p.tw);
-    __syncthreads();
-  }
+  mid_passes<S, -1, false, L, 1>(z, i, TP, tw);
+  if (row0 >= H) return;
+  // Last pass of items i and TF - i (thread 0: items 0 and TF / 2), whose
+  // outputs pair up as k and N - k: for thread 0 within each item.
+  const bool t0 = i == 0;
+  const int iy = t0 ? L::TF / 2 : L::TF - i;
+  C x[L::R3], y[L::R3];
   {
-    const int q1 = i % L::R1, q2 = i / L::R1;
-    C x[L::R3];
-    const C* base = z + q1 * L::P1 + q2 * L::PR;
+    const C* bx = z + L::last_item(i);
+    const C* by = z + L::last_item(iy);
 #pragma unroll
-    for (int m = 0; m < L::R3; ++m) x[m] = base[m];
-    Dft<T, -1, L::R3>::run(x);
-    __syncthreads();
-#pragma unroll
-    for (int q = 0; q < L::R3; ++q) z[i + q * TF] = x[q];  // natural order
-  }
-  __syncthreads();
-  // The two rows' spectra: A = (Z[c] + conj Z[-c]) / 2, B = (Z[c] - conj Z[-c]) / 2i.
-  const int cb = 1 << p.lgcb, lgh = p.lgcb - (V == 2 ? 1 : 0);
-  const int total = p.nblk * (Q << lgh);
-  dst += mat * p.nblk * (long long)H * cb;
-  for (int u = threadIdx.x; u < total; u += Q * TF) {
-    const int h = u & ((1 << lgh) - 1), ff = (u >> lgh) % Q, blk = (u >> lgh) / Q;
-    const int row = 2 * (rp0 + ff);
-    if (row >= H) continue;
-    const C* zz = s + ff * RowCfg<N>::FS;
-    V16 a, bb;
-#pragma unroll
-    for (int v = 0; v < V; ++v) {
-      const int c = blk * cb + h * V + v;
-      const C zc = zz[c], zn = zz[c == 0 ? 0 : N - c];
-      a.v[v] = mk<T>(T(0.5) * (zc.x + zn.x), T(0.5) * (zc.y - zn.y));
-      bb.v[v] = mk<T>(T(0.5) * (zc.y + zn.y), T(0.5) * (zn.x - zc.x));
+    for (int m = 0; m < L::R3; ++m) {
+      x[m] = bx[m];
+      y[m] = by[m];
     }
-    C* d = dst + ((long long)blk * H + row) * cb + h * V;
-    *reinterpret_cast<V16*>(d) = a;
-    if (row + 1 < H) *reinterpret_cast<V16*>(d + cb) = bb;
+  }
+  Dft<S, -1, L::R3>::run(x);
+  Dft<S, -1, L::R3>::run(y);
+  // The two rows' spectra: A = (Z[k] + conj Z[-k]) / 2, B = (Z[k] - conj Z[-k]) / 2i.
+  const S half = Sc<S>::bc(0.5);
+  S hs = half;
+  if constexpr (NV == 1) hs = T(0.5) * (first ? p.a.scale : p.b.scale);
+  const int cb = 1 << p.lgcb;
+  Cx<T>* dst = (first ? p.a.dst : p.b.dst) + ((long long)mat * p.nblk * H + row0) * cb;
+  const auto put = [&](int k, C zk, C zn) {
+    const C a = {mul(hs, add(zk.x, zn.x)), mul(hs, sub(zk.y, zn.y))};
+    const C bb = {mul(hs, add(zk.y, zn.y)), mul(hs, sub(zn.x, zk.x))};
+    Cx<T>* d = dst + (long long)(k >> p.lgcb) * H * cb + (k & (cb - 1));
+    if constexpr (NV == 2) {
+      *reinterpret_cast<float2*>(d) = make_float2(lo(a.x), lo(a.y));
+      if (row0 + 1 < H) *reinterpret_cast<float2*>(d + cb) = make_float2(lo(bb.x), lo(bb.y));
+      if (row0 + 2 < H) *reinterpret_cast<float2*>(d + 2 * cb) = make_float2(hi(a.x), hi(a.y));
+      if (row0 + 3 < H) *reinterpret_cast<float2*>(d + 3 * cb) = make_float2(hi(bb.x), hi(bb.y));
+    } else {
+      *reinterpret_cast<double2*>(d) = make_double2(a.x, a.y);
+      if (row0 + 1 < H) *reinterpret_cast<double2*>(d + cb) = make_double2(bb.x, bb.y);
+    }
+  };
+#pragma unroll
+  for (int q = 0; q < (L::R3 + 1) / 2; ++q)
+    put(i + q * L::TF, x[q], csel(t0, x[(L::R3 - q) % L::R3], y[L::R3 - 1 - q]));
+#pragma unroll
+  for (int q = 0; q < L::R3 / 2; ++q)
+    put(iy + q * L::TF, y[q], csel(t0, y[L::R3 - 1 - q], x[L::R3 - 1 - q]));
+  if (t0) {  // column N / 2, its own partner
+    const C h = L::R3 % 2 == 0 ? x[L::R3 / 2] : y[L::R3 / 2];
+    put(N / 2, h, h);
   }
 }
 
-template <typename T, int N>
-__global__ void __launch_bounds__(RowCfg<N>::threads) row_inverse(const RowInvArgs<T> p) {
-  using L = Len<N>;
-  using C = Cx<T>;
-  using V16 = Vec16<C>;
-  constexpr int TF = RowCfg<N>::TF, Q = RowCfg<N>::Q, V = V16::V;
+template <typename S, int N>
+__global__ void __launch_bounds__(RowCfg<N>::threads, RowCfg<N>::min_ctas) row_inverse(const RowInvArgs<typename Sc<S>::real> p) {
+  using L = RowPasses<N>;
+  using C = Cp<S>;
+  using T = typename Sc<S>::real;
+  constexpr int TP = RowCfg<N>::TP, Q = RowCfg<N>::Q, NV = Sc<S>::NV;
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  C* s = reinterpret_cast<C*>(smem_raw);
-  const int t = (int)(blockIdx.x / (unsigned)p.groups);
-  const int rp0 = (int)(blockIdx.x - (unsigned)t * (unsigned)p.groups) * Q;
-  // Z = A + i B of every row pair, whose inverse transform is row a + i row b
-  const int cb = 1 << p.lgcb, lgh = p.lgcb - (V == 2 ? 1 : 0);
-  const int total = p.nblk * (Q << lgh);
-  const C* src = p.src + (long long)t * p.nblk * p.Sy * cb;
-#pragma unroll 4
-  for (int u = threadIdx.x; u < total; u += Q * TF) {
-    const int h = u & ((1 << lgh) - 1), ff = (u >> lgh) % Q, blk = (u >> lgh) / Q;
-    const int row = 2 * (rp0 + ff);
-    V16 a, bb;
+  pdl_launch();
+  const C* __restrict__ tw = static_cast<const C*>(p.tw);
+  const unsigned t = blockIdx.x / (unsigned)p.groups;
+  const int f = threadIdx.x / TP, i = threadIdx.x - f * TP;
+  const int row0 = (int)((blockIdx.x - t * (unsigned)p.groups) * Q + f) * (2 * NV);
+  C* z = reinterpret_cast<C*>(smem_raw) + f * RowCfg<N>::FS;
+  const int cb = 1 << p.lgcb;
+  const Cx<T>* __restrict__ src = p.src + ((long long)t * p.nblk * p.Sy + row0) * cb;
+  const bool v0 = row0 < p.Sy, v1 = row0 + 1 < p.Sy, v2 = row0 + 2 < p.Sy, v3 = row0 + 3 < p.Sy;
+  // rows A and B of each row pair at column c
+  const auto get = [&](int c, C* a, C* b) {
+    const Cx<T>* d = src + (long long)(c >> p.lgcb) * p.Sy * cb + (c & (cb - 1));
+    if constexpr (NV == 2) {
+      const float2 o = make_float2(0.f, 0.f);
+      const float2 e0 = v0 ? ld(reinterpret_cast<const float2*>(d)) : o;
+      const float2 e1 = v1 ? ld(reinterpret_cast<const float2*>(d + cb)) : o;
+      const float2 e2 = v2 ? ld(reinterpret_cast<const float2*>(d + 2 * cb)) : o;
+      const float2 e3 = v3 ? ld(reinterpret_cast<const float2*>(d + 3 * cb)) : o;
+      *a = {pack(e0.x, e2.x), pack(e0.y, e2.y)};
+      *b = {pack(e1.x, e3.x), pack(e1.y, e3.y)};
+    } else {
+      const double2 o = make_double2(0.0, 0.0);
+      const double2 e0 = v0 ? ld(reinterpret_cast<const double2*>(d)) : o;
+      const double2 e1 = v1 ? ld(reinterpret_cast<const double2*>(d + cb)) : o;
+      *a = {e0.x, e0.y};
+      *b = {e1.x, e1.y};
+    }
+  };
+  pdl_wait();
+  // Z = A + i B, Z[N - c] = conj A + i conj B: the inverse transform of Z is
+  // row a + i row b.  First pass of items o and S1 - o (o = 0: items 0 and
+  // S1 / 2), which use the same columns.
+  for (int o = i; o < L::S1 / 2; o += TP) {
+    const bool o0 = o == 0;
+    const int oy = o0 ? L::S1 / 2 : L::S1 - o;
+    constexpr int M = L::R1 / 2;
+    C x[L::R1], y[L::R1];
+    C cx[M], cy[M];  // the conjugate columns' values
 #pragma unroll
-    for (int v = 0; v < V; ++v) a.v[v] = bb.v[v] = mk<T>(T(0), T(0));
-    const C* d = src + ((long long)blk * p.Sy + row) * cb + h * V;
-    if (row < p.Sy) a = *reinterpret_cast<const V16*>(d);
-    if (row + 1 < p.Sy) bb = *reinterpret_cast<const V16*>(d + cb);
-    C* zz = s + ff * RowCfg<N>::FS;
+    for (int m = 0; m < M; ++m) {
+      C a, b;
+      get(o + m * L::S1, &a, &b);
+      x[m] = cadd_i<1>(a, b);
+      cx[m] = {add(a.x, b.y), sub(b.x, a.y)};
+      if (m == 0 && o0) x[0] = {a.x, b.x};  // column 0 is real
+      get(oy + m * L::S1, &a, &b);
+      y[m] = cadd_i<1>(a, b);
+      cy[m] = {add(a.x, b.y), sub(b.x, a.y)};
+    }
 #pragma unroll
-    for (int v = 0; v < V; ++v) {
-      const int c = blk * cb + h * V + v;
-      if (c > N / 2) continue;
-      if (c == 0 || c == N / 2) {
-        zz[L::pos(c)] = mk<T>(a.v[v].x, bb.v[v].x);
-      } else {
-        zz[L::pos(c)] = mk<T>(a.v[v].x - bb.v[v].y, a.v[v].y + bb.v[v].x);
-        zz[L::pos(N - c)] = mk<T>(a.v[v].x + bb.v[v].y, bb.v[v].x - a.v[v].y);
-      }
+    for (int m = M; m < L::R1; ++m) {
+      x[m] = m == M ? cy[M - 1] : csel(o0, cx[m == M ? 0 : L::R1 - m], cy[L::R1 - 1 - m]);
+      y[m] = csel(o0, cy[L::R1 - 1 - m], cx[L::R1 - 1 - m]);
+    }
+    if (o0) {  // column N / 2 is real
+      C a, b;
+      get(N / 2, &a, &b);
+      x[M] = {a.x, b.x};
+    }
+    Dft<S, 1, L::R1>::run(x);
+    Dft<S, 1, L::R1>::run(y);
+    C* bx = z + L::in_block(o);
+    C* by = z + L::in_block(oy);
+    bx[0] = x[0];
+    by[0] = y[0];
+#pragma unroll
+    for (int q = 1; q < L::R1; ++q) {
+      bx[q * L::P1] = cmul<true>(x[q], tw[(q - 1) * L::S1 + o]);
+      by[q * L::P1] = cmul<true>(y[q], tw[(q - 1) * L::S1 + oy]);
     }
   }
   __syncthreads();
-  const int f = threadIdx.x / TF, i = threadIdx.x - f * TF;
-  C* z = s + f * RowCfg<N>::FS;
-  if (i < L::S1) {
-    C x[L::R1];
-    C* base = z + (L::three ? (i / L::R3) * L::PR + i % L::R3 : i);
+  mid_passes<S, 1, false, L, 1>(z, i, TP, tw);
+  if (!v0) return;
+  const int l = p.l0 + (int)t / p.nk, k = p.k0 + (int)t % p.nk;
+  T* o0 = p.out + ((l * p.o_l + k * p.o_k) * p.Sy + row0) * (long long)p.Sx;
 #pragma unroll
-    for (int m = 0; m < L::R1; ++m) x[m] = base[m * L::P1];
-    Dft<T, 1, L::R1>::run(x);
-    base[0] = x[0];
-#pragma unroll
-    for (int q = 1; q < L::R1; ++q) base[q * L::P1] = cmul<true>(x[q], __ldg(p.tw + (q - 1) * L::S1 + i));
-  }
-  __syncthreads();
-  if constexpr (L::three) {
-    // decimation in frequency with the conjugate twiddles
-    for (int it = i; it < N / L::R2; it += TF) {
-      const int b = it / L::R3, o = it - b * L::R3;
-      C* base = z + b * L::P1 + o;
-      C x[L::R2];
-#pragma unroll
-      for (int m = 0; m < L::R2; ++m) x[m] = base[m * L::PR];
-      Dft<T, 1, L::R2>::run(x);
-      base[0] = x[0];
-#pragma unroll
-      for (int q = 1; q < L::R2; ++q)
-        base[q * L::PR] = cmul<true>(x[q], __ldg(p.tw + L::tw2 + (q - 1) * L::R3 + o));
-    }
-    __syncthreads();
-  }
-  {
-    const int q1 = i % L::R1, q2 = i / L::R1;
+  for (int u = 0; u < 2; ++u) {
+    const int it = i + u * TP;
     C x[L::R3];
-    const C* base = z + q1 * L::P1 + q2 * L::PR;
+    const C* base = z + L::last_item(it);
 #pragma unroll
     for (int m = 0; m < L::R3; ++m) x[m] = base[m];
-    Dft<T, 1, L::R3>::run(x);
-    const int row = 2 * (rp0 + f);
-    if (row >= p.Sy) return;
-    const int l = p.l0 + t / p.nk, k = p.k0 + t % p.nk;
-    T* o0 = p.out + ((l * p.o_l + k * p.o_k) * p.Sy + row) * (long long)p.Sx;
-    const bool two = row + 1 < p.Sy;
+    Dft<S, 1, L::R3>::run(x);
 #pragma unroll
     for (int q = 0; q < L::R3; ++q) {
-      int sx = i + q * TF + p.Wr - 1;
+      int sx = it + q * L::TF + p.Wr - 1;
       if (sx >= N) sx -= N;
       if (sx >= p.Sx) continue;
-      // the scale as a sum of two terms: rounds like a scaling in higher precision
-      T va, vb;
-      if constexpr (sizeof(T) == 4) {
-        va = fmaf(x[q].x, p.scale_hi, x[q].x * p.scale_lo);
-        vb = fmaf(x[q].y, p.scale_hi, x[q].y * p.scale_lo);
+      T* d = o0 + sx;
+      if constexpr (NV == 2) {
+        // the scale as a sum of two terms: rounds like a scaling in higher precision
+        const f2 sh = pack(p.scale_hi, p.scale_hi), sl = pack(p.scale_lo, p.scale_lo);
+        const f2 a = fma(x[q].x, sh, mul(x[q].x, sl)), b = fma(x[q].y, sh, mul(x[q].y, sl));
+        d[0] = lo(a);
+        if (v1) d[p.Sx] = lo(b);
+        if (v2) d[2 * (long long)p.Sx] = hi(a);
+        if (v3) d[3 * (long long)p.Sx] = hi(b);
       } else {
-        va = x[q].x * p.scale_hi;
-        vb = x[q].y * p.scale_hi;
+        d[0] = x[q].x;
+        if (v1) d[p.Sx] = x[q].y;
       }
-      o0[sx] = va;
-      if (two) o0[p.Sx + sx] = vb;
     }
   }
 }
 
 // ---------------------------------------------------------------------------
 // Column kernels: a unit is one block of CB columns of one matrix (or pair),
-// on TU threads, lanes over the block's columns first; PU units per CTA.
+// on TU threads, lanes over the block's columns (NV at a time) first; PU
+// units per CTA.
 // ---------------------------------------------------------------------------
-template <typename T, int N>
+template <typename S, int N>
 struct ColCfg {
-  static constexpr int CB = sizeof(T) == 4 ? (N <= 2048 ? 4 : 2) : 2;
+  using L = ColPasses<N>;
+  static constexpr int CB = Sc<S>::NV == 2 ? (N <= 2048 ? 4 : 2) : 2;
   static constexpr int lgcb = CB == 4 ? 2 : 1;
-  static constexpr int TU = (N / Len<N>::R3) * CB <= 512 ? (N / Len<N>::R3) * CB : (N / Len<N>::R1) * CB;
-  static constexpr int PU = TU >= 128 ? 1 : 128 / TU;
+  static constexpr int LC = CB / Sc<S>::NV;  // lanes across a block's columns
+  // Items a pass runs side by side: the count that issues the fewest lane
+  // slots over the passes (a pass of n items takes ceil(n / JT) rounds of JT
+  // lanes; FP64 pays for idle lanes as for busy ones: at 128 points, 16
+  // against 8 of 16 lanes busy in the radix-16 pass).
+  static constexpr int slots(int jt) {
+    int c = 0;
+    for (int r : {L::R1, L::Ra, L::R3})
+      if (r > 1) c += (N / r + jt - 1) / jt * jt * r;
+    return c;
+  }
+  static constexpr int best(int a, int b) {
+    return a * LC > 256 ? b : b * LC > 256 ? a : slots(a) <= slots(b) ? a : b;
+  }
+  static constexpr int JT = best(L::TF, best(L::Ra > 1 ? N / L::Ra : L::S1, L::S1));
+  static constexpr int TU = JT * LC;
+  static constexpr int PU = TU >= 128 ? 1 : (127 + TU) / TU;
   static constexpr int threads = TU * PU;
-  static constexpr int JT = TU / CB;             // items side by side in a pass
-  static constexpr int unit = Len<N>::rows * CB;  // shared-memory elements of a unit
-  static constexpr int nblk = (N / 2 + 1 + CB - 1) / CB;  // blocks when N is the row length (callers pass theirs)
+  // 64 registers a thread while no radix exceeds 8, else 128
+  static constexpr int min_ctas = (L::R1 <= 8 ? 1024 : 512) / threads;
+  static constexpr int unit = L::rows * LC;        // shared-memory elements of a unit
 };
 
-// Forward passes of one column block from global memory (H rows of CB
-// columns) up to, not including, the last; ends with a barrier.
-template <typename T, int N>
-__device__ __forceinline__ void col_load_passes(Cx<T>* z, const Cx<T>* __restrict__ g, int H, int j0, int c,
-                                                const Cx<T>* __restrict__ tw) {
-  using L = Len<N>;
-  using C = Cx<T>;
-  using K = ColCfg<T, N>;
+// A thread's columns of one row of a block.
+__device__ __forceinline__ Cp<f2> load_row(const Cx<float>* g) {
+  const float4 v = ld(reinterpret_cast<const float4*>(g));
+  return {pack(v.x, v.z), pack(v.y, v.w)};
+}
+__device__ __forceinline__ Cp<double> load_row(const Cx<double>* g) {
+  const double2 v = ld(reinterpret_cast<const double2*>(g));
+  return {v.x, v.y};
+}
+__device__ __forceinline__ void store_row(Cx<float>* g, Cp<f2> v) {
+  *reinterpret_cast<float4*>(g) = make_float4(lo(v.x), lo(v.y), hi(v.x), hi(v.y));
+}
+__device__ __forceinline__ void store_row(Cx<double>* g, Cp<double> v) {
+  *reinterpret_cast<double2*>(g) = make_double2(v.x, v.y);
+}
+
+// Forward passes of one column block from global memory (H rows; g points at
+// the thread's columns) up to, not including, the last; ends with a barrier.
+template <typename S, int N>
+__device__ __forceinline__ void col_load_passes(Cp<S>* z, const Cx<typename Sc<S>::real>* __restrict__ g, int H,
+                                                int j0, const Cp<S>* __restrict__ tw) {
+  using L = ColPasses<N>;
+  using K = ColCfg<S, N>;
   for (int o = j0; o < L::S1; o += K::JT) {
-    C x[L::R1];
+    Cp<S> x[L::R1];
 #pragma unroll
     for (int m = 0; m < L::R1; ++m) {
       const int y = o + m * L::S1;
-      x[m] = y < H ? __ldg(g + (long long)y * K::CB + c) : mk<T>(T(0), T(0));
+      x[m] = y < H ? load_row(g + (long long)y * K::CB) : czero<S>();
     }
-    Dft<T, -1, L::R1>::run(x);
-    C* base = z + (L::three ? (o / L::R3) * L::PR + o % L::R3 : o) * K::CB + c;
+    Dft<S, -1, L::R1>::run(x);
+    Cp<S>* base = z + L::in_block(o) * K::LC;
     base[0] = x[0];
 #pragma unroll
-    for (int q = 1; q < L::R1; ++q) base[q * L::P1 * K::CB] = cmul<false>(x[q], __ldg(tw + (q - 1) * L::S1 + o));
+    for (int q = 1; q < L::R1; ++q) base[q * L::P1 * K::LC] = cmul<false>(x[q], tw[(q - 1) * L::S1 + o]);
   }
   __syncthreads();
-  if constexpr (L::three) {
-    mid_pass<T, -1, N, K::CB>(z + c, j0, K::JT, tw);
-    __syncthreads();
-  }
+  mid_passes<S, -1, false, L, K::LC>(z, j0, K::JT, tw);
 }
 
-// Place of the last pass's item j (its R3 values follow each other by CB).
-template <typename T, int N>
+// Place of the last pass's item j in shared memory: the item order of the
+// column kernels (lanes over the middle digit) keeps neighbouring lanes an odd
+// number of elements apart.
+template <typename S, int N>
 __device__ __forceinline__ int col_item(int j) {
-  using L = Len<N>;
-  const int q1 = j / L::R2, q2 = j - q1 * L::R2;
-  return (q1 * L::P1 + q2 * L::PR) * ColCfg<T, N>::CB;
+  using L = ColPasses<N>;
+  const int q1 = j / L::Ra, qa = j - q1 * L::Ra;
+  return (q1 * L::P1 + qa * L::Pa) * ColCfg<S, N>::LC;
 }
 
-// Full spectra of the columns, in pass order: row q N/R3 + j holds output q
-// of the last pass's item j.
-template <typename T, int N>
-__global__ void __launch_bounds__(ColCfg<T, N>::threads) col_forward(const ColFwdArgs<T> p) {
-  using L = Len<N>;
-  using C = Cx<T>;
-  using K = ColCfg<T, N>;
+// Full spectra of the columns, in pass order: element (q TF + j) LC + lane
+// holds output q of the last pass's item j.
+template <typename S, int N>
+__global__ void __launch_bounds__(ColCfg<S, N>::threads, ColCfg<S, N>::min_ctas) col_forward(const ColFwdArgs<typename Sc<S>::real> p) {
+  using L = ColPasses<N>;
+  using C = Cp<S>;
+  using K = ColCfg<S, N>;
   extern __shared__ __align__(16) unsigned char smem_raw[];
+  pdl_launch();
+  const C* __restrict__ tw = static_cast<const C*>(p.tw);
   const int pu = threadIdx.x / K::TU, t = threadIdx.x - pu * K::TU;
-  const int c = t % K::CB, j0 = t / K::CB;
-  C* z = reinterpret_cast<C*>(smem_raw) + pu * K::unit;
+  const int c = t % K::LC, j0 = t / K::LC;
+  C* z = reinterpret_cast<C*>(smem_raw) + pu * K::unit + c;
   const long long u = (long long)blockIdx.x * K::PU + pu;
   const bool live = u < p.units;
-  col_load_passes<T, N>(z, p.src + (live ? u : 0) * p.H * K::CB, live ? p.H : 0, j0, c, p.tw);
+  pdl_wait();
+  col_load_passes<S, N>(z, p.src + (live ? u : 0) * p.H * K::CB + c * Sc<S>::NV, live ? p.H : 0, j0, tw);
   if (!live) return;
-  C* dst = p.dst + u * N * K::CB + c;
-  for (int j = j0; j < N / L::R3; j += K::JT) {
+  C* dst = static_cast<C*>(p.dst) + u * N * K::LC + c;
+  for (int j = j0; j < L::TF; j += K::JT) {
     C x[L::R3];
-    const C* base = z + col_item<T, N>(j) + c;
+    const C* base = z + col_item<S, N>(j);
 #pragma unroll
-    for (int m = 0; m < L::R3; ++m) x[m] = base[m * K::CB];
-    Dft<T, -1, L::R3>::run(x);
+    for (int m = 0; m < L::R3; ++m) x[m] = base[m * K::LC];
+    Dft<S, -1, L::R3>::run(x);
 #pragma unroll
-    for (int q = 0; q < L::R3; ++q) dst[(q * (N / L::R3) + j) * K::CB] = x[q];
+    for (int q = 0; q < L::R3; ++q) dst[(q * L::TF + j) * K::LC] = x[q];
   }
 }
 
@@ -681,39 +920,43 @@ __global__ void __launch_bounds__(ColCfg<T, N>::threads) col_forward(const ColFw
 // the product with the left spectrum (LPRE: read from global memory;
 // otherwise transformed once per group and kept in shared memory), and the
 // inverse transform, whose rows go out in the output's row order.
-template <typename T, int N, bool LPRE, bool RPRE>
-__global__ void __launch_bounds__(ColCfg<T, N>::threads) col_pairs(const ColArgs<T> p) {
-  using L = Len<N>;
-  using C = Cx<T>;
-  using K = ColCfg<T, N>;
+template <typename S, int N, bool LPRE, bool RPRE>
+__global__ void __launch_bounds__(ColCfg<S, N>::threads, ColCfg<S, N>::min_ctas) col_pairs(const ColArgs<typename Sc<S>::real> p) {
+  using L = ColPasses<N>;
+  using C = Cp<S>;
+  using K = ColCfg<S, N>;
+  using G = Cx<typename Sc<S>::real>;
+  constexpr int NV = Sc<S>::NV;
   extern __shared__ __align__(16) unsigned char smem_raw[];
+  pdl_launch();
+  const C* __restrict__ tw = static_cast<const C*>(p.tw);
   const int pu = threadIdx.x / K::TU, t = threadIdx.x - pu * K::TU;
-  const int c = t % K::CB, j0 = t / K::CB;
-  C* z = reinterpret_cast<C*>(smem_raw) + pu * K::unit;
+  const int c = t % K::LC, j0 = t / K::LC;
+  C* z = reinterpret_cast<C*>(smem_raw) + pu * K::unit + c;
   C* zl = z + (LPRE ? 0 : K::PU * K::unit);  // left spectrum
-  const long long gu = (long long)blockIdx.x * K::PU + pu;
-  const int blk = (int)(gu % p.nblk);
-  const long long rest = gu / p.nblk;
-  const int kg = (int)(rest % p.n_kg);
-  const long long ll = rest / p.n_kg;  // left of this launch
+  const unsigned gu = blockIdx.x * K::PU + pu;
+  const unsigned blk = gu % (unsigned)p.nblk, rest = gu / (unsigned)p.nblk;
+  const int kg = (int)(rest % (unsigned)p.n_kg);
+  const int ll = (int)(rest / (unsigned)p.n_kg);  // left of this launch
   const bool live = ll < p.n_left;
   const long long l = p.l0 + (live ? ll : 0);
   const int ka = p.k0 + kg * p.kc, nk = live ? min(p.kc, p.k1 - ka) : 0;
-  constexpr int NJ = N / L::R3;
   const C* lspec = nullptr;
+  pdl_wait();
   if constexpr (LPRE) {
-    lspec = p.left + (l * p.nblk + blk) * (long long)N * K::CB + c;
+    lspec = static_cast<const C*>(p.left) + (l * p.nblk + blk) * (long long)N * K::LC + c;
   } else {
-    col_load_passes<T, N>(zl, p.left + (l * p.nblk + blk) * (long long)p.Hl * K::CB, live ? p.Hl : 0, j0, c, p.tw);
+    col_load_passes<S, N>(zl, static_cast<const G*>(p.left) + (l * p.nblk + blk) * (long long)p.Hl * K::CB + c * NV,
+                          live ? p.Hl : 0, j0, tw);
     // each thread reads back the items it writes here: no barrier needed
-    for (int j = j0; j < NJ; j += K::JT) {
+    for (int j = j0; j < L::TF; j += K::JT) {
       C x[L::R3];
-      C* base = zl + col_item<T, N>(j) + c;
+      C* base = zl + col_item<S, N>(j);
 #pragma unroll
-      for (int m = 0; m < L::R3; ++m) x[m] = base[m * K::CB];
-      Dft<T, -1, L::R3>::run(x);
+      for (int m = 0; m < L::R3; ++m) x[m] = base[m * K::LC];
+      Dft<S, -1, L::R3>::run(x);
 #pragma unroll
-      for (int m = 0; m < L::R3; ++m) base[m * K::CB] = x[m];
+      for (int m = 0; m < L::R3; ++m) base[m * K::LC] = x[m];
     }
   }
   const long long n_k = p.k1 - p.k0;
@@ -722,50 +965,43 @@ __global__ void __launch_bounds__(ColCfg<T, N>::threads) col_pairs(const ColArgs
     const bool act = kk < nk;
     const long long r = act ? l * p.r_l + k * p.r_k - p.r_off : 0;
     if constexpr (!RPRE)
-      col_load_passes<T, N>(z, p.right + (r * p.nblk + blk) * (long long)p.Hr * K::CB, act ? p.Hr : 0, j0, c, p.tw);
-    for (int j = j0; j < NJ; j += K::JT) {
+      col_load_passes<S, N>(z, static_cast<const G*>(p.right) + (r * p.nblk + blk) * (long long)p.Hr * K::CB + c * NV,
+                            act ? p.Hr : 0, j0, tw);
+    for (int j = j0; j < L::TF; j += K::JT) {
       C x[L::R3];
-      C* base = z + col_item<T, N>(j) + c;
-      C lv[L::R3];
-      if constexpr (LPRE) {
-#pragma unroll
-        for (int q = 0; q < L::R3; ++q) lv[q] = __ldg(lspec + (q * NJ + j) * K::CB);
-      }
+      C* base = z + col_item<S, N>(j);
       if constexpr (RPRE) {
-        const C* rspec = p.right + (r * p.nblk + blk) * (long long)N * K::CB + c;
+        const C* rspec = static_cast<const C*>(p.right) + (r * p.nblk + blk) * (long long)N * K::LC + c;
 #pragma unroll
-        for (int q = 0; q < L::R3; ++q) x[q] = __ldg(rspec + (q * NJ + j) * K::CB);
+        for (int q = 0; q < L::R3; ++q) x[q] = ld(rspec + (q * L::TF + j) * K::LC);
       } else {
 #pragma unroll
-        for (int m = 0; m < L::R3; ++m) x[m] = base[m * K::CB];
-        Dft<T, -1, L::R3>::run(x);
+        for (int m = 0; m < L::R3; ++m) x[m] = base[m * K::LC];
+        Dft<S, -1, L::R3>::run(x);
       }
-      const C* lb = zl + col_item<T, N>(j) + c;
+      const C* lb = zl + col_item<S, N>(j);
 #pragma unroll
-      for (int q = 0; q < L::R3; ++q) x[q] = cmul<true>(LPRE ? lv[q] : lb[q * K::CB], x[q]);
-      Dft<T, 1, L::R3>::run(x);
+      for (int q = 0; q < L::R3; ++q) x[q] = cmul<true>(LPRE ? ld(lspec + (q * L::TF + j) * K::LC) : lb[q * K::LC], x[q]);
+      Dft<S, 1, L::R3>::run(x);
 #pragma unroll
-      for (int m = 0; m < L::R3; ++m) base[m * K::CB] = x[m];
+      for (int m = 0; m < L::R3; ++m) base[m * K::LC] = x[m];
     }
     __syncthreads();
-    if constexpr (L::three) {
-      mid_pass<T, 1, N, K::CB>(z + c, j0, K::JT, p.tw);
-      __syncthreads();
-    }
+    mid_passes<S, 1, true, L, K::LC>(z, j0, K::JT, tw);
     if (act) {
-      C* out = p.out + ((ll * n_k + (k - p.k0)) * p.nblk + blk) * (long long)p.Sy * K::CB + c;
+      G* out = p.out + ((ll * n_k + (k - p.k0)) * p.nblk + blk) * (long long)p.Sy * K::CB + c * NV;
       for (int o = j0; o < L::S1; o += K::JT) {
         C x[L::R1];
-        const C* base = z + (L::three ? (o / L::R3) * L::PR + o % L::R3 : o) * K::CB + c;
+        const C* base = z + L::in_block(o) * K::LC;
         x[0] = base[0];
 #pragma unroll
-        for (int q = 1; q < L::R1; ++q) x[q] = cmul<true>(base[q * L::P1 * K::CB], __ldg(p.tw + (q - 1) * L::S1 + o));
-        Dft<T, 1, L::R1>::run(x);
+        for (int q = 1; q < L::R1; ++q) x[q] = cmul<true>(base[q * L::P1 * K::LC], tw[(q - 1) * L::S1 + o]);
+        Dft<S, 1, L::R1>::run(x);
 #pragma unroll
         for (int m = 0; m < L::R1; ++m) {
           int sy = o + m * L::S1 + p.Hr - 1;
           if (sy >= N) sy -= N;
-          if (sy < p.Sy) out[(long long)sy * K::CB] = x[m];
+          if (sy < p.Sy) store_row(out + (long long)sy * K::CB, x[m]);
         }
       }
     }
@@ -777,14 +1013,14 @@ __global__ void __launch_bounds__(ColCfg<T, N>::threads) col_pairs(const ColArgs
 struct RowKernels {
   const void* forward;
   const void* inverse;
-  int threads, q, smem;
+  int threads, q, nv, smem;
 };
 struct ColKernels {
   const void* forward;
   const void* pairs;       // left transformed in the kernel
   const void* pairs_lpre;  // left spectra from col_forward
   const void* pairs_pre;   // both
-  int threads, pu, lgcb, unit_smem;  // shared memory of one unit buffer
+  int threads, pu, lgcb, unit_smem;  // shared memory of one buffer
 };
 // false: no kernels for this length
 bool row_kernels_f32(int n, RowKernels* k);
@@ -792,18 +1028,18 @@ bool row_kernels_f64(int n, RowKernels* k);
 bool col_kernels_f32(int n, ColKernels* k);
 bool col_kernels_f64(int n, ColKernels* k);
 
-#define XC_ROW_CASE(N_, A_, B_, C_)                                                       \
-  case N_:                                                                                \
-    *k = RowKernels{(const void*)&row_forward<XC_FFT_T, N_>, (const void*)&row_inverse<XC_FFT_T, N_>, \
-                    RowCfg<N_>::threads, RowCfg<N_>::Q, RowCfg<N_>::smem<XC_FFT_T>()};    \
+#define XC_ROW_CASE(N_, ...)                                                                                       \
+  case N_:                                                                                                         \
+    *k = RowKernels{(const void*)&row_forward<XC_FFT_S, N_>, (const void*)&row_inverse<XC_FFT_S, N_>,               \
+                    RowCfg<N_>::threads, RowCfg<N_>::Q, Sc<XC_FFT_S>::NV, RowCfg<N_>::smem};                        \
     return true;
-#define XC_COL_CASE(N_, A_, B_, C_)                                                                             \
-  case N_:                                                                                                      \
-    *k = ColKernels{(const void*)&col_forward<XC_FFT_T, N_>, (const void*)&col_pairs<XC_FFT_T, N_, false, false>, \
-                    (const void*)&col_pairs<XC_FFT_T, N_, true, false>,                                         \
-                    (const void*)&col_pairs<XC_FFT_T, N_, true, true>, ColCfg<XC_FFT_T, N_>::threads,           \
-                    ColCfg<XC_FFT_T, N_>::PU, ColCfg<XC_FFT_T, N_>::lgcb,                                       \
-                    ColCfg<XC_FFT_T, N_>::PU * ColCfg<XC_FFT_T, N_>::unit * (int)sizeof(Cx<XC_FFT_T>)};         \
+#define XC_COL_CASE(N_, ...)                                                                                       \
+  case N_:                                                                                                         \
+    *k = ColKernels{(const void*)&col_forward<XC_FFT_S, N_>, (const void*)&col_pairs<XC_FFT_S, N_, false, false>,   \
+                    (const void*)&col_pairs<XC_FFT_S, N_, true, false>,                                            \
+                    (const void*)&col_pairs<XC_FFT_S, N_, true, true>, ColCfg<XC_FFT_S, N_>::threads,               \
+                    ColCfg<XC_FFT_S, N_>::PU, ColCfg<XC_FFT_S, N_>::lgcb,                                           \
+                    ColCfg<XC_FFT_S, N_>::PU * ColCfg<XC_FFT_S, N_>::unit * 16};                                   \
     return true;
 
 }  // namespace fe

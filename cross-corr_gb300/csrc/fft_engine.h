@@ -24,8 +24,8 @@ struct Engine {
   int nx = 0, ny = 0, nblk = 0;
   RowKernels rk{};
   ColKernels ck{};
-  void* tw = nullptr;      // device: row table, then column table
-  size_t tw_col = 0;       // byte offset of the column table
+  void* tw = nullptr;      // device: row table, column table, a row of zeros
+  size_t tw_col = 0, zeros = 0;  // byte offsets of the last two
   bool shared = false;     // every right serves several lefts: all spectra are made first
   bool lpre = false;       // left spectra are made first
   int l_chunk = 1, k_chunk = 1, kc = 1;
@@ -34,10 +34,10 @@ struct Engine {
 
 // Smallest length >= n that the kernels have; 0 when n is beyond the largest.
 int length_for(int n);
-// Twiddle table of a length (entries of two reals; host memory).
-size_t twiddle_count(int n);
-void fill_twiddles_f32(int n, float* out);
-void fill_twiddles_f64(int n, double* out);
+// Twiddle tables of a length's row or column passes: entries of 16 bytes, as
+// the kernels read them.
+size_t twiddle_bytes(int n, bool rows);
+void fill_twiddles(int n, bool rows, xc_dtype dtype, void* out);
 
 // Plans a problem within `ws_bytes` of workspace.  *e stays not ready (and
 // XC_OK is returned) when the sizes are beyond the kernels' lengths or the

@@ -5,10 +5,10 @@
 namespace xc {
 namespace fe {
 
-#define XC_FFT_T double
+#define XC_FFT_S double
 bool row_kernels_f64(int n, RowKernels* k) {
   switch (n) {
-    XC_FFT_LENGTHS(XC_ROW_CASE)
+    XC_FFT_ROWS(XC_ROW_CASE)
     default: return false;
   }
 }
