@@ -28,8 +28,8 @@ ARCH = ["-gencode", "arch=compute_103a,code=sm_103a"]
 NVCC_FLAGS = ["-O3", "-std=c++17", "-lineinfo", "-Xcompiler", "-fPIC", "--expt-relaxed-constexpr",
               "-I" + INCLUDE, "-I" + CSRC]
 CUDA_SOURCES = ["xc_runtime.cu", "direct_simt.cu", "ragged.cu", "fft_glue.cu", "fft_pipeline.cu", "tc_bf16x3.cu",
-                "mlp.cu", "api.cu", "fft_engine.cu", "fft_rows_f32.cu", "fft_cols_f32.cu", "fft_rows_f64.cu",
-                "fft_cols_f64.cu"]
+                "mlp.cu", "api.cu", "fft_engine.cu", "fft_rows_f32.cu", "fft_cols_f32.cu", "fft_cols_f32_long.cu",
+                "fft_rows_f64.cu", "fft_cols_f64.cu", "fft_cols_f64_long.cu", "ragged_fft.cu"]
 CLI_SOURCES = ["main.cpp", "data_array.cpp", "json_args.cpp", "algorithms.cpp"]
 
 
@@ -77,7 +77,7 @@ def build_library(verbose: bool = False, extra_flags=None) -> str:
         objs.append(o)
         if _stale(o, [s] + heads):
             jobs.append([nvcc] + ARCH + NVCC_FLAGS + list(extra_flags or []) + ["-c", s, "-o", o])
-    with cf.ThreadPoolExecutor(max_workers=min(8, max(1, len(jobs)))) as ex:
+    with cf.ThreadPoolExecutor(max_workers=min(16, max(1, len(jobs)))) as ex:
         for f in [ex.submit(_run, j, verbose) for j in jobs]:
             f.result()
     lib = os.path.join(OUT, "libxcorr.so")

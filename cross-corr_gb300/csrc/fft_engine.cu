@@ -110,15 +110,16 @@ xc_status run(const Engine& e, const void* left, const void* right, void* out, c
   Cx<T>* b = reinterpret_cast<Cx<T>*>(ws + e.off_b);
   const int lgcb = e.ck.lgcb, nblk = e.nblk;
   const int rows_per_cta = 2 * e.rk.nv * e.rk.q;
-  const double scale = 1.0 / ((double)e.nx * (double)e.ny);
+  const Scales sc = spectrum_scales(e.nx, e.ny);
 
   // rows of `nr` rights from the r0-th on, and (first) of all lefts.  FP64
-  // applies the result's scale here, in a product that is there anyway.
+  // applies all of the result's scale here, in a product that is there anyway.
   const auto rows = [&](bool lefts, long long r0, long long nr) {
     RowFwdArgs<T> a{};
-    a.a = RowSide<T>{static_cast<const T*>(left), al, g.Hl, g.Wl, div_up(g.Hl, rows_per_cta), T(1)};
+    a.a = RowSide<T>{static_cast<const T*>(left), al, g.Hl, g.Wl, div_up(g.Hl, rows_per_cta),
+                     (T)sc.left};
     a.b = RowSide<T>{static_cast<const T*>(right) + r0 * g.Hr * g.Wr, ar, g.Hr, g.Wr, div_up(g.Hr, rows_per_cta),
-                     (T)scale};
+                     (T)(sizeof(T) == 8 ? sc.right * sc.rest : sc.right)};
     const long long ab = lefts ? (long long)e.pm.n_left * a.a.groups : 0;
     if (ab + nr * a.b.groups > 0x7fffffffLL) return fail(XC_ERR_INVALID_ARGUMENT, "problem too large for one launch");
     a.a_blocks = (unsigned)ab;
@@ -184,8 +185,8 @@ xc_status run(const Engine& e, const void* left, const void* right, void* out, c
         a.nk = nk;
         a.o_l = e.pm.o_l;
         a.o_k = e.pm.o_k;
-        a.scale_hi = (T)scale;
-        a.scale_lo = (T)(scale - (double)a.scale_hi);
+        a.scale_hi = (T)sc.rest;
+        a.scale_lo = (T)(sc.rest - (double)a.scale_hi);
         a.tw = tw;
         XC_TRY(launch(e.rk.inverse, (long long)nl * nk * a.groups, e.rk.threads, e.rk.smem, a, stream));
       }
@@ -195,6 +196,15 @@ xc_status run(const Engine& e, const void* left, const void* right, void* out, c
 }
 
 }  // namespace
+
+Scales spectrum_scales(int nx, int ny) {
+  Scales s;
+  int e = 0;
+  s.rest = 1.0 / std::frexp((double)nx * (double)ny, &e);  // nx ny = m 2^e, 1/2 <= m < 1
+  s.left = std::ldexp(1.0, -(e / 2));
+  s.right = std::ldexp(1.0, -(e - e / 2));
+  return s;
+}
 
 int length_for(int n) {
   for (const Factors& f : kRows)

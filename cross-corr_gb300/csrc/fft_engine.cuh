@@ -364,12 +364,15 @@ struct Dft<S, D, 14> : DftPfa<S, D, 2, 7> {};
 // and R3 small, because a row thread holds two items of its first (inverse) or
 // last (forward) pass, and alike, so that neither pass leaves threads idle.
 // ---------------------------------------------------------------------------
-#define XC_FFT_COLS(X)                                                                                   \
+#define XC_FFT_COLS_SHORT(X)                                                                              \
   X(16, 4, 1, 4) X(32, 8, 1, 4) X(48, 8, 1, 6) X(64, 8, 1, 8) X(80, 10, 1, 8) X(96, 12, 1, 8)              \
   X(112, 14, 1, 8) X(128, 16, 1, 8) X(160, 16, 1, 10) X(192, 16, 1, 12) X(224, 16, 1, 14) X(256, 16, 1, 16) \
-  X(320, 8, 8, 5) X(384, 8, 8, 6) X(448, 8, 8, 7) X(512, 8, 8, 8) X(640, 10, 8, 8) X(768, 12, 8, 8)         \
-  X(896, 14, 8, 8) X(1024, 16, 8, 8) X(1280, 16, 10, 8) X(1536, 16, 12, 8) X(1792, 16, 14, 8)              \
-  X(2048, 16, 16, 8) X(2560, 16, 16, 10) X(3072, 16, 16, 12) X(3584, 16, 16, 14) X(4096, 16, 16, 16)
+  X(320, 8, 8, 5) X(384, 8, 8, 6) X(448, 8, 8, 7) X(512, 8, 8, 8)
+#define XC_FFT_COLS_LONG(X)                                                                               \
+  X(640, 10, 8, 8) X(768, 12, 8, 8) X(896, 14, 8, 8) X(1024, 16, 8, 8) X(1280, 16, 10, 8)                   \
+  X(1536, 16, 12, 8) X(1792, 16, 14, 8) X(2048, 16, 16, 8) X(2560, 16, 16, 10) X(3072, 16, 16, 12)           \
+  X(3584, 16, 16, 14) X(4096, 16, 16, 16)
+#define XC_FFT_COLS(X) XC_FFT_COLS_SHORT(X) XC_FFT_COLS_LONG(X)
 #define XC_FFT_ROWS(X)                                                                                     \
   X(16, 4, 1, 1, 4) X(32, 8, 1, 1, 4) X(48, 8, 1, 1, 6) X(64, 8, 1, 1, 8) X(80, 10, 1, 1, 8)                 \
   X(96, 12, 1, 1, 8) X(112, 8, 1, 1, 14) X(128, 4, 8, 1, 4) X(160, 4, 10, 1, 4) X(192, 8, 3, 1, 8)           \
@@ -490,6 +493,29 @@ struct RowSide {
   int groups;    // CTAs per matrix
   T scale;       // of the spectra (times the 1/2 of the separation)
 };
+// Ragged batches: one record per matrix (or pair), and for every CTA (column
+// kernel: every unit) the record it works on and its place in it.
+template <typename T>
+struct RagRow {
+  const T* src;
+  Cx<T>* dst;
+  int H, W, lgcb;
+  T scale;
+};
+template <typename T>
+struct RagCol {
+  const Cx<T>* left;
+  const Cx<T>* right;
+  Cx<T>* out;
+  int Hl, Hr, Sy, nblk;
+};
+template <typename T>
+struct RagInv {
+  const Cx<T>* src;
+  T* out;
+  int Sy, Sx, Wr, lgcb;
+  T scale_hi, scale_lo;
+};
 template <typename T>
 struct RowFwdArgs {
   RowSide<T> a, b;    // blocks [0, a_blocks) on side a, the rest on side b
@@ -497,6 +523,8 @@ struct RowFwdArgs {
   int nblk, lgcb;
   const void* tw;     // Cp<S> entries
   const T* zeros;     // a row of zeros, read in the place of rows past the last
+  const RagRow<T>* items;  // ragged: records, and per CTA (record, row group)
+  const int2* ctas;
 };
 
 template <typename T>
@@ -511,6 +539,9 @@ struct ColArgs {
   int n_kg, kc;       // partner groups of kc partners
   long long r_l, r_k, r_off;  // right(l, k) = l r_l + k r_k - r_off within `right`
   const void* tw;
+  const RagCol<T>* items;  // ragged: records, and per unit (record, block)
+  const int2* units;
+  int n_units;
 };
 template <typename T>
 struct ColFwdArgs {
@@ -531,6 +562,8 @@ struct RowInvArgs {
   long long o_l, o_k;
   T scale_hi, scale_lo;
   const void* tw;
+  const RagInv<T>* items;  // ragged: records, and per CTA (record, row group)
+  const int2* ctas;
 };
 
 // Row kernels: a transform (NV row pairs) on TP threads, Q of them per CTA.
@@ -600,7 +633,7 @@ __device__ __forceinline__ Cp<double> ld(const Cp<double>* g) {
 __device__ __forceinline__ Cp<f2> gather(const float* v) { return {pack(v[0], v[2]), pack(v[1], v[3])}; }
 __device__ __forceinline__ Cp<double> gather(const double* v) { return {v[0], v[1]}; }
 
-template <typename S, int N>
+template <typename S, int N, bool RAG>
 __global__ void __launch_bounds__(RowCfg<N>::threads, RowCfg<N>::min_ctas) row_forward(const RowFwdArgs<typename Sc<S>::real> p) {
   using L = RowPasses<N>;
   using C = Cp<S>;
@@ -609,15 +642,36 @@ __global__ void __launch_bounds__(RowCfg<N>::threads, RowCfg<N>::min_ctas) row_f
   extern __shared__ __align__(16) unsigned char smem_raw[];
   pdl_launch();
   const C* __restrict__ tw = static_cast<const C*>(p.tw);
-  const bool first = blockIdx.x < p.a_blocks;
-  const unsigned b = first ? blockIdx.x : blockIdx.x - p.a_blocks;
-  const int H = first ? p.a.H : p.b.H, W = first ? p.a.W : p.b.W;
-  const unsigned groups = (unsigned)(first ? p.a.groups : p.b.groups);
-  const unsigned mat = b / groups;
+  int H, W, group, lgcb;
+  const T* __restrict__ src;
+  Cx<T>* dst;
+  T scale;
+  if constexpr (RAG) {
+    const int2 e = p.ctas[blockIdx.x];
+    const RagRow<T>& it = p.items[e.x];
+    H = it.H;
+    W = it.W;
+    lgcb = it.lgcb;
+    src = it.src;
+    dst = it.dst;
+    scale = it.scale;
+    group = e.y;
+  } else {
+    const bool first = blockIdx.x < p.a_blocks;
+    const unsigned b = first ? blockIdx.x : blockIdx.x - p.a_blocks;
+    const unsigned groups = (unsigned)(first ? p.a.groups : p.b.groups);
+    const unsigned mat = b / groups;
+    H = first ? p.a.H : p.b.H;
+    W = first ? p.a.W : p.b.W;
+    lgcb = p.lgcb;
+    src = (first ? p.a.src : p.b.src) + (long long)mat * H * W;
+    dst = (first ? p.a.dst : p.b.dst) + (((long long)mat * p.nblk * H) << lgcb);
+    scale = first ? p.a.scale : p.b.scale;
+    group = (int)(b - mat * groups);
+  }
   const int f = threadIdx.x / TP, i = threadIdx.x - f * TP;
-  const int row0 = (int)((b - mat * groups) * Q + f) * (2 * NV);
+  const int row0 = (group * Q + f) * (2 * NV);
   C* z = reinterpret_cast<C*>(smem_raw) + f * RowCfg<N>::FS;
-  const T* __restrict__ src = (first ? p.a.src : p.b.src) + (long long)mat * H * W;
   const T* r[2 * NV];
 #pragma unroll
   for (int j = 0; j < 2 * NV; ++j) r[j] = row0 + j < H ? src + (long long)(row0 + j) * W : p.zeros;
@@ -657,16 +711,17 @@ __global__ void __launch_bounds__(RowCfg<N>::threads, RowCfg<N>::min_ctas) row_f
   }
   Dft<S, -1, L::R3>::run(x);
   Dft<S, -1, L::R3>::run(y);
-  // The two rows' spectra: A = (Z[k] + conj Z[-k]) / 2, B = (Z[k] - conj Z[-k]) / 2i.
-  const S half = Sc<S>::bc(0.5);
-  S hs = half;
-  if constexpr (NV == 1) hs = T(0.5) * (first ? p.a.scale : p.b.scale);
-  const int cb = 1 << p.lgcb;
-  Cx<T>* dst = (first ? p.a.dst : p.b.dst) + ((long long)mat * p.nblk * H + row0) * cb;
+  // The two rows' spectra: A = (Z[k] + conj Z[-k]) / 2, B = (Z[k] - conj Z[-k]) / 2i,
+  // with the side's scale in the same product.
+  S hs;
+  if constexpr (NV == 2) hs = pack(0.5f * scale, 0.5f * scale);
+  else hs = T(0.5) * scale;
+  const int cb = 1 << lgcb;
+  dst += (long long)row0 * cb;
   const auto put = [&](int k, C zk, C zn) {
     const C a = {mul(hs, add(zk.x, zn.x)), mul(hs, sub(zk.y, zn.y))};
     const C bb = {mul(hs, add(zk.y, zn.y)), mul(hs, sub(zn.x, zk.x))};
-    Cx<T>* d = dst + (long long)(k >> p.lgcb) * H * cb + (k & (cb - 1));
+    Cx<T>* d = dst + (long long)(k >> lgcb) * H * cb + (k & (cb - 1));
     if constexpr (NV == 2) {
       *reinterpret_cast<float2*>(d) = make_float2(lo(a.x), lo(a.y));
       if (row0 + 1 < H) *reinterpret_cast<float2*>(d + cb) = make_float2(lo(bb.x), lo(bb.y));
@@ -689,7 +744,7 @@ __global__ void __launch_bounds__(RowCfg<N>::threads, RowCfg<N>::min_ctas) row_f
   }
 }
 
-template <typename S, int N>
+template <typename S, int N, bool RAG>
 __global__ void __launch_bounds__(RowCfg<N>::threads, RowCfg<N>::min_ctas) row_inverse(const RowInvArgs<typename Sc<S>::real> p) {
   using L = RowPasses<N>;
   using C = Cp<S>;
@@ -698,16 +753,44 @@ __global__ void __launch_bounds__(RowCfg<N>::threads, RowCfg<N>::min_ctas) row_i
   extern __shared__ __align__(16) unsigned char smem_raw[];
   pdl_launch();
   const C* __restrict__ tw = static_cast<const C*>(p.tw);
-  const unsigned t = blockIdx.x / (unsigned)p.groups;
+  int Sy, Sx, Wr, group, lgcb;
+  const Cx<T>* __restrict__ src;
+  T* out;
+  T scale_hi, scale_lo;
+  if constexpr (RAG) {
+    const int2 e = p.ctas[blockIdx.x];
+    const RagInv<T>& it = p.items[e.x];
+    Sy = it.Sy;
+    Sx = it.Sx;
+    Wr = it.Wr;
+    lgcb = it.lgcb;
+    src = it.src;
+    out = it.out;
+    scale_hi = it.scale_hi;
+    scale_lo = it.scale_lo;
+    group = e.y;
+  } else {
+    const unsigned t = blockIdx.x / (unsigned)p.groups;
+    const int l = p.l0 + (int)t / p.nk, k = p.k0 + (int)t % p.nk;
+    Sy = p.Sy;
+    Sx = p.Sx;
+    Wr = p.Wr;
+    lgcb = p.lgcb;
+    src = p.src + (((long long)t * p.nblk * Sy) << lgcb);
+    out = p.out + (l * p.o_l + k * p.o_k) * Sy * (long long)Sx;
+    scale_hi = p.scale_hi;
+    scale_lo = p.scale_lo;
+    group = (int)(blockIdx.x - t * (unsigned)p.groups);
+  }
   const int f = threadIdx.x / TP, i = threadIdx.x - f * TP;
-  const int row0 = (int)((blockIdx.x - t * (unsigned)p.groups) * Q + f) * (2 * NV);
+  const int row0 = (group * Q + f) * (2 * NV);
   C* z = reinterpret_cast<C*>(smem_raw) + f * RowCfg<N>::FS;
-  const int cb = 1 << p.lgcb;
-  const Cx<T>* __restrict__ src = p.src + ((long long)t * p.nblk * p.Sy + row0) * cb;
-  const bool v0 = row0 < p.Sy, v1 = row0 + 1 < p.Sy, v2 = row0 + 2 < p.Sy, v3 = row0 + 3 < p.Sy;
+  const int cb = 1 << lgcb;
+  src += (long long)row0 * cb;
+  const bool v0 = row0 < Sy, v1 = row0 + 1 < Sy, v2 = row0 + 2 < Sy, v3 = row0 + 3 < Sy;
   // rows A and B of each row pair at column c
   const auto get = [&](int c, C* a, C* b) {
-    const Cx<T>* d = src + (long long)(c >> p.lgcb) * p.Sy * cb + (c & (cb - 1));
+    const Cx<T>* d = src + (long long)(c >> lgcb) * Sy * cb + (c & (cb - 1));
     if constexpr (NV == 2) {
       const float2 o = make_float2(0.f, 0.f);
       const float2 e0 = v0 ? ld(reinterpret_cast<const float2*>(d)) : o;
@@ -770,8 +853,7 @@ __global__ void __launch_bounds__(RowCfg<N>::threads, RowCfg<N>::min_ctas) row_i
   __syncthreads();
   mid_passes<S, 1, false, L, 1>(z, i, TP, tw);
   if (!v0) return;
-  const int l = p.l0 + (int)t / p.nk, k = p.k0 + (int)t % p.nk;
-  T* o0 = p.out + ((l * p.o_l + k * p.o_k) * p.Sy + row0) * (long long)p.Sx;
+  T* o0 = out + (long long)row0 * Sx;
 #pragma unroll
   for (int u = 0; u < 2; ++u) {
     const int it = i + u * TP;
@@ -782,21 +864,21 @@ __global__ void __launch_bounds__(RowCfg<N>::threads, RowCfg<N>::min_ctas) row_i
     Dft<S, 1, L::R3>::run(x);
 #pragma unroll
     for (int q = 0; q < L::R3; ++q) {
-      int sx = it + q * L::TF + p.Wr - 1;
+      int sx = it + q * L::TF + Wr - 1;
       if (sx >= N) sx -= N;
-      if (sx >= p.Sx) continue;
+      if (sx >= Sx) continue;
       T* d = o0 + sx;
       if constexpr (NV == 2) {
         // the scale as a sum of two terms: rounds like a scaling in higher precision
-        const f2 sh = pack(p.scale_hi, p.scale_hi), sl = pack(p.scale_lo, p.scale_lo);
+        const f2 sh = pack(scale_hi, scale_hi), sl = pack(scale_lo, scale_lo);
         const f2 a = fma(x[q].x, sh, mul(x[q].x, sl)), b = fma(x[q].y, sh, mul(x[q].y, sl));
         d[0] = lo(a);
-        if (v1) d[p.Sx] = lo(b);
-        if (v2) d[2 * (long long)p.Sx] = hi(a);
-        if (v3) d[3 * (long long)p.Sx] = hi(b);
+        if (v1) d[Sx] = lo(b);
+        if (v2) d[2 * (long long)Sx] = hi(a);
+        if (v3) d[3 * (long long)Sx] = hi(b);
       } else {
         d[0] = x[q].x;
-        if (v1) d[p.Sx] = x[q].y;
+        if (v1) d[Sx] = x[q].y;
       }
     }
   }
@@ -920,7 +1002,7 @@ __global__ void __launch_bounds__(ColCfg<S, N>::threads, ColCfg<S, N>::min_ctas)
 // the product with the left spectrum (LPRE: read from global memory;
 // otherwise transformed once per group and kept in shared memory), and the
 // inverse transform, whose rows go out in the output's row order.
-template <typename S, int N, bool LPRE, bool RPRE>
+template <typename S, int N, bool LPRE, bool RPRE, bool RAG>
 __global__ void __launch_bounds__(ColCfg<S, N>::threads, ColCfg<S, N>::min_ctas) col_pairs(const ColArgs<typename Sc<S>::real> p) {
   using L = ColPasses<N>;
   using C = Cp<S>;
@@ -935,19 +1017,50 @@ __global__ void __launch_bounds__(ColCfg<S, N>::threads, ColCfg<S, N>::min_ctas)
   C* z = reinterpret_cast<C*>(smem_raw) + pu * K::unit + c;
   C* zl = z + (LPRE ? 0 : K::PU * K::unit);  // left spectrum
   const unsigned gu = blockIdx.x * K::PU + pu;
-  const unsigned blk = gu % (unsigned)p.nblk, rest = gu / (unsigned)p.nblk;
-  const int kg = (int)(rest % (unsigned)p.n_kg);
-  const int ll = (int)(rest / (unsigned)p.n_kg);  // left of this launch
-  const bool live = ll < p.n_left;
-  const long long l = p.l0 + (live ? ll : 0);
-  const int ka = p.k0 + kg * p.kc, nk = live ? min(p.kc, p.k1 - ka) : 0;
+  unsigned blk;
+  int ll = 0, ka = 0, nk, kc = 1, Hl, Hr, Sy, nblk;
+  long long l = 0;
+  bool live;
+  const G* gl;  // row spectra of the left's and the (first) right's block
+  const G* gr;
+  G* out;
+  if constexpr (RAG) {
+    live = gu < (unsigned)p.n_units;
+    const int2 e = p.units[live ? gu : 0];
+    const RagCol<typename Sc<S>::real>& it = p.items[e.x];
+    blk = (unsigned)e.y;
+    Hl = it.Hl;
+    Hr = it.Hr;
+    Sy = it.Sy;
+    nblk = it.nblk;
+    nk = live ? 1 : 0;
+    gl = it.left;
+    gr = it.right;
+    out = it.out;
+  } else {
+    nblk = p.nblk;
+    blk = gu % (unsigned)nblk;
+    const unsigned rest = gu / (unsigned)nblk;
+    const int kg = (int)(rest % (unsigned)p.n_kg);
+    ll = (int)(rest / (unsigned)p.n_kg);  // left of this launch
+    live = ll < p.n_left;
+    l = p.l0 + (live ? ll : 0);
+    kc = p.kc;
+    ka = p.k0 + kg * kc;
+    nk = live ? min(kc, p.k1 - ka) : 0;
+    Hl = p.Hl;
+    Hr = p.Hr;
+    Sy = p.Sy;
+    gl = static_cast<const G*>(p.left);
+    gr = static_cast<const G*>(p.right);
+    out = p.out;
+  }
   const C* lspec = nullptr;
   pdl_wait();
   if constexpr (LPRE) {
-    lspec = static_cast<const C*>(p.left) + (l * p.nblk + blk) * (long long)N * K::LC + c;
+    lspec = static_cast<const C*>(p.left) + (l * nblk + blk) * (long long)N * K::LC + c;
   } else {
-    col_load_passes<S, N>(zl, static_cast<const G*>(p.left) + (l * p.nblk + blk) * (long long)p.Hl * K::CB + c * NV,
-                          live ? p.Hl : 0, j0, tw);
+    col_load_passes<S, N>(zl, gl + (l * nblk + blk) * (long long)Hl * K::CB + c * NV, live ? Hl : 0, j0, tw);
     // each thread reads back the items it writes here: no barrier needed
     for (int j = j0; j < L::TF; j += K::JT) {
       C x[L::R3];
@@ -959,19 +1072,18 @@ __global__ void __launch_bounds__(ColCfg<S, N>::threads, ColCfg<S, N>::min_ctas)
       for (int m = 0; m < L::R3; ++m) base[m * K::LC] = x[m];
     }
   }
-  const long long n_k = p.k1 - p.k0;
-  for (int kk = 0; kk < p.kc; ++kk) {
+  const long long n_k = RAG ? 1 : p.k1 - p.k0;
+  for (int kk = 0; kk < kc; ++kk) {
     const int k = ka + kk;
     const bool act = kk < nk;
-    const long long r = act ? l * p.r_l + k * p.r_k - p.r_off : 0;
+    const long long r = !RAG && act ? l * p.r_l + k * p.r_k - p.r_off : 0;
     if constexpr (!RPRE)
-      col_load_passes<S, N>(z, static_cast<const G*>(p.right) + (r * p.nblk + blk) * (long long)p.Hr * K::CB + c * NV,
-                            act ? p.Hr : 0, j0, tw);
+      col_load_passes<S, N>(z, gr + (r * nblk + blk) * (long long)Hr * K::CB + c * NV, act ? Hr : 0, j0, tw);
     for (int j = j0; j < L::TF; j += K::JT) {
       C x[L::R3];
       C* base = z + col_item<S, N>(j);
       if constexpr (RPRE) {
-        const C* rspec = static_cast<const C*>(p.right) + (r * p.nblk + blk) * (long long)N * K::LC + c;
+        const C* rspec = static_cast<const C*>(p.right) + (r * nblk + blk) * (long long)N * K::LC + c;
 #pragma unroll
         for (int q = 0; q < L::R3; ++q) x[q] = ld(rspec + (q * L::TF + j) * K::LC);
       } else {
@@ -989,23 +1101,23 @@ __global__ void __launch_bounds__(ColCfg<S, N>::threads, ColCfg<S, N>::min_ctas)
     __syncthreads();
     mid_passes<S, 1, true, L, K::LC>(z, j0, K::JT, tw);
     if (act) {
-      G* out = p.out + ((ll * n_k + (k - p.k0)) * p.nblk + blk) * (long long)p.Sy * K::CB + c * NV;
-      for (int o = j0; o < L::S1; o += K::JT) {
+      G* o = out + ((ll * n_k + (RAG ? 0 : k - p.k0)) * nblk + blk) * (long long)Sy * K::CB + c * NV;
+      for (int i = j0; i < L::S1; i += K::JT) {
         C x[L::R1];
-        const C* base = z + L::in_block(o) * K::LC;
+        const C* base = z + L::in_block(i) * K::LC;
         x[0] = base[0];
 #pragma unroll
-        for (int q = 1; q < L::R1; ++q) x[q] = cmul<true>(base[q * L::P1 * K::LC], tw[(q - 1) * L::S1 + o]);
+        for (int q = 1; q < L::R1; ++q) x[q] = cmul<true>(base[q * L::P1 * K::LC], tw[(q - 1) * L::S1 + i]);
         Dft<S, 1, L::R1>::run(x);
 #pragma unroll
         for (int m = 0; m < L::R1; ++m) {
-          int sy = o + m * L::S1 + p.Hr - 1;
+          int sy = i + m * L::S1 + Hr - 1;
           if (sy >= N) sy -= N;
-          if (sy < p.Sy) store_row(out + (long long)sy * K::CB, x[m]);
+          if (sy < Sy) store_row(o + (long long)sy * K::CB, x[m]);
         }
       }
     }
-    if (kk + 1 < p.kc) __syncthreads();  // the next partner's passes overwrite z
+    if (kk + 1 < kc) __syncthreads();  // the next partner's passes overwrite z
   }
 }
 
@@ -1013,6 +1125,8 @@ __global__ void __launch_bounds__(ColCfg<S, N>::threads, ColCfg<S, N>::min_ctas)
 struct RowKernels {
   const void* forward;
   const void* inverse;
+  const void* rag_forward;  // over a ragged batch's records (FP32 only)
+  const void* rag_inverse;
   int threads, q, nv, smem;
 };
 struct ColKernels {
@@ -1020,6 +1134,7 @@ struct ColKernels {
   const void* pairs;       // left transformed in the kernel
   const void* pairs_lpre;  // left spectra from col_forward
   const void* pairs_pre;   // both
+  const void* rag_pairs;   // `pairs` over a ragged batch's records (FP32 only)
   int threads, pu, lgcb, unit_smem;  // shared memory of one buffer
 };
 // false: no kernels for this length
@@ -1027,19 +1142,46 @@ bool row_kernels_f32(int n, RowKernels* k);
 bool row_kernels_f64(int n, RowKernels* k);
 bool col_kernels_f32(int n, ColKernels* k);
 bool col_kernels_f64(int n, ColKernels* k);
+bool col_kernels_f32_long(int n, ColKernels* k);  // the longer half of the lengths
+bool col_kernels_f64_long(int n, ColKernels* k);
 
-#define XC_ROW_CASE(N_, ...)                                                                                       \
-  case N_:                                                                                                         \
-    *k = RowKernels{(const void*)&row_forward<XC_FFT_S, N_>, (const void*)&row_inverse<XC_FFT_S, N_>,               \
-                    RowCfg<N_>::threads, RowCfg<N_>::Q, Sc<XC_FFT_S>::NV, RowCfg<N_>::smem};                        \
+template <typename S, int N>
+RowKernels row_kernels_of() {
+  RowKernels k{};
+  k.forward = (const void*)&row_forward<S, N, false>;
+  k.inverse = (const void*)&row_inverse<S, N, false>;
+  if constexpr (Sc<S>::NV == 2) {
+    k.rag_forward = (const void*)&row_forward<S, N, true>;
+    k.rag_inverse = (const void*)&row_inverse<S, N, true>;
+  }
+  k.threads = RowCfg<N>::threads;
+  k.q = RowCfg<N>::Q;
+  k.nv = Sc<S>::NV;
+  k.smem = RowCfg<N>::smem;
+  return k;
+}
+template <typename S, int N>
+ColKernels col_kernels_of() {
+  using K = ColCfg<S, N>;
+  ColKernels k{};
+  k.forward = (const void*)&col_forward<S, N>;
+  k.pairs = (const void*)&col_pairs<S, N, false, false, false>;
+  k.pairs_lpre = (const void*)&col_pairs<S, N, true, false, false>;
+  k.pairs_pre = (const void*)&col_pairs<S, N, true, true, false>;
+  if constexpr (Sc<S>::NV == 2) k.rag_pairs = (const void*)&col_pairs<S, N, false, false, true>;
+  k.threads = K::threads;
+  k.pu = K::PU;
+  k.lgcb = K::lgcb;
+  k.unit_smem = K::PU * K::unit * 16;
+  return k;
+}
+#define XC_ROW_CASE(N_, ...)              \
+  case N_:                                \
+    *k = row_kernels_of<XC_FFT_S, N_>();  \
     return true;
-#define XC_COL_CASE(N_, ...)                                                                                       \
-  case N_:                                                                                                         \
-    *k = ColKernels{(const void*)&col_forward<XC_FFT_S, N_>, (const void*)&col_pairs<XC_FFT_S, N_, false, false>,   \
-                    (const void*)&col_pairs<XC_FFT_S, N_, true, false>,                                            \
-                    (const void*)&col_pairs<XC_FFT_S, N_, true, true>, ColCfg<XC_FFT_S, N_>::threads,               \
-                    ColCfg<XC_FFT_S, N_>::PU, ColCfg<XC_FFT_S, N_>::lgcb,                                           \
-                    ColCfg<XC_FFT_S, N_>::PU * ColCfg<XC_FFT_S, N_>::unit * 16};                                   \
+#define XC_COL_CASE(N_, ...)              \
+  case N_:                                \
+    *k = col_kernels_of<XC_FFT_S, N_>();  \
     return true;
 
 }  // namespace fe

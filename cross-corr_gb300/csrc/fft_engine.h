@@ -32,6 +32,14 @@ struct Engine {
   size_t off_al = 0, off_ar = 0, off_fl = 0, off_fr = 0, off_b = 0, bytes = 0;
 };
 
+// 1 / (nx ny), the scale of an unnormalised pair of transforms, as powers of
+// two on the left and right spectra (half the exponent each, as a unitary
+// transform has, so that neither spectrum nor product leaves the type's range
+// before the result does) and a rest in (1, 2] at the end.
+struct Scales {
+  double left, right, rest;
+};
+Scales spectrum_scales(int nx, int ny);
 // Smallest length >= n that the kernels have; 0 when n is beyond the largest.
 int length_for(int n);
 // Twiddle tables of a length's row or column passes: entries of 16 bytes, as

@@ -12,11 +12,13 @@
 //    into the padded copies, reset the tile queue, one persistent launch of
 //    the plain kernel whose CTAs pull tiles from the queue until it is empty.
 // A variant is a tile shape of the plain kernel and, for FP32 batches, a
-// route: the pairs with at least the route's multiply-add count run instead
-// as one_to_one calls of the split-BF16 tensor-core path, dealt out over
-// up to kMaxTcStreams side streams (longest first, each to the least loaded stream)
-// and captured into the same graph, beside the plain kernel's branch.  Route
-// 0 keeps every pair on the plain kernel.
+// route: the pairs with at least the route's multiply-add count leave the
+// plain kernel and run on side streams captured into the same graph, beside
+// its branch: through the fused FFT kernels, a few launches for all of them
+// (ragged_fft.cu), or, where an output is beyond those kernels' lengths, as
+// one_to_one calls of the split-BF16 tensor-core path, dealt out over up to
+// kMaxTcStreams side streams (longest first, each to the least loaded
+// stream).  Route 0 keeps every pair on the plain kernel.
 // Executing the plan replays the chosen variant's graph.  The autotuner times
 // every tile shape with route 0, then the routes with the best shape, keeps
 // the fastest and remembers the choice in a small JSON-lines cache keyed by
@@ -34,6 +36,7 @@
 #include <string>
 #include <vector>
 
+#include "ragged_fft.h"
 #include "ragged_route.h"
 #include "xc_common.cuh"
 #include "xc_internal.h"
@@ -42,7 +45,10 @@ namespace xc {
 
 namespace {
 
-constexpr int kMaxTcStreams = 8;  // side streams of the split-BF16 route (XC_RAGGED_TC_STREAMS, default 8)
+constexpr int kMaxTcStreams = 8;  // side streams of the routes (XC_RAGGED_TC_STREAMS, default 8)
+// Spectra of the routed pairs held at once; a larger batch runs in several
+// chunks.
+constexpr size_t kFftWorkspace = (size_t)1 << 30;
 // Left rows per work item of a routed pair.  A lone call shortens its items
 // until they give two per SM; with eight calls in flight longer items pay
 // (512-pair batch, 448 pairs routed: 33.3 ms with the lone-call rule, 31.1 /
@@ -54,16 +60,31 @@ struct CopyJob {  // one matrix into its padded copy
   int rows, cols, pitch;
 };
 
-// One block per (job, row); copies a row and zero-fills the pitch tail.
+constexpr int kRepackRows = 16;  // rows per block of repack_kernel, four warps
+
+// Blocks [0, left_blocks) copy left matrices, the rest right ones; `first[j]`
+// is the first block of job j (of both sides, lefts first).  A block finds its
+// job by bisection; each warp copies rows and zero-fills the pitch tail.
 template <typename T>
-__global__ void repack_kernel(const T* __restrict__ src, T* __restrict__ dst, const CopyJob* __restrict__ jobs,
-                              int max_rows) {
-  const CopyJob jb = jobs[blockIdx.x / max_rows];
-  const int r = blockIdx.x % max_rows;
-  if (r >= jb.rows) return;
-  const T* s = src + jb.src + (long long)r * jb.cols;
-  T* d = dst + jb.dst + (long long)r * jb.pitch;
-  for (int c = threadIdx.x; c < jb.pitch; c += blockDim.x) d[c] = c < jb.cols ? s[c] : T(0);
+__global__ void __launch_bounds__(128) repack_kernel(const T* __restrict__ left, T* __restrict__ lpad,
+                                                     const T* __restrict__ right, T* __restrict__ rpad,
+                                                     const CopyJob* __restrict__ jobs, const int* __restrict__ first,
+                                                     int n_left, int n_jobs) {
+  int a = 0, b = n_jobs;  // first[a] <= block < first[b]
+  while (b - a > 1) {
+    const int m = (a + b) >> 1;
+    if (first[m] <= (int)blockIdx.x) a = m;
+    else b = m;
+  }
+  const CopyJob jb = jobs[a];
+  const T* s0 = (a < n_left ? left : right) + jb.src;
+  T* d0 = (a < n_left ? lpad : rpad) + jb.dst;
+  const int r0 = ((int)blockIdx.x - first[a]) * kRepackRows;
+  for (int r = r0 + (threadIdx.x >> 5); r < min(jb.rows, r0 + kRepackRows); r += 4) {
+    const T* s = s0 + (long long)r * jb.cols;
+    T* d = d0 + (long long)r * jb.pitch;
+    for (int c = threadIdx.x & 31; c < jb.pitch; c += 32) d[c] = c < jb.cols ? s[c] : T(0);
+  }
 }
 
 }  // namespace
@@ -79,8 +100,7 @@ struct RaggedPlanImpl {
   // device state
   void* lpad = nullptr;
   void* rpad = nullptr;
-  CopyJob* jobs = nullptr;
-  int n_jobs = 0, max_rows = 0;
+  std::vector<CopyJob> jobs;  // one per matrix: lefts, then rights
   RaggedPairDev* dpairs = nullptr;
   unsigned int* queue = nullptr;
   cudaStream_t capture_stream = nullptr;
@@ -88,6 +108,9 @@ struct RaggedPlanImpl {
     bool built = false;
     RaggedTile* tiles = nullptr;
     int n_tiles = 0;
+    CopyJob* jobs = nullptr;  // the matrices the variant's plain pairs use, and the first block of each
+    int* first = nullptr;
+    int n_left = 0, n_jobs = 0, repack_blocks = 0;
     int tc_pairs = 0;  // pairs of the variant's route (split-BF16 calls)
     int grid = 0;
     cudaGraph_t graph = nullptr;
@@ -98,9 +121,12 @@ struct RaggedPlanImpl {
   int n_shapes = 1, n_routes = 1;
   int chosen = 0;
   double tuned_ms = -1.0;
-  // split-BF16 routes (FP32)
+  // routes (FP32)
   std::vector<double> pair_mac;          // multiply-adds of each pair
   std::vector<char> tc_ok;               // the split path takes the pair
+  std::vector<char> fft_ok;              // the FFT kernels do (preferred)
+  std::vector<fe::RaggedFft> ffts;       // per route: the launches of its pairs
+  void* fft_ws = nullptr;
   int n_streams = kMaxTcStreams;
   cudaStream_t tc_streams[kMaxTcStreams] = {};
   cudaEvent_t fork = nullptr;
@@ -181,29 +207,45 @@ xc_status shape_maps(RaggedPlanImpl* P, int shape, const RaggedShape& sh) {
   return XC_OK;
 }
 
-// Side streams, fork/join events and one workspace per side stream (sized
-// for the largest pair the split path takes), made on the first route that
-// needs them.
-xc_status tc_resources(RaggedPlanImpl* P) {
+Geometry pair_geometry(const RaggedPairDev& d) {
+  return Geometry{d.Hl, d.Wl, d.Hr, d.Wr, d.Hl + d.Hr - 1, d.Wl + d.Wr - 1};
+}
+
+// The FFT pairs of a route, most multiply-adds first.
+std::vector<fe::FftPair> fft_pairs(const RaggedPlanImpl* P, int route) {
+  std::vector<fe::FftPair> v;
+  for (size_t i : route_pairs(P->pair_mac, P->tc_ok, route)) {
+    if (!P->fft_ok[i]) continue;
+    const RaggedPairDev d = pair_dev(P, i);
+    v.push_back(fe::FftPair{(const float*)P->left + P->lefts[d.left].offset,
+                            (const float*)P->right + P->rights[d.right].offset, (float*)P->out + d.out_off,
+                            pair_geometry(d)});
+  }
+  return v;
+}
+
+// Side streams, fork/join events, one spectra workspace for the largest route
+// and, where some pair needs it, a split-path workspace per side stream
+// (sized for the largest such pair), made on the first route that needs them.
+xc_status route_resources(RaggedPlanImpl* P) {
   if (P->fork != nullptr) return XC_OK;
   PairMap pm;
   uint64_t n_out = 0;
   make_pair_map(XC_ONE_TO_ONE, 1, 1, &pm, &n_out);
-  size_t ws = 0;
+  size_t ws = 0, fws = 0;
   for (size_t i = 0; i < P->pairs.size(); ++i)
-    if (P->tc_ok[i]) {
-      const RaggedPairDev d = pair_dev(P, i);
-      ws = std::max(ws, tc_workspace_size(Geometry{d.Hl, d.Wl, d.Hr, d.Wr, d.Hl + d.Hr - 1, d.Wl + d.Wr - 1}, pm,
-                                          false));
-    }
+    if (P->tc_ok[i] && !P->fft_ok[i])
+      ws = std::max(ws, tc_workspace_size(pair_geometry(pair_dev(P, i)), pm, false));
+  for (int r = 1; r < P->n_routes; ++r) fws = std::max(fws, fe::ragged_fft_workspace(fft_pairs(P, r), kFftWorkspace));
   // (what an earlier, failed attempt made is kept and reused)
   for (int k = 0; k < P->n_streams; ++k) {
     if (P->tc_streams[k] == nullptr)
       XC_CUDA_TRY(cudaStreamCreateWithFlags(&P->tc_streams[k], cudaStreamNonBlocking));
     if (P->joins[k] == nullptr) XC_CUDA_TRY(cudaEventCreateWithFlags(&P->joins[k], cudaEventDisableTiming));
-    if (P->tc_ws[k] == nullptr) XC_CUDA_TRY(cudaMalloc(&P->tc_ws[k], std::max<size_t>(ws, 256)));
+    if (P->tc_ws[k] == nullptr && ws > 0) XC_CUDA_TRY(cudaMalloc(&P->tc_ws[k], ws));
   }
-  P->tc_ws_bytes = std::max<size_t>(ws, 256);
+  P->tc_ws_bytes = ws;
+  if (P->fft_ws == nullptr && fws > 0) XC_CUDA_TRY(cudaMalloc(&P->fft_ws, fws));
   XC_CUDA_TRY(cudaEventCreateWithFlags(&P->fork, cudaEventDisableTiming));
   return XC_OK;
 }
@@ -217,11 +259,13 @@ xc_status build_variant(RaggedPlanImpl* P, int index) {
   // the route, longest first
   std::vector<RaggedPairDev> hp(P->pairs.size());
   std::vector<std::pair<double, RaggedTile>> tiles;
+  std::vector<char> used(P->jobs.size(), 0);  // matrices of the pairs the plain kernel keeps
   const std::vector<size_t> tc_pairs = route_pairs(P->pair_mac, P->tc_ok, route);
   for (size_t i = 0; i < P->pairs.size(); ++i) {
     const RaggedPairDev d = pair_dev(P, i);
     hp[i] = d;
     if (pair_in_route(P, i, route)) continue;
+    used[d.left] = used[P->lefts.size() + d.right] = 1;
     const int Sy = d.Hl + d.Hr - 1, Sx = d.Wl + d.Wr - 1;
     const int rem = (d.Wr - 1) % sh.vec;
     const int origin = rem == 0 ? 0 : rem - sh.vec;
@@ -247,7 +291,29 @@ xc_status build_variant(RaggedPlanImpl* P, int index) {
     cudaFree(v.tiles);
     v.tiles = nullptr;
   }
+  cudaFree(v.jobs);
+  cudaFree(v.first);
+  v.jobs = nullptr;
+  v.first = nullptr;
   if (v.n_tiles > 0) {
+    std::vector<CopyJob> jobs;
+    std::vector<int> first;
+    long long blocks = 0;
+    v.n_left = 0;
+    for (size_t j = 0; j < used.size(); ++j) {
+      if (!used[j]) continue;
+      if (j < P->lefts.size()) ++v.n_left;
+      jobs.push_back(P->jobs[j]);
+      first.push_back((int)blocks);
+      blocks += div_up(P->jobs[j].rows, kRepackRows);
+      if (blocks > 0x7fffffffLL) return fail(XC_ERR_INVALID_ARGUMENT, "ragged batch has too many rows");
+    }
+    v.n_jobs = (int)jobs.size();
+    v.repack_blocks = (int)blocks;
+    XC_CUDA_TRY(cudaMalloc(&v.jobs, sizeof(CopyJob) * jobs.size()));
+    XC_CUDA_TRY(cudaMemcpy(v.jobs, jobs.data(), sizeof(CopyJob) * jobs.size(), cudaMemcpyHostToDevice));
+    XC_CUDA_TRY(cudaMalloc(&v.first, sizeof(int) * first.size()));
+    XC_CUDA_TRY(cudaMemcpy(v.first, first.data(), sizeof(int) * first.size(), cudaMemcpyHostToDevice));
     XC_CUDA_TRY(cudaMalloc(&v.tiles, sizeof(RaggedTile) * ht.size()));
     XC_CUDA_TRY(cudaMemcpy(v.tiles, ht.data(), sizeof(RaggedTile) * ht.size(), cudaMemcpyHostToDevice));
     XC_TRY(shape_maps(P, shape, sh));
@@ -260,29 +326,33 @@ xc_status build_variant(RaggedPlanImpl* P, int index) {
     v.grid = std::max(1, std::min(v.n_tiles, sms * std::max(1, per_sm)));
   }
 
-  // the route's pairs: each to the side stream with the least work so far
+  // the route's pairs: the FFT kernels' launches, and the others each to the
+  // side stream with the least work so far
   PairMap pm1;
   uint64_t n_out1 = 0;
   make_pair_map(XC_ONE_TO_ONE, 1, 1, &pm1, &n_out1);
-  const std::vector<std::vector<size_t>> per_stream = deal_route(tc_pairs, P->pair_mac, P->n_streams);
+  std::vector<size_t> split;
+  for (size_t i : tc_pairs)
+    if (!P->fft_ok[i]) split.push_back(i);
+  const std::vector<std::vector<size_t>> per_stream = deal_route(split, P->pair_mac, P->n_streams);
   if (!tc_pairs.empty()) {
-    XC_TRY(tc_resources(P));
-    for (size_t i : tc_pairs) {
-      const RaggedPairDev& d = hp[i];
-      XC_TRY(tc_prepare(Geometry{d.Hl, d.Wl, d.Hr, d.Wr, d.Hl + d.Hr - 1, d.Wl + d.Wr - 1}, pm1, false));
-    }
+    XC_TRY(route_resources(P));
+    for (size_t i : split) XC_TRY(tc_prepare(pair_geometry(hp[i]), pm1, false));
+    if (split.size() < tc_pairs.size() && P->ffts[route].phases.empty())
+      XC_TRY(fe::ragged_fft_build(&P->ffts[route], fft_pairs(P, route), P->fft_ws, kFftWorkspace));
   }
 
-  // capture the step into a graph: the split-path branches fork from the
-  // capture stream first, so they depend on nothing; the plain branch runs
-  // beside them; the branches join before the capture ends
+  // capture the step into a graph: the route's branches fork from the capture
+  // stream first, so they depend on nothing; the plain branch runs beside
+  // them; the branches join before the capture ends
   cudaStream_t s = P->capture_stream;
   XC_CUDA_TRY(cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal));
   xc_status st = XC_OK;
   const bool forked = !tc_pairs.empty();
   if (forked && cudaEventRecord(P->fork, s) != cudaSuccess) st = fail(XC_ERR_CUDA, "ragged capture: fork failed");
   for (int k = 0; k < P->n_streams && forked; ++k)
-    if (st == XC_OK && !per_stream[k].empty() && cudaStreamWaitEvent(P->tc_streams[k], P->fork, 0) != cudaSuccess)
+    if (st == XC_OK && (k == 0 || !per_stream[k].empty()) &&
+        cudaStreamWaitEvent(P->tc_streams[k], P->fork, 0) != cudaSuccess)
       st = fail(XC_ERR_CUDA, "ragged capture: a side stream could not join");
   if (st == XC_OK && v.n_tiles > 0) {
     RaggedLaunch rl;
@@ -296,29 +366,22 @@ xc_status build_variant(RaggedPlanImpl* P, int index) {
     rl.queue = P->queue;
     rl.n_tiles = v.n_tiles;
     rl.grid = v.grid;
-    const unsigned nb_l = (unsigned)P->lefts.size() * (unsigned)P->max_rows;  // left jobs only
-    if (P->es == 4) {
-      repack_kernel<float><<<nb_l, 128, 0, s>>>((const float*)P->left, (float*)P->lpad, P->jobs, P->max_rows);
-    } else {
-      repack_kernel<double><<<nb_l, 128, 0, s>>>((const double*)P->left, (double*)P->lpad, P->jobs, P->max_rows);
-    }
-    // rights: jobs after the lefts in the same table, different source / destination
-    const int nl = (int)P->lefts.size();
-    const unsigned nb_r = (unsigned)(P->n_jobs - nl) * (unsigned)P->max_rows;
-    if (nb_r > 0) {
-      if (P->es == 4)
-        repack_kernel<float><<<nb_r, 128, 0, s>>>((const float*)P->right, (float*)P->rpad, P->jobs + nl,
-                                                  P->max_rows);
-      else
-        repack_kernel<double><<<nb_r, 128, 0, s>>>((const double*)P->right, (double*)P->rpad, P->jobs + nl,
-                                                   P->max_rows);
-    }
+    if (P->es == 4)
+      repack_kernel<float><<<v.repack_blocks, 128, 0, s>>>((const float*)P->left, (float*)P->lpad,
+                                                           (const float*)P->right, (float*)P->rpad, v.jobs, v.first,
+                                                           v.n_left, v.n_jobs);
+    else
+      repack_kernel<double><<<v.repack_blocks, 128, 0, s>>>((const double*)P->left, (double*)P->lpad,
+                                                            (const double*)P->right, (double*)P->rpad, v.jobs,
+                                                            v.first, v.n_left, v.n_jobs);
     if (cudaMemsetAsync(P->queue, 0, sizeof(unsigned int), s) != cudaSuccess)
       st = fail(XC_ERR_CUDA, "ragged capture: queue reset failed");
     if (st == XC_OK) st = ragged_launch(P->dtype, shape, rl, s);
   }
+  if (forked && st == XC_OK && split.size() < tc_pairs.size())
+    st = fe::ragged_fft_enqueue(P->ffts[route], P->tc_streams, P->n_streams, P->fork, P->joins);
   for (int k = 0; k < P->n_streams && forked; ++k) {
-    if (per_stream[k].empty()) continue;
+    if (k > 0 && per_stream[k].empty()) continue;
     const cudaStream_t sk = P->tc_streams[k];
     for (size_t i : per_stream[k]) {
       if (st != XC_OK) break;
@@ -326,8 +389,8 @@ xc_status build_variant(RaggedPlanImpl* P, int index) {
       const xc_matrix_desc& L = P->lefts[d.left];
       const xc_matrix_desc& R = P->rights[d.right];
       st = tc_correlate((const float*)P->left + L.offset, (const float*)P->right + R.offset,
-                        (float*)P->out + d.out_off, Geometry{d.Hl, d.Wl, d.Hr, d.Wr, d.Hl + d.Hr - 1, d.Wl + d.Wr - 1},
-                        pm1, P->tc_ws[k], P->tc_ws_bytes, sk, false, kTcItemRows, kTcItemRows);
+                        (float*)P->out + d.out_off, pair_geometry(d), pm1, P->tc_ws[k], P->tc_ws_bytes, sk, false,
+                        kTcItemRows, kTcItemRows);
     }
     // every forked stream joins, also after an error, so that the capture can end
     cudaEventRecord(P->joins[k], sk);
@@ -388,7 +451,7 @@ std::string signature(const RaggedPlanImpl* P) {
   std::ostringstream ss;
   ss << prop.name << "|dtype=" << (int)P->dtype << "|pairs=" << P->pairs.size() << "|mac_log2="
      << (int)std::floor(std::log2(std::max(1.0, mac / std::max<size_t>(1, P->pairs.size())))) << "|variants="
-     << P->n_shapes << "x" << P->n_routes;
+     << P->n_shapes << "x" << P->n_routes << "|routed=fft";
   return ss.str();
 }
 
@@ -424,6 +487,7 @@ xc_status ragged_plan_create(RaggedPlanImpl** out, xc_dtype dtype, const void* d
   P->n_routes = dtype == XC_F32 && tc_routes_enabled() ? kRaggedRoutes : 1;
   P->n_streams = tc_stream_count();
   P->variants.resize((size_t)P->n_shapes * P->n_routes);
+  P->ffts.resize(P->n_routes);
   P->maps_for_shape.assign(2 * (size_t)P->n_shapes, nullptr);
   // multiply-adds of every pair, and whether the split path takes it
   {
@@ -436,6 +500,7 @@ xc_status ragged_plan_create(RaggedPlanImpl** out, xc_dtype dtype, const void* d
       P->pair_mac.push_back((double)L.rows * L.cols * R.rows * R.cols);
       const Geometry g = make_geometry(xc_size2{L.cols, L.rows}, xc_size2{R.cols, R.rows});
       P->tc_ok.push_back(dtype == XC_F32 && tc_workspace_size(g, pm1, false) > 0 ? 1 : 0);
+      P->fft_ok.push_back(dtype == XC_F32 && fe::ragged_fft_takes(g) ? 1 : 0);
     }
   }
   auto cleanup = [&](xc_status s) {
@@ -444,13 +509,12 @@ xc_status ragged_plan_create(RaggedPlanImpl** out, xc_dtype dtype, const void* d
   };
 
   // padded copies and the repack jobs (lefts first, then rights)
-  std::vector<CopyJob> jobs;
+  std::vector<CopyJob>& jobs = P->jobs;
   long long off = 0;
   for (const auto& m : P->lefts) {
     const int pitch = (int)pitch_of((int)m.cols, P->es);
     jobs.push_back(CopyJob{(long long)m.offset, off, (int)m.rows, (int)m.cols, pitch});
     off += (long long)pitch * m.rows;
-    P->max_rows = std::max(P->max_rows, (int)m.rows);
   }
   const long long lbytes = off * (long long)P->es;
   off = 0;
@@ -458,16 +522,11 @@ xc_status ragged_plan_create(RaggedPlanImpl** out, xc_dtype dtype, const void* d
     const int pitch = (int)pitch_of((int)m.cols, P->es);
     jobs.push_back(CopyJob{(long long)m.offset, off, (int)m.rows, (int)m.cols, pitch});
     off += (long long)pitch * m.rows;
-    P->max_rows = std::max(P->max_rows, (int)m.rows);
   }
   const long long rbytes = off * (long long)P->es;
-  P->n_jobs = (int)jobs.size();
   if (cudaMalloc(&P->lpad, lbytes) != cudaSuccess || cudaMalloc(&P->rpad, rbytes) != cudaSuccess ||
-      cudaMalloc(&P->jobs, sizeof(CopyJob) * jobs.size()) != cudaSuccess ||
       cudaMalloc(&P->queue, sizeof(unsigned int)) != cudaSuccess)
     return cleanup(fail(XC_ERR_CUDA, "device allocation for the ragged plan failed"));
-  if (cudaMemcpy(P->jobs, jobs.data(), sizeof(CopyJob) * jobs.size(), cudaMemcpyHostToDevice) != cudaSuccess)
-    return cleanup(fail(XC_ERR_CUDA, "upload of the repack table failed"));
   if (cudaStreamCreateWithFlags(&P->capture_stream, cudaStreamNonBlocking) != cudaSuccess)
     return cleanup(fail(XC_ERR_CUDA, "stream creation failed"));
   device_flags();  // resolve the flag word's address outside any stream capture
@@ -587,7 +646,11 @@ void ragged_plan_destroy(RaggedPlanImpl* P) {
     if (v.exec) cudaGraphExecDestroy(v.exec);
     if (v.graph) cudaGraphDestroy(v.graph);
     cudaFree(v.tiles);
+    cudaFree(v.jobs);
+    cudaFree(v.first);
   }
+  for (fe::RaggedFft& f : P->ffts) fe::ragged_fft_release(&f);
+  cudaFree(P->fft_ws);
   for (void* m : P->maps_for_shape) cudaFree(m);
   for (int k = 0; k < kMaxTcStreams; ++k) {
     cudaFree(P->tc_ws[k]);
@@ -598,7 +661,6 @@ void ragged_plan_destroy(RaggedPlanImpl* P) {
   cudaFree(P->dpairs);
   cudaFree(P->lpad);
   cudaFree(P->rpad);
-  cudaFree(P->jobs);
   cudaFree(P->queue);
   if (P->capture_stream) cudaStreamDestroy(P->capture_stream);
   delete P;
