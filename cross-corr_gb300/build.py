@@ -27,7 +27,7 @@ INCLUDE = os.path.join(ROOT, "include")
 ARCH = ["-gencode", "arch=compute_103a,code=sm_103a"]
 NVCC_FLAGS = ["-O3", "-std=c++17", "-lineinfo", "-Xcompiler", "-fPIC", "--expt-relaxed-constexpr",
               "-I" + INCLUDE, "-I" + CSRC]
-CUDA_SOURCES = ["xc_runtime.cu", "direct_simt.cu", "ragged.cu", "fft_glue.cu", "fft_pipeline.cu", "tc_bf16x3.cu",
+CUDA_SOURCES = ["xc_runtime.cu", "direct_simt.cu", "direct_cyclic.cu", "ragged.cu", "fft_glue.cu", "fft_pipeline.cu", "tc_bf16x3.cu",
                 "mlp.cu", "api.cu", "fft_engine.cu", "fft_rows_f32.cu", "fft_cols_f32.cu", "fft_cols_f32_long.cu",
                 "fft_rows_f64.cu", "fft_cols_f64.cu", "fft_cols_f64_long.cu", "ragged_fft.cu"]
 CLI_SOURCES = ["main.cpp", "data_array.cpp", "json_args.cpp", "algorithms.cpp"]

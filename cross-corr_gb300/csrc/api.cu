@@ -508,6 +508,9 @@ xc_status xc_correlate(xc_mode mode, xc_dtype dtype, xc_method method, const voi
     double ms = 0.0;
     XC_TRY(xc_autotune_algorithm(mode, dtype, d_left, left, n_left, d_right, right, n_right, d_out, stream, &a, &ms));
   }
+  // the plain kernel's own choice of form is the faster one where the
+  // selector's timings (of its tiled forms) favour the plain kernel
+  if (method == XC_METHOD_AUTO && a.method == XC_METHOD_DIRECT) a.tile = 0;
   if (a.method != XC_METHOD_DIRECT && a.method != XC_METHOD_FFT && a.method != XC_METHOD_TC_BF16X3 &&
       a.method != XC_METHOD_TC_TF32X3)
     return fail(XC_ERR_INVALID_ARGUMENT, "unknown method");

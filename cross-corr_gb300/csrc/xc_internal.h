@@ -62,6 +62,12 @@ xc_status direct_launch(xc_dtype dtype, const void* left, const void* right, voi
                         const PairMap& pm, cudaStream_t stream, int force_loader /* -1 auto, 0 cp.async, 1 TMA */,
                         DirectAccumulate acc = DirectAccumulate::kAuto, int tile = 0);
 
+// The same by cyclic column classes (direct_cyclic.cu); `add`: into an output
+// the caller zeroed.  *taken is false, and nothing is launched, when the rows
+// are too wide for it.
+xc_status direct_cyclic(xc_dtype dtype, const void* left, const void* right, void* out, const Geometry& g,
+                        const PairMap& pm, cudaStream_t stream, bool add, bool* taken);
+
 // Ragged batches (ragged.cu drives direct_simt.cu's persistent mode).
 struct RaggedTile {     // one tile of shifts of one pair
   int pair;
