@@ -126,13 +126,14 @@ struct TcCfg {
   static constexpr int kCm = TF ? 4 : 8;            // elements per 16-byte core-matrix row
   static constexpr int kQ = TF ? kTQTf32 : kTQBf16;  // core matrices in T
   static constexpr int kTBytes = kQ * 128;          // one plane of T
+  static constexpr int kXWords = TF ? kXLen : kXLen / 2;  // staged row, one part, 32-bit words
   static constexpr int kTransW = TF ? 16 : 32;
   static constexpr int kTransBytes = kEpiWarps * 32 * (kTransW + 1) * 4;
   static constexpr int kOffBytes = kEpiWarps * 32 * 8;
   static constexpr int kTabBytes = 2 * (kMaxKSteps + 1) * 4 + 8;  // the issuers' K-step windows
-  static constexpr int kSmem = 1024 + kStages * kStageBytes + 4 * kTBytes + 4 * kXLen * 4 + kTransBytes +
+  static constexpr int kSmem = 1024 + kStages * kStageBytes + 4 * kTBytes + 4 * kXWords * 4 + kTransBytes +
                                kOffBytes + kTabBytes + kBarBytes;
-  static_assert(kCm * (kQ - 1) + 7 + kCm - 1 < kXLen, "T reads inside the staged row");
+  static_assert(kCm * (kQ - 1) + 7 + kCm <= kXLen, "T reads inside the staged row");
 };
 
 struct TcParams {
@@ -154,6 +155,7 @@ struct TcParams {
                     // covers [512 xp + h half_w, 512 xp + (h+1) half_w)
   int nkc;          // 128-byte column chunks of a whole k-part (64 BF16 or 32 TF32 columns each)
   int kstep;        // columns per K-step: 16 (BF16) or 8 (TF32)
+  int nq;           // core matrices of the Toeplitz buffer the windows reach
   const int* flush_tab;  // drain TMEM every this many left rows, per (left matrix, partner group)
   int chunk_rows;   // left rows per work item (a longer row range is split over items)
   const int* items;  // non-empty work items, most left rows first (tc_item encoding)
@@ -463,8 +465,8 @@ __global__ void __launch_bounds__(kThreads, 1)
       reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   unsigned char* a_tiles = smem;                                       // kStages x (128 rows x 128 B)
   unsigned char* t_buf = a_tiles + C::kStages * kStageBytes;           // [row buffer][hi, lo] Toeplitz core matrices
-  float* xs = reinterpret_cast<float*>(t_buf + 4 * C::kTBytes);        // [row buffer][hi, lo] x kXLen staged row
-  float* trans = xs + 4 * kXLen;                                       // [epilogue warp] transpose tile
+  uint32_t* xs = reinterpret_cast<uint32_t*>(t_buf + 4 * C::kTBytes);  // [row buffer][hi, lo] x kXWords staged row
+  float* trans = reinterpret_cast<float*>(xs + 4 * C::kXWords);        // [epilogue warp] transpose tile
   long long* offs = reinterpret_cast<long long*>(trans + kEpiWarps * 32 * (C::kTransW + 1));  // [warp][lane row]
   uint32_t* ktab_all = reinterpret_cast<uint32_t*>(offs + kEpiWarps * 32);  // [half][K-step, then reset]
   uint64_t* bars = reinterpret_cast<uint64_t*>(ktab_all + 2 * (kMaxKSteps + 1) + 2);
@@ -669,76 +671,103 @@ __global__ void __launch_bounds__(kThreads, 1)
   } else if (warp < 2 + kBuilderWarps) {
     // ------------------------------------------------------------ Toeplitz builders
     // Per left row: stage the centred, split row X[i] = Lp[s0 + kbase + i]
-    // (hi and lo parts; Lp[j] = L[a][j - (Wr-1)], zero outside the row), then write the
-    // core-matrix buffer T[q][r][t] = X[kCm q + r + t] of both parts into the
-    // free row buffer.
+    // (hi and lo parts; Lp[j] = L[a][j - (Wr-1)], zero outside the row), packed
+    // as the operand type, then write the core-matrix buffer
+    // T[q][r][t] = X[kCm q + r + t] of both parts into the free row buffer: the
+    // p.nq core matrices this launch's windows reach.  The next row's values
+    // (the next item's first row at an item's end) are loaded before the
+    // current row's buffer is built, so their latency passes under it.  With
+    // all 98 (194) core matrices built per row from single FP32 values the
+    // builders, not the tensor cores, set the pace of narrow problems:
+    // n_to_m 8 x 32 of 64x64, kernel 134 us against TCNEW1 now.
     const int bt = threadIdx.x - 64;  // 0..127
-    constexpr int kChunks = 2 * C::kQ * 8;  // 16-byte rows of T, both parts
+    constexpr int kPairs = (kXLen / 2 + 32 * kBuilderWarps - 1) / (32 * kBuilderWarps);  // element pairs per thread
+    const int n_pairs = ((p.nq - 1) * C::kCm + 7 + C::kCm + 1) / 2;  // X[0 .. kCm (nq - 1) + 7 + kCm)
+    float pv[2 * kPairs];
+    float mu = 0.0f;
+    // row `row` of item w into registers; mu stands for the zeros outside
+    const auto fetch = [&](const TcItem& w, int row) {
+      const float* src = p.left + ((long long)w.l * p.Hl + w.a_lo + row) * p.Wl;
+      const int x_off = w.s0 + w.kbase - (p.Wr - 1);  // left column of X[0]
+      mu = __ldg(p.mu_left + w.l);
+#pragma unroll
+      for (int u = 0; u < kPairs; ++u) {
+        const int i = bt + u * 32 * kBuilderWarps, x = x_off + 2 * i;
+        pv[2 * u] = i < n_pairs && x >= 0 && x < p.Wl ? __ldg(src + x) : mu;
+        pv[2 * u + 1] = i < n_pairs && x + 1 >= 0 && x + 1 < p.Wl ? __ldg(src + x + 1) : mu;
+      }
+    };
     int rows_done = 0;
     bool ok = true;
-    for (long long round = 0; round < n_round; ++round) {
-      TcItem w;
-      if (!round_item(p, n_items, round, &w)) continue;
-      const float* lrow_base = p.left + (long long)w.l * p.Hl * p.Wl;
-      const float mu = __ldg(p.mu_left + w.l);
-      const int x_off = w.s0 + w.kbase - (p.Wr - 1);  // left column of X[0]
-      int ai = 0;
-      for (; ai < w.n_rows; ++ai, ++rows_done) {
-        const int rbuf = rows_done & 1;
-        float* xh = xs + rbuf * (2 * kXLen);
-        float* xl = xh + kXLen;
-        const float* src = lrow_base + (long long)(w.a_lo + ai) * p.Wl;
-        for (int i = bt; i < kXLen; i += 32 * kBuilderWarps) {
-          const int x = x_off + i;
-          const float v = (x >= 0 && x < p.Wl) ? __ldg(src + x) - mu : 0.0f;
-          float hv, lv;
-          if constexpr (TF) {
-            hv = tf32_round(v);
-            lv = tf32_round(v - hv);
-          } else {
-            hv = __bfloat162float(__float2bfloat16_rn(v));
-            lv = v - hv;
-          }
-          xh[i] = hv;
-          xl[i] = lv;
-        }
-        // the staged row is complete; the builder threads also leave together here
-        if (bar_red_or(!ok, 1, 32 * kBuilderWarps)) {
-          ok = false;
-          break;
-        }
-        bool wt = wait_or_abort_sleep(&r_empty[rbuf], ((rows_done >> 1) & 1) ^ 1, abort_flag, p.flags, 15);
-        ok = __all_sync(0xffffffffu, wt);
-        if (ok) {
-          unsigned char* tb = t_buf + rbuf * (2 * C::kTBytes);
-          for (int c = bt; c < kChunks; c += 32 * kBuilderWarps) {
-            const int part = c / (C::kQ * 8), q = (c >> 3) % C::kQ, r = c & 7;
-            const float* x = (part ? xl : xh) + C::kCm * q + r;
-            uint4 v;
-            if constexpr (TF) {
-              v.x = __float_as_uint(x[0]);
-              v.y = __float_as_uint(x[1]);
-              v.z = __float_as_uint(x[2]);
-              v.w = __float_as_uint(x[3]);
-            } else {
-              auto pk = [](float lo_half, float hi_half) {
-                const __nv_bfloat162 b = __floats2bfloat162_rn(lo_half, hi_half);
-                return *reinterpret_cast<const uint32_t*>(&b);
-              };
-              v.x = pk(x[0], x[1]);
-              v.y = pk(x[2], x[3]);
-              v.z = pk(x[4], x[5]);
-              v.w = pk(x[6], x[7]);
-            }
-            *reinterpret_cast<uint4*>(tb + part * C::kTBytes + q * 128 + r * 16) = v;
-          }
-          // generic-proxy writes become visible to the tensor core's reads
-          fence_proxy_async_shared();
-          __syncwarp();
-          if (lane == 0) mbar_arrive(&r_full[rbuf]);  // one arrival per warp
+    TcItem w;
+    long long round = 0;
+    const auto next_item = [&]() {  // the first item from `round` on
+      for (; round < n_round; ++round)
+        if (round_item(p, n_items, round, &w)) return true;
+      return false;
+    };
+    bool have = next_item();
+    if (have) fetch(w, 0);
+    for (int ai = 0; have; ++rows_done) {
+      const int rbuf = rows_done & 1;
+      uint32_t* xh = xs + rbuf * (2 * C::kXWords);
+      uint32_t* xl = xh + C::kXWords;
+#pragma unroll
+      for (int u = 0; u < kPairs; ++u) {
+        const int i = bt + u * 32 * kBuilderWarps;
+        if (i >= n_pairs) continue;
+        const float v0 = pv[2 * u] - mu, v1 = pv[2 * u + 1] - mu;
+        if constexpr (TF) {
+          const float h0 = tf32_round(v0), h1 = tf32_round(v1);
+          reinterpret_cast<float2*>(xh)[i] = make_float2(h0, h1);
+          reinterpret_cast<float2*>(xl)[i] = make_float2(tf32_round(v0 - h0), tf32_round(v1 - h1));
+        } else {
+          const __nv_bfloat162 h = __floats2bfloat162_rn(v0, v1);
+          const __nv_bfloat162 l = __floats2bfloat162_rn(v0 - __low2float(h), v1 - __high2float(h));
+          xh[i] = *reinterpret_cast<const uint32_t*>(&h);
+          xl[i] = *reinterpret_cast<const uint32_t*>(&l);
         }
       }
-      if (ai < w.n_rows) break;  // a failed wait: every builder left at the same barrier
+      if (++ai == w.n_rows) {
+        ai = 0;
+        ++round;
+        have = next_item();
+      }
+      if (have) fetch(w, ai);
+      // the staged row is complete; the builder threads also leave together here
+      if (bar_red_or(!ok, 1, 32 * kBuilderWarps)) break;
+      bool wt = wait_or_abort_sleep(&r_empty[rbuf], ((rows_done >> 1) & 1) ^ 1, abort_flag, p.flags, 15);
+      ok = __all_sync(0xffffffffu, wt);
+      if (!ok) continue;  // to the next row's barrier, where every builder leaves (or past the last row)
+      unsigned char* tb = t_buf + rbuf * (2 * C::kTBytes);
+#pragma unroll 2
+      for (int c = bt; c < p.nq * 8; c += 32 * kBuilderWarps) {
+        // 16-byte row r of core matrix q: elements kCm q + r .. + kCm - 1 of X
+        const int q = c >> 3, r = c & 7;
+        uint4 vh, vl;
+        if constexpr (TF) {
+          const uint32_t* sh = xh + 4 * q + r;
+          const uint32_t* sl = xl + 4 * q + r;
+          vh = make_uint4(sh[0], sh[1], sh[2], sh[3]);
+          vl = make_uint4(sl[0], sl[1], sl[2], sl[3]);
+        } else {
+          // two elements per word: an odd r takes the halves of five words
+          const uint32_t* sh = xh + 4 * q + (r >> 1);
+          const uint32_t* sl = xl + 4 * q + (r >> 1);
+          const uint32_t sel = (r & 1) ? 0x5432u : 0x3210u;
+          const uint32_t h1 = sh[1], h2 = sh[2], h3 = sh[3], l1 = sl[1], l2 = sl[2], l3 = sl[3];
+          vh = make_uint4(__byte_perm(sh[0], h1, sel), __byte_perm(h1, h2, sel), __byte_perm(h2, h3, sel),
+                          __byte_perm(h3, sh[4], sel));
+          vl = make_uint4(__byte_perm(sl[0], l1, sel), __byte_perm(l1, l2, sel), __byte_perm(l2, l3, sel),
+                          __byte_perm(l3, sl[4], sel));
+        }
+        *reinterpret_cast<uint4*>(tb + q * 128 + r * 16) = vh;
+        *reinterpret_cast<uint4*>(tb + C::kTBytes + q * 128 + r * 16) = vl;
+      }
+      // generic-proxy writes become visible to the tensor core's reads
+      fence_proxy_async_shared();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&r_full[rbuf]);  // one arrival per warp
     }
   } else if (warp < 2 + kBuilderWarps + kEpiWarps) {
     // ------------------------------------------------------------ epilogue
@@ -1585,6 +1614,7 @@ xc_status tc_correlate_banded(const float* left, const float* right, float* out,
   prm.half_w = t.half_w;
   prm.nkc = t.nkc;
   prm.kstep = t.kstep;
+  prm.nq = tc_core_matrices(t.half_w, g.Wr, tf32);
   prm.flush_tab = w.flush;
   prm.chunk_rows = t.chunk_rows;
   prm.n_chunks = t.n_chunks;

@@ -1,0 +1,37 @@
+// Checks on the CPU that the Toeplitz buffer of a launch (tc_core_matrices in
+// tc_schedule.h, the core matrices the builder warps write) holds everything
+// the MMA windows read: for every case "Wl Wr tf32" on standard input prints
+// "ok <core matrices> <largest read + 1>" or "FAIL".
+#include <algorithm>
+#include <cstdio>
+
+#include "tc_schedule.h"
+
+using namespace xc;
+
+int main() {
+  int Wl, Wr, tf;
+  while (std::scanf("%d %d %d", &Wl, &Wr, &tf) == 3) {
+    const int Sx = Wl + Wr - 1;
+    const TcParts t = tc_parts(Sx, Wr, tf != 0);
+    const int nq = tc_core_matrices(t.half_w, Wr, tf != 0);
+    // one group of eight shifts is one core matrix (BF16) or two (TF32), one
+    // K-step two
+    const int group = tf ? 2 : 1;
+    int most = 0;
+    for (int xp = 0; xp < t.n_xparts; ++xp)
+      for (int kp = 0; kp < t.n_kparts; ++kp)
+        for (int h = 0; h < 2; ++h)
+          for (int j = -1; j < 256 / t.kstep; ++j) {
+            const int kbase = 256 * kp, k0 = kbase + std::max(0, j) * t.kstep;
+            const uint32_t e = window_of(Sx, Wl, Wr, t.half_w, t.kstep, 512 * xp, kbase, h, k0, j < 0);
+            if (!((e >> 14) & 1u)) continue;
+            const int n = (int)((e >> 9) & 31u) * 16;
+            most = std::max(most, (int)(e >> 16) + (n / 8 - 1) * group + 1 + 1);
+          }
+    const int kq = tf ? kTQTf32 : kTQBf16;
+    if (most <= nq && nq <= kq) std::printf("ok %d %d\n", nq, most);
+    else std::printf("FAIL %d %d of %d\n", nq, most, kq);
+  }
+  return 0;
+}
