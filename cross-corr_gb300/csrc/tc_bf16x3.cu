@@ -120,11 +120,14 @@ constexpr int kMaxKSteps = 32;             // K-steps of a 256-column right row 
 // through shared memory (rows padded by one float): 32 for BF16, so that one
 // reduction instruction covers one output row's 32 shifts (a 128-byte line);
 // 16 for TF32, whose larger Toeplitz buffer leaves less room.
-template <bool TF>
+// RS (rowsplit, at most 256 shifts): a shorter T (256 shifts and 256 columns)
+// leaves room for six stages, three for each issuer.
+template <bool TF, bool RS>
 struct TcCfg {
-  static constexpr int kStages = TF ? 4 : 5;
+  static constexpr int kStages = RS ? 6 : TF ? 4 : 5;
+  static constexpr int kRing = RS ? kStages / 2 : kStages;  // stages of one issuer's ring
   static constexpr int kCm = TF ? 4 : 8;            // elements per 16-byte core-matrix row
-  static constexpr int kQ = TF ? kTQTf32 : kTQBf16;  // core matrices in T
+  static constexpr int kQ = RS ? 512 / kCm : TF ? kTQTf32 : kTQBf16;  // core matrices in T
   static constexpr int kTBytes = kQ * 128;          // one plane of T
   static constexpr int kXWords = TF ? kXLen : kXLen / 2;  // staged row, one part, 32-bit words
   static constexpr int kTransW = TF ? 16 : 32;
@@ -153,6 +156,9 @@ struct TcParams {
   int n_kparts;
   int half_w;       // shifts per half (a multiple of 16, at most 256): half h of x-part xp
                     // covers [512 xp + h half_w, 512 xp + (h+1) half_w)
+  int rowsplit;     // 1 (Sx <= 256): issuer h takes every other left row, each over all
+                    // shifts (half_w of them) in its own accumulator, instead of a half of
+                    // the shifts of every row
   int nkc;          // 128-byte column chunks of a whole k-part (64 BF16 or 32 TF32 columns each)
   int kstep;        // columns per K-step: 16 (BF16) or 8 (TF32)
   int nq;           // core matrices of the Toeplitz buffer the windows reach
@@ -329,7 +335,23 @@ __device__ __forceinline__ bool bar_red_or(bool v, int id, int nthreads) {
 // (window_of in tc_schedule.h) for this launch's geometry.
 __host__ __device__ __forceinline__ uint32_t kstep_window(const TcParams& p, int s0, int kbase, int h, int k0,
                                                           bool reset) {
+  if (p.rowsplit != 0) {  // the whole shift range, in issuer h's columns
+    const uint32_t e = window_of(p.Sx, p.Wl, p.Wr, p.half_w, p.kstep, s0, kbase, 0, k0, reset);
+    return e == 0 ? 0u : e + (uint32_t)(h * kHalfCols);
+  }
   return window_of(p.Sx, p.Wl, p.Wr, p.half_w, p.kstep, s0, kbase, h, k0, reset);
+}
+
+// Rows of an item that issuer h works on: every row, or (rowsplit) the rows
+// ai = first, first + 2, ... of its parity; `row0` counts the CTA's rows before
+// the item.
+struct OwnRows {
+  int first, count;
+};
+__device__ __forceinline__ OwnRows own_rows(bool rowsplit, int h, int row0, int n_rows) {
+  if (!rowsplit) return {0, n_rows};
+  const int first = (h - row0) & 1;
+  return {first, (n_rows - first + 1) >> 1};
 }
 
 // One work item: every shift of one (left matrix, partner group, row-shift
@@ -443,9 +465,10 @@ __device__ __forceinline__ bool round_item(const TcParams& p, long long n_live, 
 
 __device__ __forceinline__ long long n_rounds(long long n_live) { return (n_live + gridDim.x - 1) / gridDim.x; }
 
-// Accumulator windows of an item: half 0 drains after every `flush` left
-// rows, half 1 first after (flush + 1) / 2 rows and then every `flush`; both
-// drain after the item's last row.  True when row ai (0-based) ends a window.
+// Accumulator windows of an item: half (issuer) 0 drains after every `flush`
+// of its left rows, half 1 first after (flush + 1) / 2 and then every `flush`;
+// both drain after their last row of the item.  True when row ai (0-based,
+// among the n_rows of the half) ends a window.
 __device__ __forceinline__ bool window_end(int h, int ai, int n_rows, int flush) {
   if (ai == n_rows - 1) return true;
   const int off = h == 0 ? 0 : flush - (flush + 1) / 2;
@@ -455,11 +478,11 @@ __device__ __forceinline__ bool window_end(int h, int ai, int n_rows, int flush)
 
 // 23 warps: at most 6 on one SM sub-partition, whose 16K registers cap a
 // thread at 80.  TF: TF32 operands (K = 8 per MMA) instead of BF16 (K = 16).
-template <bool TF>
+template <bool TF, bool RS>
 __global__ void __launch_bounds__(kThreads, 1)
     tc_kernel(const __grid_constant__ CUtensorMap map_hi, const __grid_constant__ CUtensorMap map_lo,
               const __grid_constant__ TcParams p) {
-  using C = TcCfg<TF>;
+  using C = TcCfg<TF, RS>;
   extern __shared__ __align__(1024) unsigned char smem_raw[];
   unsigned char* smem =
       reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
@@ -489,14 +512,16 @@ __global__ void __launch_bounds__(kThreads, 1)
   const long long n_items = *p.n_live;
   const long long n_round = n_rounds(n_items);
   if (threadIdx.x == 0) {
-    // consumed barriers take one commit from each issuer
+    // consumed barriers take one commit from each issuer that reads the stage
+    // or row
+    const uint32_t readers = RS ? 1 : 2;
     for (int s = 0; s < C::kStages; ++s) {
       mbar_init(&a_full[s], 1);
-      mbar_init(&a_empty[s], 2);
+      mbar_init(&a_empty[s], readers);
     }
     for (int s = 0; s < 2; ++s) {
       mbar_init(&r_full[s], kBuilderWarps);
-      mbar_init(&r_empty[s], 2);
+      mbar_init(&r_empty[s], readers);
       mbar_init(&t_full[s], 1);
       mbar_init(&t_empty[s], kEpiWarps);
       mbar_init(&mma_done[s], 1);
@@ -521,17 +546,20 @@ __global__ void __launch_bounds__(kThreads, 1)
     // ------------------------------------------------------------ producer
     // per (row, column chunk): the hi plane, then the lo plane
     if (lane == 0) {
-      int it = 0;
+      int its[2] = {0, 0};  // stages filled so far, per ring
+      int ring = 0;         // rowsplit: rows go to the issuers' rings in turn
       bool ok = true;
       for (long long round = 0; round < n_round && ok; ++round) {
         TcItem w;
         if (!round_item(p, n_items, round, &w)) continue;
         for (int ai = 0; ai < w.n_rows && ok; ++ai) {
           const int a = w.a_lo + ai;
+          int it = RS && ring ? its[1] : its[0];
+          const int base = RS ? ring * C::kRing : 0;
           for (int kc = 0; kc < w.nkc && ok; ++kc) {
             for (int pl = 0; pl < 2; ++pl, ++it) {
-              const int s = it % C::kStages;
-              if (!wait_or_abort_sleep(&a_empty[s], ((it / C::kStages) & 1) ^ 1, abort_flag, p.flags, 11)) {
+              const int s = base + it % C::kRing;
+              if (!wait_or_abort_sleep(&a_empty[s], ((it / C::kRing) & 1) ^ 1, abort_flag, p.flags, 11)) {
                 ok = false;
                 break;
               }
@@ -549,11 +577,15 @@ __global__ void __launch_bounds__(kThreads, 1)
               }
             }
           }
+          if (RS && ring) its[1] = it;
+          else its[0] = it;
+          if (RS) ring ^= 1;
         }
       }
       if (!ok) {
-        for (int q = max(0, it - C::kStages); q < it; ++q)
-          mbar_wait_bounded(&a_full[q % C::kStages], (q / C::kStages) & 1, 1u << 16);
+        for (int r = 0; r < (RS ? 2 : 1); ++r)
+          for (int q = max(0, its[r] - C::kRing); q < its[r]; ++q)
+            mbar_wait_bounded(&a_full[r * C::kRing + q % C::kRing], (q / C::kRing) & 1, 1u << 16);
       }
     }
   } else if (warp == 1 || warp == kIssuer1Warp) {
@@ -561,6 +593,11 @@ __global__ void __launch_bounds__(kThreads, 1)
     // Both walk the same items, rows and stages; issuer h issues the MMAs of
     // shift half h (its own accumulator, tensor-memory columns
     // [256 h, 256 h + 256)) and commits to the shared consumed barriers.
+    // With at most 256 shifts (RS) one MMA covers what the two halves
+    // took two for: issuer h then issues the MMAs of every other left row
+    // over all shifts, which halves their number (each costs an issuer about
+    // 79 cycles however narrow: n_to_m 8 x 32 of 64x64, kernel 103 us with
+    // halves, 92 with rows).
     const int h = warp == 1 ? 0 : 1;
     uint32_t* ktab = ktab_all + h * (kMaxKSteps + 1);
     {
@@ -572,7 +609,10 @@ __global__ void __launch_bounds__(kThreads, 1)
       const uint32_t idesc0 = TF ? idesc_tf32_f32(128, 0) : idesc_bf16_f32(128, 0);
       const uint32_t a_word = ((smem_u32(a_tiles) >> 4) & 0x3FFFu) | (1u << 16);
       const uint32_t t_word = ((smem_u32(t_buf) >> 4) & 0x3FFFu) | ((128u >> 4) << 16);
-      int s = 0, rb = 0;                      // stage, Toeplitz row buffer
+      constexpr int kRing = C::kRing;
+      const int ring_lo = RS ? h * kRing : 0;
+      int s = ring_lo, rb = RS ? h : 0;       // stage, Toeplitz row buffer
+      int row0 = 0;                           // the CTA's rows before the item
       uint32_t s_phase = 0, r_phase = 0, t_phase = 1;
       bool s_ready = false;                   // stage s seen landed ahead of time
       bool ok = true;
@@ -587,7 +627,7 @@ __global__ void __launch_bounds__(kThreads, 1)
         __syncwarp();
         if (lane == 0) {
         const uint32_t kres = ktab[kMaxKSteps];
-        const int n_rows = w.n_rows;
+        const int n_rows = RS ? own_rows(true, h, row0, w.n_rows).count : w.n_rows;
         const int flush = p.flush_tab[w.l * p.n_pgroups + w.p0 / p.P];
         int rows_in = 0;
         for (int ai = 0; ai < n_rows && ok; ++ai) {
@@ -619,8 +659,8 @@ __global__ void __launch_bounds__(kThreads, 1)
               tc_fence_after();
               {
                 // ask for the following stage now, use the answer after this one's MMAs
-                const int s2 = s + 1 == C::kStages ? 0 : s + 1;
-                s_ready = mbar_test_wait(&a_full[s2], s2 == 0 ? s_phase ^ 1u : s_phase);
+                const int s2 = s + 1 == ring_lo + kRing ? ring_lo : s + 1;
+                s_ready = mbar_test_wait(&a_full[s2], s2 == ring_lo ? s_phase ^ 1u : s_phase);
               }
               const uint32_t aw = a_word + (uint32_t)s * (kStageBytes >> 4);
 #pragma unroll
@@ -645,14 +685,18 @@ __global__ void __launch_bounds__(kThreads, 1)
               }
               mma_commit(&a_empty[s]);
               // next stage, without a branch
-              s = s + 1 == C::kStages ? 0 : s + 1;
-              s_phase ^= s == 0 ? 1u : 0u;
+              s = s + 1 == ring_lo + kRing ? ring_lo : s + 1;
+              s_phase ^= s == ring_lo ? 1u : 0u;
             }
           }
           if (!ok) break;
           mma_commit(&r_empty[rb]);
-          rb ^= 1;
-          if (rb == 0) r_phase ^= 1u;
+          if (RS) {
+            r_phase ^= 1u;  // every row of this issuer is in row buffer h
+          } else {
+            rb ^= 1;
+            if (rb == 0) r_phase ^= 1u;
+          }
           ++rows_in;
           if (window_end(h, ai, n_rows, flush)) {
             mma_commit(&t_full[h]);
@@ -660,6 +704,7 @@ __global__ void __launch_bounds__(kThreads, 1)
           }
         }
         }
+        if (RS) row0 += w.n_rows;
         ok = __shfl_sync(0xffffffffu, ok ? 1 : 0, 0) != 0;
       }
       // All MMAs issued by this thread must finish before TMEM is released.
@@ -679,7 +724,7 @@ __global__ void __launch_bounds__(kThreads, 1)
     // current row's buffer is built, so their latency passes under it.  With
     // all 98 (194) core matrices built per row from single FP32 values the
     // builders, not the tensor cores, set the pace of narrow problems:
-    // n_to_m 8 x 32 of 64x64, kernel 134 us against TCNEW1 now.
+    // n_to_m 8 x 32 of 64x64, kernel 134 us, 103 with this.
     const int bt = threadIdx.x - 64;  // 0..127
     constexpr int kPairs = (kXLen / 2 + 32 * kBuilderWarps - 1) / (32 * kBuilderWarps);  // element pairs per thread
     const int n_pairs = ((p.nq - 1) * C::kCm + 7 + C::kCm + 1) / 2;  // X[0 .. kCm (nq - 1) + 7 + kCm)
@@ -787,6 +832,7 @@ __global__ void __launch_bounds__(kThreads, 1)
     long long* my_off = offs + ew * 32;
     const int lgP = __ffs(p.P) - 1, lgDY = __ffs(p.DY) - 1;
     int drained0 = 0, drained1 = 0;  // drains of each half so far
+    int row0 = 0;                    // the CTA's rows before the item
     bool ok = true;
     for (long long round = 0; round < n_round && ok; ++round) {
       TcItem w;
@@ -816,7 +862,12 @@ __global__ void __launch_bounds__(kThreads, 1)
       const int flush = p.flush_tab[w.l * p.n_pgroups + w.p0 / p.P];
       for (int ai = 0; ai < w.n_rows && ok; ++ai) {
         for (int h = 0; h < 2; ++h) {
-          if (!window_end(h, ai, w.n_rows, flush)) continue;
+          if (RS) {
+            const OwnRows own = own_rows(RS, h, row0, w.n_rows);
+            if (((ai - own.first) & 1) || !window_end(h, (ai - own.first) >> 1, own.count, flush)) continue;
+          } else if (!window_end(h, ai, w.n_rows, flush)) {
+            continue;
+          }
           bool wt = wait_or_abort_sleep(&t_full[h], (h ? drained1 : drained0) & 1, abort_flag, p.flags, 16);
           if (h) ++drained1;
           else ++drained0;
@@ -826,8 +877,9 @@ __global__ void __launch_bounds__(kThreads, 1)
             break;
           }
           tc_fence_after();
-          const int sx_end = min(p.Sx, w.s0 + (h + 1) * p.half_w);  // this half's shifts end here
-          const int sx_base = w.s0 + h * p.half_w + 64 * cq;
+          const int first_sx = w.s0 + (RS ? 0 : h * p.half_w);
+          const int sx_end = min(p.Sx, first_sx + p.half_w);  // this accumulator's shifts end here
+          const int sx_base = first_sx + 64 * cq;
           const bool live = sx_base < sx_end;
           const uint32_t col0 = tmem_base + ((uint32_t)(q * 32) << 16) + (uint32_t)(h * kHalfCols + 64 * cq);
           // reductions of lane rows x TW shifts from the transpose tile: shift
@@ -890,6 +942,7 @@ __global__ void __launch_bounds__(kThreads, 1)
           }
         }
       }
+      if (RS) row0 += w.n_rows;
       if (p.band_done != nullptr) {
         // this thread's reductions become visible before the band count moves
         __threadfence();
@@ -1325,11 +1378,17 @@ __global__ void __launch_bounds__(256) correction_kernel(float* __restrict__ out
 }
 
 struct TcPlan {
-  int P, DY, mats_mode, half_w, nkc, kstep, es, pitch, n_chunks, chunk_rows, n_parts, n_kparts;
+  int P, DY, mats_mode, rowsplit, half_w, nkc, kstep, es, pitch, n_chunks, chunk_rows, n_parts, n_kparts;
   long long n_items;
   long long n_items_ws;  // items at 32-row chunks: the work list and schedule space of either form of launch
   int smem_bytes;
 };
+
+using TcKernel = void (*)(const CUtensorMap, const CUtensorMap, const TcParams);
+TcKernel tc_kernel_of(bool tf32, bool rowsplit) {
+  if (tf32) return rowsplit ? tc_kernel<true, true> : tc_kernel<true, false>;
+  return rowsplit ? tc_kernel<false, true> : tc_kernel<false, false>;
+}
 
 int chunk_rows_fixed();
 int sm_count();
@@ -1346,7 +1405,15 @@ bool tc_plan(const Geometry& g, const PairMap& pm, bool tf32, TcPlan* t, bool ba
   t->mats_mode = P >= 8 ? 1 : 0;
   // x-parts of 512 shifts (two halves), k-parts of 256 right columns
   const TcParts parts = tc_parts(g.Sx, g.Wr, tf32);
-  t->half_w = parts.half_w;
+  // One accumulator holds every shift: the issuers split the rows instead.
+  // BF16 rights of more than one column chunk only up to 208 shifts: with four
+  // or more stages a row, three stages per issuer hold less than a row (us,
+  // halves against rows: n_to_m 8 x 32 of 64x64 137 and 128, one_to_many
+  // 200x200 by 50x50 x 64 111 and 103, 100x100 x 64 138 and 128, n_to_m 4 x 4
+  // of 120x130 by 120x120 90 and 94; TF32 221 and 187, 170 and 147, 238 and
+  // 195, 142 and 124).
+  t->rowsplit = g.Sx <= kHalfCols && (tf32 || g.Wr <= 64 || g.Sx <= 208) ? 1 : 0;
+  t->half_w = t->rowsplit ? div_up(g.Sx, 16) * 16 : parts.half_w;
   t->n_kparts = parts.n_kparts;
   t->n_parts = parts.n_xparts * parts.n_kparts;
   t->es = tf32 ? 4 : 2;                 // bytes per operand element
@@ -1370,7 +1437,8 @@ bool tc_plan(const Geometry& g, const PairMap& pm, bool tf32, TcPlan* t, bool ba
   t->n_chunks = (int)div_up(span, (long long)t->chunk_rows);
   t->n_items = (long long)t->n_chunks * per_tile_key;
   t->n_items_ws = std::max(t->n_items, div_up(span, (long long)chunk32) * per_tile_key);
-  t->smem_bytes = tf32 ? TcCfg<true>::kSmem : TcCfg<false>::kSmem;
+  t->smem_bytes = tf32 ? (t->rowsplit ? TcCfg<true, true>::kSmem : TcCfg<true, false>::kSmem)
+                       : (t->rowsplit ? TcCfg<false, true>::kSmem : TcCfg<false, false>::kSmem);
   return t->smem_bytes <= 227 * 1024;
 }
 
@@ -1612,9 +1680,10 @@ xc_status tc_correlate_banded(const float* left, const float* right, float* out,
   prm.n_parts = t.n_parts;
   prm.n_kparts = t.n_kparts;
   prm.half_w = t.half_w;
+  prm.rowsplit = t.rowsplit;
   prm.nkc = t.nkc;
   prm.kstep = t.kstep;
-  prm.nq = tc_core_matrices(t.half_w, g.Wr, tf32);
+  prm.nq = tc_core_matrices(t.rowsplit ? t.half_w : 2 * t.half_w, g.Wr, tf32);
   prm.flush_tab = w.flush;
   prm.chunk_rows = t.chunk_rows;
   prm.n_chunks = t.n_chunks;
@@ -1700,7 +1769,7 @@ xc_status tc_correlate_banded(const float* left, const float* right, float* out,
 
   // persistent: one CTA per SM (about 205 KB of shared memory and all 512 TMEM
   // columns each), walking the list in snake order
-  auto kern = tf32 ? tc_kernel<true> : tc_kernel<false>;
+  const auto kern = tc_kernel_of(tf32, t.rowsplit != 0);
   XC_TRY(raise_smem_limit((const void*)kern, t.smem_bytes));
   const long long blocks = std::max(1LL, std::min<long long>(n_list, sm_count()));
   if (band_done) {
@@ -1730,7 +1799,7 @@ xc_status tc_prepare(const Geometry& g, const PairMap& pm, bool tf32) {
   const size_t corr_smem = corr_smem_bytes(g);
   if (corr_smem > 200 * 1024) return fail(XC_ERR_UNSUPPORTED, "split tensor-core paths: right matrices too wide");
   if (corr_smem > 48 * 1024) XC_TRY(raise_smem_limit((const void*)correction_kernel, (int)corr_smem));
-  XC_TRY(raise_smem_limit(tf32 ? (const void*)tc_kernel<true> : (const void*)tc_kernel<false>, t.smem_bytes));
+  XC_TRY(raise_smem_limit((const void*)tc_kernel_of(tf32, t.rowsplit != 0), t.smem_bytes));
   return XC_OK;
 }
 

@@ -42,14 +42,14 @@ inline TcParts tc_parts(int Sx, int Wr, bool tf32) {
   return t;
 }
 
-// Core matrices of the Toeplitz buffer that the windows of both halves reach:
-// a window at shift offset w - s0 and column offset k0 - kbase covers elements
-// X[(w - s0) + (k0 - kbase) ...) for N shifts and one K-step, at most
-// 2 half_w + the k-part's columns (whole K-steps) in all.
-inline int tc_core_matrices(int half_w, int Wr, bool tf32) {
+// Core matrices of the Toeplitz buffer that the windows of `shifts` shifts
+// reach: a window at shift offset w - s0 and column offset k0 - kbase covers
+// elements X[(w - s0) + (k0 - kbase) ...) for N shifts and one K-step, at most
+// the shifts (whole windows) + the k-part's columns (whole K-steps) in all.
+inline int tc_core_matrices(int shifts, int Wr, bool tf32) {
   const int kstep = tf32 ? 8 : 16, cm = tf32 ? 4 : 8;
   const int cols = ((Wr < 256 ? Wr : 256) + kstep - 1) / kstep * kstep;
-  return (2 * half_w + cols) / cm;
+  return (shifts + cols) / cm;
 }
 
 // The MMA window of half h and the K-step whose first right column is k0,
