@@ -245,6 +245,25 @@ __device__ __forceinline__ void mma_commit(uint64_t* bar) {
 __device__ __forceinline__ void tc_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ void tc_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
 
+// Programmatic dependent launch (launch_after): the next kernel may start
+// becoming resident; wait for the whole previous kernel.
+__device__ __forceinline__ void pdl_begin() {
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+}
+// Loads of what an earlier kernel may have written.  Not __ldg: the compiler
+// may move a non-coherent load above the wait; volatile assembly stays below.
+__device__ __forceinline__ float ld_after(const float* g) {
+  float v;
+  asm volatile("ld.global.f32 %0, [%1];" : "=f"(v) : "l"(g));
+  return v;
+}
+__device__ __forceinline__ float4 ld_after(const float4* g) {
+  float4 v;
+  asm volatile("ld.global.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "l"(g));
+  return v;
+}
+
 // 32 consecutive columns of this warp's 32 lanes: one register each.
 __device__ __forceinline__ void tmem_ld32(uint32_t taddr, float* v) {
   uint32_t r[32];
@@ -509,8 +528,6 @@ __global__ void __launch_bounds__(kThreads, 1)
   // r*G + G-1-c on odd rounds); every role walks the same items and keeps its
   // pipeline counters running across them, so the next item's loads and
   // MMAs overlap the previous item's final adds.
-  const long long n_items = *p.n_live;
-  const long long n_round = n_rounds(n_items);
   if (threadIdx.x == 0) {
     // consumed barriers take one commit from each issuer that reads the stage
     // or row
@@ -541,6 +558,9 @@ __global__ void __launch_bounds__(kThreads, 1)
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
+  pdl_begin();  // the barriers and tensor memory are set up under the previous kernel
+  const long long n_items = *p.n_live;
+  const long long n_round = n_rounds(n_items);
 
   if (warp == 0) {
     // ------------------------------------------------------------ producer
@@ -734,12 +754,12 @@ __global__ void __launch_bounds__(kThreads, 1)
     const auto fetch = [&](const TcItem& w, int row) {
       const float* src = p.left + ((long long)w.l * p.Hl + w.a_lo + row) * p.Wl;
       const int x_off = w.s0 + w.kbase - (p.Wr - 1);  // left column of X[0]
-      mu = __ldg(p.mu_left + w.l);
+      mu = p.mu_left[w.l];
 #pragma unroll
       for (int u = 0; u < kPairs; ++u) {
         const int i = bt + u * 32 * kBuilderWarps, x = x_off + 2 * i;
-        pv[2 * u] = i < n_pairs && x >= 0 && x < p.Wl ? __ldg(src + x) : mu;
-        pv[2 * u + 1] = i < n_pairs && x + 1 >= 0 && x + 1 < p.Wl ? __ldg(src + x + 1) : mu;
+        pv[2 * u] = i < n_pairs && x >= 0 && x < p.Wl ? ld_after(src + x) : mu;
+        pv[2 * u + 1] = i < n_pairs && x + 1 >= 0 && x + 1 < p.Wl ? ld_after(src + x + 1) : mu;
       }
     };
     int rows_done = 0;
@@ -1009,13 +1029,13 @@ __device__ __forceinline__ void sum_block(const PrepSide& sd_, int b) {
     const long long lo4 = lo >> 2, hi4 = hi >> 2;
 #pragma unroll 8
     for (long long i = lo4 + threadIdx.x; i < hi4; i += blockDim.x) {
-      const float4 x = __ldg(a4 + i);
+      const float4 x = ld_after(a4 + i);
       part += (x.x + x.y) + (x.z + x.w);
       part2 = fmaf(x.x, x.x, fmaf(x.y, x.y, fmaf(x.z, x.z, fmaf(x.w, x.w, part2))));
     }
   } else {
     for (long long i = lo + threadIdx.x; i < hi; i += blockDim.x) {
-      const float x = __ldg(a + i);
+      const float x = ld_after(a + i);
       part += x;
       part2 = fmaf(x, x, part2);
     }
@@ -1042,6 +1062,7 @@ __device__ __forceinline__ void sum_block(const PrepSide& sd_, int b) {
 }
 
 __global__ void __launch_bounds__(256) sum_kernel(const PrepSide a, const PrepSide b, unsigned a_blocks) {
+  pdl_begin();
   if (blockIdx.x < a_blocks)
     sum_block(a, (int)blockIdx.x);
   else
@@ -1137,7 +1158,7 @@ __device__ __forceinline__ void split_block(const PrepSide& sd_, int b, int bpm)
     if (vec && c0 + E <= W) {
 #pragma unroll
       for (int q = 0; q < E; q += 4) {
-        const float4 f = __ldg(reinterpret_cast<const float4*>(row + c0 + q));
+        const float4 f = ld_after(reinterpret_cast<const float4*>(row + c0 + q));
         v[q] = f.x;
         v[q + 1] = f.y;
         v[q + 2] = f.z;
@@ -1145,7 +1166,7 @@ __device__ __forceinline__ void split_block(const PrepSide& sd_, int b, int bpm)
       }
     } else {
 #pragma unroll
-      for (int q = 0; q < E; ++q) v[q] = c0 + q < W ? __ldg(row + c0 + q) : mv;
+      for (int q = 0; q < E; ++q) v[q] = c0 + q < W ? ld_after(row + c0 + q) : mv;
     }
     uint4 oh, ol;
     uint32_t* ph = reinterpret_cast<uint32_t*>(&oh);
@@ -1170,11 +1191,12 @@ __device__ __forceinline__ void split_block(const PrepSide& sd_, int b, int bpm)
   }
 }
 
+template <int NW>
 __device__ __forceinline__ void colsum_block(const PrepSide& sd_, int b) {
   const float* __restrict__ src = sd_.src;
   const int H = sd_.H, W = sd_.W;
   float* __restrict__ C = sd_.sat;
-  __shared__ float seg[8][32];
+  __shared__ float seg[NW][32];
   __shared__ float carry[32];
   const int strips = (W + 31) / 32;
   const int m = b / strips;
@@ -1191,13 +1213,13 @@ __device__ __forceinline__ void colsum_block(const PrepSide& sd_, int b) {
     carry[lane] = 0.0f;
     if (x < W) c[x] = 0.0f;
   }
-  for (int y0 = 0; y0 < H; y0 += 64) {
+  for (int y0 = 0; y0 < H; y0 += 8 * NW) {
     const int yb = y0 + 8 * w;
     float run[8];
     float acc = 0.0f;
 #pragma unroll
     for (int i = 0; i < 8; ++i) {
-      const float v = (x < W && yb + i < H) ? __ldg(a + (long long)(yb + i) * W + x) - mv : 0.0f;
+      const float v = (x < W && yb + i < H) ? ld_after(a + (long long)(yb + i) * W + x) - mv : 0.0f;
       acc += v;
       run[i] = acc;
     }
@@ -1213,7 +1235,7 @@ __device__ __forceinline__ void colsum_block(const PrepSide& sd_, int b) {
     __syncthreads();
     if (w == 0) {
       float t = 0.0f;
-      for (int j = 0; j < 8; ++j) t += seg[j][lane];
+      for (int j = 0; j < NW; ++j) t += seg[j][lane];
       carry[lane] += t;
     }
     __syncthreads();
@@ -1226,11 +1248,13 @@ __device__ __forceinline__ void colsum_block(const PrepSide& sd_, int b) {
 // split planes, then those of the accumulation windows: independent jobs in
 // one launch, the split filling the SMs the latency-bound column sums leave
 // idle and the work list's serial steps hidden under both.
-__global__ void __launch_bounds__(256) colsum_kernel(const PrepSide a, const PrepSide b, unsigned a_blocks,
+template <int NW>
+__global__ void __launch_bounds__(32 * NW) colsum_kernel(const PrepSide a, const PrepSide b, unsigned a_blocks,
                                                      unsigned ab_blocks, unsigned split_end, int split_bpm,
                                                      const WinArgs wa, const TcParams p, int list, int n_items,
                                                      int* items, int* n_live) {
   extern __shared__ int wl_cnt[];  // the work list's counts (its block only)
+  pdl_begin();
   if (list) {
     if (blockIdx.x == 0) {
       worklist_block(p, n_items, items, n_live, wl_cnt);
@@ -1239,9 +1263,9 @@ __global__ void __launch_bounds__(256) colsum_kernel(const PrepSide a, const Pre
   }
   const unsigned bid = blockIdx.x - (list ? 1u : 0u);
   if (bid < a_blocks)
-    colsum_block(a, (int)bid);
+    colsum_block<NW>(a, (int)bid);
   else if (bid < ab_blocks)
-    colsum_block(b, (int)(bid - a_blocks));
+    colsum_block<NW>(b, (int)(bid - a_blocks));
   else if (bid < split_end) {
     if (b.split_tf32)
       split_block<float>(b, (int)(bid - ab_blocks), split_bpm);
@@ -1257,6 +1281,7 @@ __global__ void __launch_bounds__(256) colsum_kernel(const PrepSide a, const Pre
 // The warp scans 32 consecutive columns at a time (coalesced), carrying the
 // running total (FP32 chains of at most W/32 + 5 terms).
 __global__ void __launch_bounds__(256) rowscan_kernel(const PrepSide a, const PrepSide b, unsigned a_blocks) {
+  pdl_begin();
   const bool first = blockIdx.x < a_blocks;
   const PrepSide& sd_ = first ? a : b;
   float* __restrict__ S = sd_.sat;
@@ -1305,13 +1330,14 @@ __global__ void __launch_bounds__(256) rowscan_kernel(const PrepSide a, const Pr
 // Staged floats: D_L (Wl + 1) and D_R (Wr + 1), each padded to 4.
 inline int corr_stage(int W) { return (W + 1 + 3) / 4 * 4; }
 constexpr int kCorrPartners = 8;  // partners per block, one warp each
-__global__ void __launch_bounds__(256) correction_kernel(float* __restrict__ out, const float* __restrict__ SL,
-                                                         const float* __restrict__ SR,
-                                                         const float* __restrict__ mu_l,
-                                                         const float* __restrict__ mu_r, int Hl, int Wl, int Hr,
+__global__ void __launch_bounds__(256) correction_kernel(float* out, const float* SL,
+                                                         const float* SR,
+                                                         const float* mu_l,
+                                                         const float* mu_r, int Hl, int Wl, int Hr,
                                                          int Wr, int Sy, int Sx, PairMap pm, int n_kgroups,
                                                          int stage_l, int stage_r) {
   extern __shared__ float stage_all[];  // D_L, then one D_R per warp
+  pdl_begin();
   __shared__ float mr[kCorrPartners];
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
   long long bid = blockIdx.x;
@@ -1326,7 +1352,7 @@ __global__ void __launch_bounds__(256) correction_kernel(float* __restrict__ out
   {  // D_L, all threads
     const float* l0 = SL + (l * (Hl + 1) + y0) * (long long)(Wl + 1);
     const float* l1 = SL + (l * (Hl + 1) + y1) * (long long)(Wl + 1);
-    for (int t = threadIdx.x; t < Wl + 1; t += blockDim.x) stage_all[t] = __ldg(l1 + t) - __ldg(l0 + t);
+    for (int t = threadIdx.x; t < Wl + 1; t += blockDim.x) stage_all[t] = ld_after(l1 + t) - ld_after(l0 + t);
   }
   if (wid < n_here) {  // warp-uniform: D_R of partner k0 + wid
     const long long r = l * pm.r_l + (long long)(k0 + wid) * pm.r_k;
@@ -1338,8 +1364,8 @@ __global__ void __launch_bounds__(256) correction_kernel(float* __restrict__ out
 #pragma unroll
       for (int u = 0; u < 8; ++u) {
         const int t = t0 + 32 * u + lane;
-        a[u] = t < Wr + 1 ? __ldg(r1 + t) : 0.0f;
-        b[u] = t < Wr + 1 ? __ldg(r0 + t) : 0.0f;
+        a[u] = t < Wr + 1 ? ld_after(r1 + t) : 0.0f;
+        b[u] = t < Wr + 1 ? ld_after(r0 + t) : 0.0f;
       }
 #pragma unroll
       for (int u = 0; u < 8; ++u) {
@@ -1375,6 +1401,26 @@ __global__ void __launch_bounds__(256) correction_kernel(float* __restrict__ out
       o += ostep;
     }
   }
+}
+
+// Launches a kernel of the chain so that its CTAs may become resident while
+// the previous kernel's last ones run (programmatic dependent launch); every
+// kernel here waits for the whole previous one (pdl_wait) before it reads or
+// writes memory that others touch.
+template <typename... P, typename... A>
+xc_status launch_after(void (*kern)(P...), unsigned blocks, int threads, size_t smem, cudaStream_t stream, A... args) {
+  cudaLaunchAttribute attr{};
+  attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr.val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3(blocks);
+  cfg.blockDim = dim3((unsigned)threads);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = stream;
+  cfg.attrs = &attr;
+  cfg.numAttrs = 1;
+  XC_CUDA_TRY(cudaLaunchKernelEx(&cfg, kern, static_cast<P>(args)...));
+  return XC_OK;
 }
 
 struct TcPlan {
@@ -1728,8 +1774,7 @@ xc_status tc_correlate_banded(const float* left, const float* right, float* out,
     const PrepSide sr{right, g.Hr, g.Wr, ra, rs, w.sums + nl, w.sq + nl, w.mu + nl, w.CR, (long long)nr * (g.Hr + 1),
                       w.hi, w.lo, t.pitch, tf32 ? 1 : 0};
     XC_CUDA_TRY(cudaMemsetAsync(w.sums, 0, 2 * sizeof(double) * (nl + nr), stream));
-    sum_kernel<<<(unsigned)(nl * ls + nr * rs), 256, 0, stream>>>(sl, sr, (unsigned)(nl * ls));
-    XC_CUDA_TRY(cudaGetLastError());
+    XC_TRY(launch_after(sum_kernel, (unsigned)(nl * ls + nr * rs), 256, 0, stream, sl, sr, (unsigned)(nl * ls)));
     const int npg = div_up(pm.K, t.P);
     const WinArgs wa{w.sums, w.sq, nl, (double)la, (double)ra, pm, npg, t.P, flush_rows(t.nkc), t.chunk_rows,
                      flush_fixed(), w.flush};
@@ -1739,18 +1784,18 @@ xc_status tc_correlate_banded(const float* left, const float* right, float* out,
     const long long chunks = (long long)g.Hr * (t.pitch / (16 / t.es));
     const int bpm = (int)std::max(1LL, std::min(64LL, chunks / 2048));
     const unsigned split_end = lrc + (unsigned)(nr * bpm);
-    const unsigned wb = (unsigned)((32LL * nl * npg + 255) / 256);
+    const bool tall = std::max(g.Hl, g.Hr) > 256;
+    const int col_threads = tall ? 1024 : 256;
+    const unsigned wb = (unsigned)((32LL * nl * npg + col_threads - 1) / col_threads);
     if ((long long)split_end + wb + 1 > 0x7fffffffLL)
       return fail(XC_ERR_INVALID_ARGUMENT, "problem too large for one launch");
     const int list = band_done == nullptr ? 1 : 0;
     const size_t list_smem = list ? sizeof(int) * (size_t)prm.n_bands * (t.chunk_rows + 1) : 0;
-    colsum_kernel<<<split_end + wb + (unsigned)list, 256, list_smem, stream>>>(
-        sl, sr, lc, lrc, split_end, bpm, wa, prm, list, (int)n_list, w.items, w.items + t.n_items);
-    XC_CUDA_TRY(cudaGetLastError());
+    XC_TRY(launch_after(tall ? colsum_kernel<32> : colsum_kernel<8>, split_end + wb + (unsigned)list, col_threads, list_smem, stream, sl, sr, lc, lrc,
+                        split_end, bpm, wa, prm, list, (int)n_list, w.items, w.items + t.n_items));
     // second pass: every row of the left and of the right tables
     const unsigned lb = (unsigned)((sl.sat_rows + 7) / 8);
-    rowscan_kernel<<<(unsigned)(lb + (sr.sat_rows + 7) / 8), 256, 0, stream>>>(sl, sr, lb);
-    XC_CUDA_TRY(cudaGetLastError());
+    XC_TRY(launch_after(rowscan_kernel, (unsigned)(lb + (sr.sat_rows + 7) / 8), 256, 0, stream, sl, sr, lb));
   }
   // 4. the mean terms initialise the output
   {
@@ -1761,11 +1806,10 @@ xc_status tc_correlate_banded(const float* left, const float* right, float* out,
     const int n_kgroups = div_up(pm.K, kCorrPartners);
     const long long n_blocks = (long long)nl * n_kgroups * g.Sy;
     if (n_blocks > 0x7fffffffLL) return fail(XC_ERR_INVALID_ARGUMENT, "problem too large for one launch");
-    correction_kernel<<<(unsigned)n_blocks, 256, corr_smem, stream>>>(out, w.CL, w.CR, w.mu, w.mu + nl, g.Hl, g.Wl,
-                                                                      g.Hr, g.Wr, g.Sy, g.Sx, pm, n_kgroups, stage_l,
-                                                                      stage_r);
+    XC_TRY(launch_after(correction_kernel, (unsigned)n_blocks, 256, corr_smem, stream, out, (const float*)w.CL,
+                        (const float*)w.CR, (const float*)w.mu, (const float*)(w.mu + nl), g.Hl, g.Wl, g.Hr, g.Wr,
+                        g.Sy, g.Sx, pm, n_kgroups, stage_l, stage_r));
   }
-  XC_CUDA_TRY(cudaGetLastError());
 
   // persistent: one CTA per SM (about 205 KB of shared memory and all 512 TMEM
   // columns each), walking the list in snake order
@@ -1783,9 +1827,9 @@ xc_status tc_correlate_banded(const float* left, const float* right, float* out,
       for (int k = 0; k < prm.n_bands; ++k) bands->items[k] = band_items[k];
   }
   const int slot = kernel_timer_begin(stream);
-  kern<<<(unsigned)blocks, kThreads, (size_t)t.smem_bytes, stream>>>(mhi, mlo, prm);
+  const xc_status st = launch_after(kern, (unsigned)blocks, kThreads, (size_t)t.smem_bytes, stream, mhi, mlo, prm);
   kernel_timer_end(slot, stream);
-  XC_CUDA_TRY(cudaGetLastError());
+  XC_TRY(st);
   if (band_done) {
     band_release_kernel<<<1, 32, 0, stream>>>(band_done, prm.n_bands);
     XC_CUDA_TRY(cudaGetLastError());
