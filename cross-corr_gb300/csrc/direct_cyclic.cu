@@ -191,6 +191,24 @@ __device__ __forceinline__ void stage_rows(char* dst, int pitch, const T* __rest
   }
 }
 
+// One output's sum over a block's right rows by the definition: left row y +
+// dy, column x + dx.  For outputs whose sum came out as NaN: the zero columns
+// and rows around the matrices make NaN of an infinity, and of a NaN, that the
+// shift does not meet.  A sum that is NaN stays one, so the loop ends there.
+template <typename T>
+__device__ __forceinline__ T overlap_sum(const T* __restrict__ L, const T* __restrict__ R, int Hl, int Wl, int rows,
+                                         int Wr, int dy, int dx) {
+  T s = T(0);
+  const int y1 = min(rows, Hl - dy), xa = max(0, -dx), x1 = min(Wr, Wl - dx);
+  for (int y = max(0, -dy); y < y1; ++y) {
+    const T* l = L + (long long)(y + dy) * Wl + dx;
+    const T* r = R + (long long)y * Wr;
+    for (int x = xa; x < x1; ++x) s = fma(__ldg(l + x), __ldg(r + x), s);
+    if (s != s) break;
+  }
+  return s;
+}
+
 template <typename T, int TSY, bool WIN>
 __global__ void __launch_bounds__(256, 2) cyclic_kernel(const CycArgs<T> p) {
   using Tl = Tile<T, TSY>;
@@ -275,13 +293,19 @@ __global__ void __launch_bounds__(256, 2) cyclic_kernel(const CycArgs<T> p) {
   const int sy = u * TSY - (b0 + p.hb - 1) + p.Hr - 1;  // of t = 0
   const int sx = c * TSX + p.Wr - 1;                    // of q = 0, m = 0
   const int P = p.C * TSX;
+  // a sum that is NaN is made again from what its shift meets (`redo`)
   const auto emit = [&](T* dst, T v) {
     if (p.accumulate) atomicAdd(dst, v);  // result unused: red.global.add
     else *dst = v;
   };
+  const auto redo = [&](int oy, int ox) {
+    emit(out + (long long)oy * p.Sx + ox,
+         overlap_sum(L, R, p.Hl, p.Wl, hbj, p.Wr, oy - (p.Hr - 1) + b0, ox - (p.Wr - 1)));
+  };
   // the warp's buffer, as the sums of segment mm of every lane in `mask`
   const auto flush = [&](int mm, unsigned mask) {
     __syncwarp();
+    unsigned bad = 0;  // NaN sums, by j TSY + t
 #pragma unroll
     for (int j = 0; j < TSX; ++j) {
       const int from = j * (32 / TSX) + lane / TSX;
@@ -290,7 +314,19 @@ __global__ void __launch_bounds__(256, 2) cyclic_kernel(const CycArgs<T> p) {
       if (!((mask >> from) & 1u) || fx < 0 || fx >= p.Sx) continue;
 #pragma unroll
       for (int t = 0; t < TSY; ++t)
-        if (fy + t >= 0 && fy + t < p.Sy) emit(out + (long long)(fy + t) * p.Sx + fx, buf[t * (32 * TSX) + j * 32 + lane]);
+        if (fy + t >= 0 && fy + t < p.Sy) {
+          const T v = buf[t * (32 * TSX) + j * 32 + lane];
+          if (v == v) emit(out + (long long)(fy + t) * p.Sx + fx, v);
+          else bad |= 1u << (j * TSY + t);
+        }
+    }
+    while (__any_sync(0xffffffffu, bad != 0)) {
+      const int i = bad ? __ffs((int)bad) - 1 : 0, j = i / TSY;
+      const int from = j * (32 / TSX) + lane / TSX;
+      const int fy = __shfl_sync(0xffffffffu, sy, from) + i % TSY;
+      const int fx = __shfl_sync(0xffffffffu, sx, from) - mm * P + lane % TSX;
+      if (bad) redo(fy, fx);
+      bad &= bad - 1;
     }
     __syncwarp();
   };
@@ -318,13 +354,22 @@ __global__ void __launch_bounds__(256, 2) cyclic_kernel(const CycArgs<T> p) {
 #pragma unroll
         for (int t = 0; t < TSY; ++t) a.put(buf + t * (32 * TSX) + lane * TSX, t);
       } else if (live) {
+        unsigned bad = 0;
 #pragma unroll
         for (int t = 0; t < TSY; ++t)
 #pragma unroll
           for (int q = 0; q < TSX; ++q) {
             const int x = sx - m * P + q;
-            if (sy + t >= 0 && sy + t < p.Sy && x >= 0 && x < p.Sx) emit(out + (long long)(sy + t) * p.Sx + x, a.get(t, q));
+            if (sy + t >= 0 && sy + t < p.Sy && x >= 0 && x < p.Sx) {
+              const T v = a.get(t, q);
+              if (v == v) emit(out + (long long)(sy + t) * p.Sx + x, v);
+              else bad |= 1u << (t * TSX + q);
+            }
           }
+        for (; bad; bad &= bad - 1) {
+          const int i = __ffs((int)bad) - 1;
+          redo(sy + i / TSX, sx - m * P + i % TSX);
+        }
       }
       a.zero();
     }

@@ -57,3 +57,27 @@ def test_rows_too_wide_keep_the_tiled_kernel():
     out = xcorr.correlate("one_to_one", torch.from_numpy(left).cuda(), torch.from_numpy(right).cuda())
     torch.cuda.synchronize()
     assert rel_to_max(out.cpu().numpy(), ref) <= TOL["f32"]
+
+
+@pytest.mark.parametrize("dtype", ["f32", "f64"])
+@pytest.mark.parametrize("ls,rs", [((32, 32), (32, 32)), ((17, 33), (9, 21)), ((5, 3), (7, 50)), ((64, 300), (64, 40)),
+                                   ((6, 1030), (35, 16))])
+@pytest.mark.parametrize("value", [float("inf"), float("nan")])
+def test_non_finite_values_stay_where_they_are_met(value, ls, rs, dtype):
+    """One non-finite value reaches the shifts that multiply it and no others
+    (the kernel's zero columns and rows would make NaN of it elsewhere): the
+    others equal, within the method's bound, the result with a zero there."""
+    npdt = np.float32 if dtype == "f32" else np.float64
+    for side, at in [(s, (int(fy * (h - 1)), int(fx * (w - 1)))) for s, (h, w) in ((0, ls), (1, rs))
+                     for fy, fx in ((0, 0), (1, 1), (1, 0), (0.5, 0.5))]:
+        pair = [seeded((1,) + ls, 37, "uniform", npdt) + npdt(0.5), seeded((1,) + rs, 38, "uniform", npdt) + npdt(0.5)]
+        pair[side][0][at] = 0
+        ref = oracle.run_mode("one_to_one", *pair, dtype="f32acc64" if dtype == "f32" else "f64", threads=4)[0]
+        mark = [np.zeros_like(pair[0]), np.ones_like(pair[1])] if side == 0 else [np.ones_like(pair[0]), np.zeros_like(pair[1])]
+        mark[side][0][at] = 1
+        met = oracle.run_mode("one_to_one", *mark, dtype="f32acc64" if dtype == "f32" else "f64", threads=4)[0] > 0.5
+        pair[side][0][at] = value
+        out = xcorr.correlate("one_to_one", *[torch.from_numpy(x).cuda() for x in pair])[0].cpu().numpy()
+        assert np.array_equal(~np.isfinite(out), met)
+        assert np.array_equal(np.isnan(out), met if np.isnan(value) else np.zeros_like(met))
+        assert rel_to_max(np.where(met, 0, out), np.where(met, 0, ref)) <= TOL[dtype]
