@@ -250,10 +250,15 @@ xc_status engine_plan(Engine* e, xc_dtype dtype, const Geometry& g, const PairMa
   if (!(f32 ? row_kernels_f32(e->nx, &e->rk) : row_kernels_f64(e->nx, &e->rk)) ||
       !(f32 ? col_kernels_f32(e->ny, &e->ck) : col_kernels_f64(e->ny, &e->ck)))
     return XC_OK;
+  if (e->ck.rq == 4) {
+    e->rk.forward = e->rk.forward_rq4;
+    e->rk.inverse = e->rk.inverse_rq4;
+  }
   const size_t ce = f32 ? sizeof(float2) : sizeof(double2);
   const int cb = 1 << e->ck.lgcb;
   e->nblk = div_up(e->nx / 2 + 1, cb);
   const size_t row = (size_t)e->nblk * cb * ce;  // bytes of one spectrum row
+  const auto rows = [&](int H) { return row * spectrum_rows(H, e->ck.rq); };
   e->shared = pm.r_l == 0 && pm.n_left > 1;
   // The left spectra are made first (col_forward) when several partners use
   // them: transforming the left's columns in every CTA of the column kernel
@@ -268,7 +273,7 @@ xc_status engine_plan(Engine* e, xc_dtype dtype, const Geometry& g, const PairMa
   // whose spectra stay in the L2 cache, measured slower: the launches' ramps
   // cost more than the traffic; 2048x2048 x 16: 1.78 ms in one chunk, 2.06 in
   // sixteen; 256x256 x 64: 86 us in one, 112 in two).
-  const size_t ar1 = row * g.Hr, b1 = row * g.Sy;
+  const size_t ar1 = rows(g.Hr), b1 = rows(g.Sy);
   size_t off = 0;
   const auto take = [&](size_t bytes) {
     const size_t at = off;
@@ -279,7 +284,7 @@ xc_status engine_plan(Engine* e, xc_dtype dtype, const Geometry& g, const PairMa
   if (e->shared) {
     e->off_fr = take(row * e->ny * n_right);
     const size_t at = off;
-    e->off_al = take(row * g.Hl * pm.n_left);
+    e->off_al = take(rows(g.Hl) * pm.n_left);
     e->off_ar = take(ar1 * n_right);
     const size_t a_end = off;
     e->off_b = at;  // products replace the row spectra, which are done with by then
@@ -294,7 +299,7 @@ xc_status engine_plan(Engine* e, xc_dtype dtype, const Geometry& g, const PairMa
     off = std::max(a_end, at + align256(b1 * e->l_chunk * e->k_chunk));
     e->kc = 1;
   } else {
-    e->off_al = take(row * g.Hl * pm.n_left);
+    e->off_al = take(rows(g.Hl) * pm.n_left);
     e->l_chunk = pm.n_left;
     const size_t per_k = (ar1 + b1) * pm.n_left;  // r_k = n_left rights (one for a single left)
     if (off + per_k + 512 > ws_bytes) return XC_OK;

@@ -476,11 +476,25 @@ __device__ __forceinline__ void mid_passes(Cp<S>* z, int it0, int step, const Cp
 
 // ---------------------------------------------------------------------------
 // Layout of the half spectra between the kernels: matrix by matrix, blocks of
-// CB = 2^lgcb columns, [block][row][column in block] of complex values,
-// columns 0..N/2 rounded up to whole blocks (the columns beyond N/2 are never
-// written by the row kernels nor read by them).  A row pair's share of a
-// block is contiguous (row kernels), and so is a whole block (column kernels).
+// CB = 2^lgcb columns, [block][row / RQ][column in block][row % RQ] of complex
+// values, rows rounded up to whole groups of RQ and columns 0..N/2 to whole
+// blocks (the columns beyond N/2 are never written by the row kernels nor read
+// by them).  A whole block is contiguous (column kernels).  RQ is 4 for FP32
+// blocks of two columns (lengths over 2048): a thread of the row kernels moves
+// its four rows of a column as 32 contiguous bytes instead of four times 8,
+// each of those instructions in 16 lines (2048x2048 x 16: 1.64 ms, 1.80 with
+// RQ = 1).  Blocks of four columns keep RQ = 1: their lines are half as many,
+// and the column kernels' two 8-byte accesses in the place of one of 16 cost
+// more than the row kernels gain (511x511 x 64: row kernels 43 us against 49,
+// column kernel 39 against 31); so do ragged batches, whose row launches mix
+// both kinds of blocks.
 // ---------------------------------------------------------------------------
+__host__ __device__ constexpr int spectrum_rows(int H, int rq) { return (H + rq - 1) / rq * rq; }
+// element offset of row y in a block of CB columns (columns RQ apart)
+template <int CB, int RQ>
+__device__ __forceinline__ int row_at(int y) {
+  return y / RQ * (RQ * CB) + y % RQ;
+}
 template <typename T>
 struct Cx {
   T x, y;
@@ -553,7 +567,7 @@ struct ColFwdArgs {
 };
 template <typename T>
 struct RowInvArgs {
-  const Cx<T>* src;   // [output of this launch][block][Sy][CB]
+  const Cx<T>* src;   // [output of this launch][block], Sy rows
   T* out;
   int Sy, Sx, Wr;
   int groups;         // CTAs per output
@@ -620,6 +634,23 @@ __device__ __forceinline__ double2 ld(const double2* g) {
   asm volatile("ld.global.v2.f64 {%0, %1}, [%2];" : "=d"(v.x), "=d"(v.y) : "l"(g));
   return v;
 }
+// 32 bytes: a column's RQ = 4 rows
+struct alignas(32) Col4 {
+  float2 r[4];
+};
+__device__ __forceinline__ Col4 ld(const Col4* g) {
+  Col4 v;
+  asm volatile("ld.global.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+               : "=f"(v.r[0].x), "=f"(v.r[0].y), "=f"(v.r[1].x), "=f"(v.r[1].y), "=f"(v.r[2].x), "=f"(v.r[2].y),
+                 "=f"(v.r[3].x), "=f"(v.r[3].y)
+               : "l"(g));
+  return v;
+}
+__device__ __forceinline__ void st(Col4* g, float2 r0, float2 r1, float2 r2, float2 r3) {
+  asm volatile("st.global.v8.f32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(g), "f"(r0.x), "f"(r0.y), "f"(r1.x),
+               "f"(r1.y), "f"(r2.x), "f"(r2.y), "f"(r3.x), "f"(r3.y)
+               : "memory");
+}
 __device__ __forceinline__ Cp<f2> ld(const Cp<f2>* g) {
   Cp<f2> v;
   asm volatile("ld.global.v2.b64 {%0, %1}, [%2];" : "=l"(v.x.v), "=l"(v.y.v) : "l"(g));
@@ -633,7 +664,7 @@ __device__ __forceinline__ Cp<double> ld(const Cp<double>* g) {
 __device__ __forceinline__ Cp<f2> gather(const float* v) { return {pack(v[0], v[2]), pack(v[1], v[3])}; }
 __device__ __forceinline__ Cp<double> gather(const double* v) { return {v[0], v[1]}; }
 
-template <typename S, int N, bool RAG>
+template <typename S, int N, bool RAG, int RQ>
 __global__ void __launch_bounds__(RowCfg<N>::threads, RowCfg<N>::min_ctas) row_forward(const RowFwdArgs<typename Sc<S>::real> p) {
   using L = RowPasses<N>;
   using C = Cp<S>;
@@ -665,7 +696,7 @@ __global__ void __launch_bounds__(RowCfg<N>::threads, RowCfg<N>::min_ctas) row_f
     W = first ? p.a.W : p.b.W;
     lgcb = p.lgcb;
     src = (first ? p.a.src : p.b.src) + (long long)mat * H * W;
-    dst = (first ? p.a.dst : p.b.dst) + (((long long)mat * p.nblk * H) << lgcb);
+    dst = (first ? p.a.dst : p.b.dst) + (((long long)mat * p.nblk * spectrum_rows(H, RQ)) << lgcb);
     scale = first ? p.a.scale : p.b.scale;
     group = (int)(b - mat * groups);
   }
@@ -716,13 +747,16 @@ __global__ void __launch_bounds__(RowCfg<N>::threads, RowCfg<N>::min_ctas) row_f
   S hs;
   if constexpr (NV == 2) hs = pack(0.5f * scale, 0.5f * scale);
   else hs = T(0.5) * scale;
-  const int cb = 1 << lgcb;
+  const int cb = 1 << lgcb, HP = spectrum_rows(H, RQ);
   dst += (long long)row0 * cb;
   const auto put = [&](int k, C zk, C zn) {
     const C a = {mul(hs, add(zk.x, zn.x)), mul(hs, sub(zk.y, zn.y))};
     const C bb = {mul(hs, add(zk.y, zn.y)), mul(hs, sub(zn.x, zk.x))};
-    Cx<T>* d = dst + (long long)(k >> lgcb) * H * cb + (k & (cb - 1));
-    if constexpr (NV == 2) {
+    Cx<T>* d = dst + (long long)(k >> lgcb) * HP * cb + (k & (cb - 1)) * RQ;
+    if constexpr (RQ == 4) {
+      st(reinterpret_cast<Col4*>(d), make_float2(lo(a.x), lo(a.y)), make_float2(lo(bb.x), lo(bb.y)),
+         make_float2(hi(a.x), hi(a.y)), make_float2(hi(bb.x), hi(bb.y)));
+    } else if constexpr (NV == 2) {
       *reinterpret_cast<float2*>(d) = make_float2(lo(a.x), lo(a.y));
       if (row0 + 1 < H) *reinterpret_cast<float2*>(d + cb) = make_float2(lo(bb.x), lo(bb.y));
       if (row0 + 2 < H) *reinterpret_cast<float2*>(d + 2 * cb) = make_float2(hi(a.x), hi(a.y));
@@ -744,7 +778,7 @@ __global__ void __launch_bounds__(RowCfg<N>::threads, RowCfg<N>::min_ctas) row_f
   }
 }
 
-template <typename S, int N, bool RAG>
+template <typename S, int N, bool RAG, int RQ>
 __global__ void __launch_bounds__(RowCfg<N>::threads, RowCfg<N>::min_ctas) row_inverse(const RowInvArgs<typename Sc<S>::real> p) {
   using L = RowPasses<N>;
   using C = Cp<S>;
@@ -776,7 +810,7 @@ __global__ void __launch_bounds__(RowCfg<N>::threads, RowCfg<N>::min_ctas) row_i
     Sx = p.Sx;
     Wr = p.Wr;
     lgcb = p.lgcb;
-    src = p.src + (((long long)t * p.nblk * Sy) << lgcb);
+    src = p.src + (((long long)t * p.nblk * spectrum_rows(Sy, RQ)) << lgcb);
     out = p.out + (l * p.o_l + k * p.o_k) * Sy * (long long)Sx;
     scale_hi = p.scale_hi;
     scale_lo = p.scale_lo;
@@ -786,12 +820,17 @@ __global__ void __launch_bounds__(RowCfg<N>::threads, RowCfg<N>::min_ctas) row_i
   const int row0 = (group * Q + f) * (2 * NV);
   C* z = reinterpret_cast<C*>(smem_raw) + f * RowCfg<N>::FS;
   const int cb = 1 << lgcb;
+  const int SP = spectrum_rows(Sy, RQ);
   src += (long long)row0 * cb;
   const bool v0 = row0 < Sy, v1 = row0 + 1 < Sy, v2 = row0 + 2 < Sy, v3 = row0 + 3 < Sy;
   // rows A and B of each row pair at column c
   const auto get = [&](int c, C* a, C* b) {
-    const Cx<T>* d = src + (long long)(c >> lgcb) * Sy * cb + (c & (cb - 1));
-    if constexpr (NV == 2) {
+    const Cx<T>* d = src + (long long)(c >> lgcb) * SP * cb + (c & (cb - 1)) * RQ;
+    if constexpr (RQ == 4) {  // rows beyond the last are the circular result's next ones
+      const Col4 e = v0 ? ld(reinterpret_cast<const Col4*>(d)) : Col4{};
+      *a = {pack(e.r[0].x, e.r[2].x), pack(e.r[0].y, e.r[2].y)};
+      *b = {pack(e.r[1].x, e.r[3].x), pack(e.r[1].y, e.r[3].y)};
+    } else if constexpr (NV == 2) {
       const float2 o = make_float2(0.f, 0.f);
       const float2 e0 = v0 ? ld(reinterpret_cast<const float2*>(d)) : o;
       const float2 e1 = v1 ? ld(reinterpret_cast<const float2*>(d + cb)) : o;
@@ -894,6 +933,7 @@ struct ColCfg {
   using L = ColPasses<N>;
   static constexpr int CB = Sc<S>::NV == 2 ? (N <= 2048 ? 4 : 2) : 2;
   static constexpr int lgcb = CB == 4 ? 2 : 1;
+  static constexpr int RQ = Sc<S>::NV == 2 && CB == 2 ? 4 : 1;  // rows side by side (but ragged batches: 1)
   static constexpr int LC = CB / Sc<S>::NV;  // lanes across a block's columns
   // Items a pass runs side by side: the count that issues the fewest lane
   // slots over the passes (a pass of n items takes ceil(n / JT) rounds of JT
@@ -917,25 +957,38 @@ struct ColCfg {
   static constexpr int unit = L::rows * LC;        // shared-memory elements of a unit
 };
 
-// A thread's columns of one row of a block.
+// A thread's columns of one row of a block, RQ elements apart.
+template <int RQ>
 __device__ __forceinline__ Cp<f2> load_row(const Cx<float>* g) {
-  const float4 v = ld(reinterpret_cast<const float4*>(g));
-  return {pack(v.x, v.z), pack(v.y, v.w)};
+  if constexpr (RQ == 1) {
+    const float4 v = ld(reinterpret_cast<const float4*>(g));
+    return {pack(v.x, v.z), pack(v.y, v.w)};
+  }
+  const float2 u = ld(reinterpret_cast<const float2*>(g)), v = ld(reinterpret_cast<const float2*>(g + RQ));
+  return {pack(u.x, v.x), pack(u.y, v.y)};
 }
+template <int RQ>
 __device__ __forceinline__ Cp<double> load_row(const Cx<double>* g) {
   const double2 v = ld(reinterpret_cast<const double2*>(g));
   return {v.x, v.y};
 }
+template <int RQ>
 __device__ __forceinline__ void store_row(Cx<float>* g, Cp<f2> v) {
-  *reinterpret_cast<float4*>(g) = make_float4(lo(v.x), lo(v.y), hi(v.x), hi(v.y));
+  if constexpr (RQ == 1) {
+    *reinterpret_cast<float4*>(g) = make_float4(lo(v.x), lo(v.y), hi(v.x), hi(v.y));
+    return;
+  }
+  *reinterpret_cast<float2*>(g) = make_float2(lo(v.x), lo(v.y));
+  *reinterpret_cast<float2*>(g + RQ) = make_float2(hi(v.x), hi(v.y));
 }
+template <int RQ>
 __device__ __forceinline__ void store_row(Cx<double>* g, Cp<double> v) {
   *reinterpret_cast<double2*>(g) = make_double2(v.x, v.y);
 }
 
 // Forward passes of one column block from global memory (H rows; g points at
 // the thread's columns) up to, not including, the last; ends with a barrier.
-template <typename S, int N>
+template <typename S, int N, int RQ>
 __device__ __forceinline__ void col_load_passes(Cp<S>* z, const Cx<typename Sc<S>::real>* __restrict__ g, int H,
                                                 int j0, const Cp<S>* __restrict__ tw) {
   using L = ColPasses<N>;
@@ -945,7 +998,9 @@ __device__ __forceinline__ void col_load_passes(Cp<S>* z, const Cx<typename Sc<S
 #pragma unroll
     for (int m = 0; m < L::R1; ++m) {
       const int y = o + m * L::S1;
-      x[m] = y < H ? load_row(g + (long long)y * K::CB) : czero<S>();
+      x[m] = y < H ? load_row<RQ>(g + (L::S1 % RQ == 0 ? row_at<K::CB, RQ>(o) + m * L::S1 * K::CB
+                                                             : row_at<K::CB, RQ>(y)))
+                   : czero<S>();
     }
     Dft<S, -1, L::R1>::run(x);
     Cp<S>* base = z + L::in_block(o) * K::LC;
@@ -983,7 +1038,7 @@ __global__ void __launch_bounds__(ColCfg<S, N>::threads, ColCfg<S, N>::min_ctas)
   const long long u = (long long)blockIdx.x * K::PU + pu;
   const bool live = u < p.units;
   pdl_wait();
-  col_load_passes<S, N>(z, p.src + (live ? u : 0) * p.H * K::CB + c * Sc<S>::NV, live ? p.H : 0, j0, tw);
+  col_load_passes<S, N, K::RQ>(z, p.src + (live ? u : 0) * spectrum_rows(p.H, K::RQ) * K::CB + c * (Sc<S>::NV * K::RQ), live ? p.H : 0, j0, tw);
   if (!live) return;
   C* dst = static_cast<C*>(p.dst) + u * N * K::LC + c;
   for (int j = j0; j < L::TF; j += K::JT) {
@@ -1008,7 +1063,7 @@ __global__ void __launch_bounds__(ColCfg<S, N>::threads, ColCfg<S, N>::min_ctas)
   using C = Cp<S>;
   using K = ColCfg<S, N>;
   using G = Cx<typename Sc<S>::real>;
-  constexpr int NV = Sc<S>::NV;
+  constexpr int NV = Sc<S>::NV, RQ = RAG ? 1 : K::RQ;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   pdl_launch();
   const C* __restrict__ tw = static_cast<const C*>(p.tw);
@@ -1039,11 +1094,14 @@ __global__ void __launch_bounds__(ColCfg<S, N>::threads, ColCfg<S, N>::min_ctas)
     out = it.out;
   } else {
     nblk = p.nblk;
-    blk = gu % (unsigned)nblk;
-    const unsigned rest = gu / (unsigned)nblk;
-    const int kg = (int)(rest % (unsigned)p.n_kg);
-    ll = (int)(rest / (unsigned)p.n_kg);  // left of this launch
-    live = ll < p.n_left;
+    // partners first, then lefts: the CTAs that read one block's spectra run
+    // side by side and find them in the L2 cache
+    const int kg = (int)(gu % (unsigned)p.n_kg);
+    const unsigned rest = gu / (unsigned)p.n_kg;
+    ll = (int)(rest % (unsigned)p.n_left);  // left of this launch
+    blk = rest / (unsigned)p.n_left;
+    live = blk < (unsigned)nblk;
+    if (!live) blk = 0;
     l = p.l0 + (live ? ll : 0);
     kc = p.kc;
     ka = p.k0 + kg * kc;
@@ -1060,7 +1118,8 @@ __global__ void __launch_bounds__(ColCfg<S, N>::threads, ColCfg<S, N>::min_ctas)
   if constexpr (LPRE) {
     lspec = static_cast<const C*>(p.left) + (l * nblk + blk) * (long long)N * K::LC + c;
   } else {
-    col_load_passes<S, N>(zl, gl + (l * nblk + blk) * (long long)Hl * K::CB + c * NV, live ? Hl : 0, j0, tw);
+    col_load_passes<S, N, RQ>(zl, gl + (l * nblk + blk) * (long long)spectrum_rows(Hl, RQ) * K::CB + c * (NV * RQ),
+                          live ? Hl : 0, j0, tw);
     // each thread reads back the items it writes here: no barrier needed
     for (int j = j0; j < L::TF; j += K::JT) {
       C x[L::R3];
@@ -1078,7 +1137,8 @@ __global__ void __launch_bounds__(ColCfg<S, N>::threads, ColCfg<S, N>::min_ctas)
     const bool act = kk < nk;
     const long long r = !RAG && act ? l * p.r_l + k * p.r_k - p.r_off : 0;
     if constexpr (!RPRE)
-      col_load_passes<S, N>(z, gr + (r * nblk + blk) * (long long)Hr * K::CB + c * NV, act ? Hr : 0, j0, tw);
+      col_load_passes<S, N, RQ>(z, gr + (r * nblk + blk) * (long long)spectrum_rows(Hr, RQ) * K::CB + c * (NV * RQ),
+                            act ? Hr : 0, j0, tw);
     for (int j = j0; j < L::TF; j += K::JT) {
       C x[L::R3];
       C* base = z + col_item<S, N>(j);
@@ -1101,7 +1161,8 @@ __global__ void __launch_bounds__(ColCfg<S, N>::threads, ColCfg<S, N>::min_ctas)
     __syncthreads();
     mid_passes<S, 1, true, L, K::LC>(z, j0, K::JT, tw);
     if (act) {
-      G* o = out + ((ll * n_k + (RAG ? 0 : k - p.k0)) * nblk + blk) * (long long)Sy * K::CB + c * NV;
+      const int SP = spectrum_rows(Sy, RQ);  // at most N: a multiple of 16
+      G* o = out + ((ll * n_k + (RAG ? 0 : k - p.k0)) * nblk + blk) * (long long)SP * K::CB + c * (NV * RQ);
       for (int i = j0; i < L::S1; i += K::JT) {
         C x[L::R1];
         const C* base = z + L::in_block(i) * K::LC;
@@ -1113,7 +1174,7 @@ __global__ void __launch_bounds__(ColCfg<S, N>::threads, ColCfg<S, N>::min_ctas)
         for (int m = 0; m < L::R1; ++m) {
           int sy = i + m * L::S1 + Hr - 1;
           if (sy >= N) sy -= N;
-          if (sy < Sy) store_row(o + (long long)sy * K::CB, x[m]);
+          if (sy < SP) store_row<RQ>(o + row_at<K::CB, RQ>(sy), x[m]);
         }
       }
     }
@@ -1125,6 +1186,8 @@ __global__ void __launch_bounds__(ColCfg<S, N>::threads, ColCfg<S, N>::min_ctas)
 struct RowKernels {
   const void* forward;
   const void* inverse;
+  const void* forward_rq4;  // for column kernels with rq = 4 (FP32 only)
+  const void* inverse_rq4;
   const void* rag_forward;  // over a ragged batch's records (FP32 only)
   const void* rag_inverse;
   int threads, q, nv, smem;
@@ -1135,7 +1198,7 @@ struct ColKernels {
   const void* pairs_lpre;  // left spectra from col_forward
   const void* pairs_pre;   // both
   const void* rag_pairs;   // `pairs` over a ragged batch's records (FP32 only)
-  int threads, pu, lgcb, unit_smem;  // shared memory of one buffer
+  int threads, pu, lgcb, rq, unit_smem;  // shared memory of one buffer
 };
 // false: no kernels for this length
 bool row_kernels_f32(int n, RowKernels* k);
@@ -1148,11 +1211,13 @@ bool col_kernels_f64_long(int n, ColKernels* k);
 template <typename S, int N>
 RowKernels row_kernels_of() {
   RowKernels k{};
-  k.forward = (const void*)&row_forward<S, N, false>;
-  k.inverse = (const void*)&row_inverse<S, N, false>;
+  k.forward = (const void*)&row_forward<S, N, false, 1>;
+  k.inverse = (const void*)&row_inverse<S, N, false, 1>;
   if constexpr (Sc<S>::NV == 2) {
-    k.rag_forward = (const void*)&row_forward<S, N, true>;
-    k.rag_inverse = (const void*)&row_inverse<S, N, true>;
+    k.forward_rq4 = (const void*)&row_forward<S, N, false, 4>;
+    k.inverse_rq4 = (const void*)&row_inverse<S, N, false, 4>;
+    k.rag_forward = (const void*)&row_forward<S, N, true, 1>;
+    k.rag_inverse = (const void*)&row_inverse<S, N, true, 1>;
   }
   k.threads = RowCfg<N>::threads;
   k.q = RowCfg<N>::Q;
@@ -1172,6 +1237,7 @@ ColKernels col_kernels_of() {
   k.threads = K::threads;
   k.pu = K::PU;
   k.lgcb = K::lgcb;
+  k.rq = K::RQ;
   k.unit_smem = K::PU * K::unit * 16;
   return k;
 }
