@@ -212,10 +212,10 @@ int length_for(int n) {
   return 0;
 }
 
-size_t twiddle_bytes(int n, bool rows) {
+size_t twiddle_bytes(int n, bool rows, xc_dtype dtype) {
   size_t count = 0;
   each_twiddle(*factors(n, rows), [&](long long, long long) { ++count; });
-  return 16 * count;
+  return align256((dtype == XC_F32 ? sizeof(float2) : sizeof(double2)) * count);
 }
 
 void fill_twiddles(int n, bool rows, xc_dtype dtype, void* out) {
@@ -224,10 +224,10 @@ void fill_twiddles(int n, bool rows, xc_dtype dtype, void* out) {
   each_twiddle(*factors(n, rows), [&](long long k, long long m) {
     double re, im;
     root(k, m, &re, &im);
-    if (dtype == XC_F32) {  // one entry serves the two packed transforms
-      of[0] = of[1] = (float)re;
-      of[2] = of[3] = (float)im;
-      of += 4;
+    if (dtype == XC_F32) {
+      of[0] = (float)re;
+      of[1] = (float)im;
+      of += 2;
     } else {
       od[0] = re;
       od[1] = im;
@@ -318,8 +318,8 @@ xc_status engine_plan(Engine* e, xc_dtype dtype, const Geometry& g, const PairMa
   XC_TRY(raise_limit(e->ck.pairs_lpre, e->ck.unit_smem));
   XC_TRY(raise_limit(e->ck.pairs_pre, e->ck.unit_smem));
   if (2 * e->ck.unit_smem <= 227 * 1024) XC_TRY(raise_limit(e->ck.pairs, 2 * e->ck.unit_smem));
-  e->tw_col = twiddle_bytes(e->nx, true);
-  e->zeros = e->tw_col + twiddle_bytes(e->ny, false);
+  e->tw_col = twiddle_bytes(e->nx, true, dtype);
+  e->zeros = e->tw_col + twiddle_bytes(e->ny, false, dtype);
   std::vector<char> host(e->zeros + (size_t)e->nx * (f32 ? 4 : 8), 0);
   fill_twiddles(e->nx, true, dtype, host.data());
   fill_twiddles(e->ny, false, dtype, host.data() + e->tw_col);

@@ -24,8 +24,12 @@
 // in packed pairs (add, mul and fma .f32x2: the same rate per value in half
 // the instructions): two adjacent columns or two row pairs.  With that the
 // instructions fell by a third to two fifths and the kernels wait for their
-// loads and for shared memory (64% of its wavefronts in col_pairs), 16 to 24
-// warps per SM: 64 outputs of 511x511 take 80 us, 113 in the scalar form.
+// loads and for shared memory (50 to 65% of its wavefronts), 16 to 24 warps
+// per SM: 64 outputs of 511x511 take 73 us, 113 in the scalar form.  Of the
+// column kernel's time at 4096 points, the passes themselves are 57%, the left
+// spectra's loads 14%, the stores 12%, the twiddles' loads 10%, the rows' 1%
+// (each left out in turn, before the twiddles were halved and half of the left
+// spectra loaded ahead).
 // FP64 is bound by its pipe (85% busy; 1.0 TFLOP/s measured).
 #pragma once
 
@@ -94,12 +98,14 @@ template <>
 struct Sc<f2> {
   using real = float;
   static constexpr int NV = 2;  // transforms per thread
+  using Tw = float2;  // a twiddle, the same for both transforms
   static __device__ __forceinline__ f2 bc(double c) { return pack((float)c, (float)c); }
 };
 template <>
 struct Sc<double> {
   using real = double;
   static constexpr int NV = 1;
+  using Tw = double2;
   static __device__ __forceinline__ double bc(double c) { return c; }
 };
 
@@ -139,6 +145,14 @@ __device__ __forceinline__ Cp<S> cmul(Cp<S> a, Cp<S> b) {
   const S nby = neg(b.y);
   if (CONJ) return {fma(a.y, b.y, mul(a.x, b.x)), fma(a.x, nby, mul(a.y, b.x))};
   return {fma(a.y, nby, mul(a.x, b.x)), fma(a.x, b.y, mul(a.y, b.x))};
+}
+template <bool CONJ>
+__device__ __forceinline__ Cp<f2> cmul(Cp<f2> a, float2 w) {
+  return cmul<CONJ>(a, Cp<f2>{pack(w.x, w.x), pack(w.y, w.y)});
+}
+template <bool CONJ>
+__device__ __forceinline__ Cp<double> cmul(Cp<double> a, double2 w) {
+  return cmul<CONJ>(a, Cp<double>{w.x, w.y});
 }
 template <typename S>
 __device__ __forceinline__ Cp<S> czero() {
@@ -435,7 +449,7 @@ XC_FFT_COLS(XC_DEF)
 // decimation in frequency (twiddles after), column-inverse ones decimation in
 // time (twiddles before).
 template <typename S, int D, bool DIT, int R, int PS, int STEP>
-__device__ __forceinline__ void butterfly(Cp<S>* base, const Cp<S>* __restrict__ tw, int tw_step) {
+__device__ __forceinline__ void butterfly(Cp<S>* base, const typename Sc<S>::Tw* __restrict__ tw, int tw_step) {
   Cp<S> x[R];
   if (!DIT) {
 #pragma unroll
@@ -454,7 +468,7 @@ __device__ __forceinline__ void butterfly(Cp<S>* base, const Cp<S>* __restrict__
   }
 }
 template <typename S, int D, bool DIT, typename L, int STEP>
-__device__ __forceinline__ void mid_passes(Cp<S>* z, int it0, int step, const Cp<S>* __restrict__ tw) {
+__device__ __forceinline__ void mid_passes(Cp<S>* z, int it0, int step, const typename Sc<S>::Tw* __restrict__ tw) {
   if constexpr (L::Ra > 1) {
     for (int it = it0; it < L::N / L::Ra; it += step) {
       const int b = it / L::Sa, o = it - b * L::Sa;
@@ -535,7 +549,7 @@ struct RowFwdArgs {
   RowSide<T> a, b;    // blocks [0, a_blocks) on side a, the rest on side b
   unsigned a_blocks;
   int nblk, lgcb;
-  const void* tw;     // Cp<S> entries
+  const void* tw;     // Sc<S>::Tw entries
   const T* zeros;     // a row of zeros, read in the place of rows past the last
   const RagRow<T>* items;  // ragged: records, and per CTA (record, row group)
   const int2* ctas;
@@ -672,7 +686,7 @@ __global__ void __launch_bounds__(RowCfg<N>::threads, RowCfg<N>::min_ctas) row_f
   constexpr int TP = RowCfg<N>::TP, Q = RowCfg<N>::Q, NV = Sc<S>::NV;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   pdl_launch();
-  const C* __restrict__ tw = static_cast<const C*>(p.tw);
+  const auto* __restrict__ tw = static_cast<const typename Sc<S>::Tw*>(p.tw);
   int H, W, group, lgcb;
   const T* __restrict__ src;
   Cx<T>* dst;
@@ -786,7 +800,7 @@ __global__ void __launch_bounds__(RowCfg<N>::threads, RowCfg<N>::min_ctas) row_i
   constexpr int TP = RowCfg<N>::TP, Q = RowCfg<N>::Q, NV = Sc<S>::NV;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   pdl_launch();
-  const C* __restrict__ tw = static_cast<const C*>(p.tw);
+  const auto* __restrict__ tw = static_cast<const typename Sc<S>::Tw*>(p.tw);
   int Sy, Sx, Wr, group, lgcb;
   const Cx<T>* __restrict__ src;
   T* out;
@@ -990,7 +1004,7 @@ __device__ __forceinline__ void store_row(Cx<double>* g, Cp<double> v) {
 // the thread's columns) up to, not including, the last; ends with a barrier.
 template <typename S, int N, int RQ>
 __device__ __forceinline__ void col_load_passes(Cp<S>* z, const Cx<typename Sc<S>::real>* __restrict__ g, int H,
-                                                int j0, const Cp<S>* __restrict__ tw) {
+                                                int j0, const typename Sc<S>::Tw* __restrict__ tw) {
   using L = ColPasses<N>;
   using K = ColCfg<S, N>;
   for (int o = j0; o < L::S1; o += K::JT) {
@@ -1031,7 +1045,7 @@ __global__ void __launch_bounds__(ColCfg<S, N>::threads, ColCfg<S, N>::min_ctas)
   using K = ColCfg<S, N>;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   pdl_launch();
-  const C* __restrict__ tw = static_cast<const C*>(p.tw);
+  const auto* __restrict__ tw = static_cast<const typename Sc<S>::Tw*>(p.tw);
   const int pu = threadIdx.x / K::TU, t = threadIdx.x - pu * K::TU;
   const int c = t % K::LC, j0 = t / K::LC;
   C* z = reinterpret_cast<C*>(smem_raw) + pu * K::unit + c;
@@ -1066,7 +1080,7 @@ __global__ void __launch_bounds__(ColCfg<S, N>::threads, ColCfg<S, N>::min_ctas)
   constexpr int NV = Sc<S>::NV, RQ = RAG ? 1 : K::RQ;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   pdl_launch();
-  const C* __restrict__ tw = static_cast<const C*>(p.tw);
+  const auto* __restrict__ tw = static_cast<const typename Sc<S>::Tw*>(p.tw);
   const int pu = threadIdx.x / K::TU, t = threadIdx.x - pu * K::TU;
   const int c = t % K::LC, j0 = t / K::LC;
   C* z = reinterpret_cast<C*>(smem_raw) + pu * K::unit + c;
@@ -1140,7 +1154,13 @@ __global__ void __launch_bounds__(ColCfg<S, N>::threads, ColCfg<S, N>::min_ctas)
       col_load_passes<S, N, RQ>(z, gr + (r * nblk + blk) * (long long)spectrum_rows(Hr, RQ) * K::CB + c * (NV * RQ),
                             act ? Hr : 0, j0, tw);
     for (int j = j0; j < L::TF; j += K::JT) {
-      C x[L::R3];
+      // half of the left spectrum's values are on their way while the right's
+      // last pass runs (all of them do not fit the registers): 4096 points,
+      // 8 partners, 350 us against 387
+      constexpr int PF = LPRE ? L::R3 / 2 : 0;
+      C x[L::R3], ahead[PF > 0 ? PF : 1];
+#pragma unroll
+      for (int q = 0; q < PF; ++q) ahead[q] = ld(lspec + (q * L::TF + j) * K::LC);
       C* base = z + col_item<S, N>(j);
       if constexpr (RPRE) {
         const C* rspec = static_cast<const C*>(p.right) + (r * nblk + blk) * (long long)N * K::LC + c;
@@ -1153,7 +1173,7 @@ __global__ void __launch_bounds__(ColCfg<S, N>::threads, ColCfg<S, N>::min_ctas)
       }
       const C* lb = zl + col_item<S, N>(j);
 #pragma unroll
-      for (int q = 0; q < L::R3; ++q) x[q] = cmul<true>(LPRE ? ld(lspec + (q * L::TF + j) * K::LC) : lb[q * K::LC], x[q]);
+      for (int q = 0; q < L::R3; ++q) x[q] = cmul<true>(q < PF ? ahead[q < PF ? q : 0] : LPRE ? ld(lspec + (q * L::TF + j) * K::LC) : lb[q * K::LC], x[q]);
       Dft<S, 1, L::R3>::run(x);
 #pragma unroll
       for (int m = 0; m < L::R3; ++m) base[m * K::LC] = x[m];

@@ -123,7 +123,7 @@ xc_status ragged_fft_build(RaggedFft* f, const std::vector<FftPair>& pairs, void
       const int n = rows ? p.nx : p.ny;
       auto& m = rows ? twx : twy;
       if (m.count(n)) continue;
-      std::vector<char> t(twiddle_bytes(n, rows != 0));
+      std::vector<char> t(twiddle_bytes(n, rows != 0, XC_F32));
       fill_twiddles(n, rows != 0, XC_F32, t.data());
       m[n] = image.put(t);
     }
