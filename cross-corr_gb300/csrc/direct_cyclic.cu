@@ -39,8 +39,10 @@
 //    overlap another's products).  Results go through a small transpose
 //    buffer, so that each instruction covers 32 consecutive outputs.
 //  * With one block of right rows the output is written; with several, it
-//    starts zeroed and each block adds (red.global.add).  hb bounds an FP32
-//    chain to 4096 products, as the tiled kernel's flushes do.
+//    starts zeroed and each block adds (red.global.add).  The zeros are a
+//    kernel whose dependent launch this one is, so that its CTAs load their
+//    rows meanwhile (one pair of 128x128: 24.6 us, 28.5 after a memset).  hb
+//    bounds an FP32 chain to 4096 products, as the tiled kernel's flushes do.
 //
 // What bounds it: instruction issue (81% of the slots, FMA pipe 73%; a bare
 // loop of such bodies reaches 62 of the 75 TFLOP/s of independent FMAs) in
@@ -209,6 +211,22 @@ __device__ __forceinline__ T overlap_sum(const T* __restrict__ L, const T* __res
   return s;
 }
 
+// Zeros for the blocks to add to.  Launched in stream order: everything before
+// it is done when it starts, so the correlation kernel, which may start right
+// after it did, can read its inputs without waiting.
+template <typename T>
+__global__ void __launch_bounds__(256) zero_kernel(T* out, long long n) {
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  constexpr int V = 16 / (int)sizeof(T);
+  const long long head = min(n, (long long)((16 - (reinterpret_cast<uintptr_t>(out) & 15)) & 15) / (int)sizeof(T));
+  const long long nv = (n - head) / V, tail = head + nv * V;
+  const long long i0 = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+  if (i0 < head) out[i0] = T(0);
+  if (i0 < n - tail) out[tail + i0] = T(0);
+  for (long long i = i0; i < nv; i += (long long)gridDim.x * blockDim.x)
+    reinterpret_cast<float4*>(out + head)[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+}
+
 template <typename T, int TSY, bool WIN>
 __global__ void __launch_bounds__(256, 2) cyclic_kernel(const CycArgs<T> p) {
   using Tl = Tile<T, TSY>;
@@ -259,6 +277,7 @@ __global__ void __launch_bounds__(256, 2) cyclic_kernel(const CycArgs<T> p) {
   }
   stage_rows(sr, p.r_pitch, R, 0, p.hb, hbj, p.Wr, 2 * p.NB, [](int j) { return j * V; },
              [](int j) { return j * 16; });
+  asm volatile("griddepcontrol.wait;" ::: "memory");  // for the zeros
   __syncthreads();
 
   int u, c, uw0, uw1;
@@ -535,15 +554,27 @@ xc_status cyc_launch(const T* left, const T* right, T* out, const Geometry& g, c
   const long long blocks = (long long)pm.n_left * pm.K * c.n_rb * c.groups;
   if (c.n_rb > 1 && !add) {
     const long long n_out = (long long)(pm.n_left - 1) * pm.o_l + (long long)(pm.K - 1) * pm.o_k + 1;
-    XC_CUDA_TRY(cudaMemsetAsync(out, 0, (size_t)n_out * g.Sy * g.Sx * sizeof(T), stream));
+    const long long n = n_out * g.Sy * g.Sx;
+    const long long want = (n * (long long)sizeof(T) + 4095) / 4096;  // 16 bytes a thread
+    zero_kernel<T><<<(unsigned)std::min<long long>(8LL * sm_count(), want), 256, 0, stream>>>(out, n);
+    XC_CUDA_TRY(cudaGetLastError());
   }
   auto kern = c.win ? (c.tsy == 4 ? cyclic_kernel<T, 4, true> : cyclic_kernel<T, 2, true>)
                     : (c.tsy == 4 ? cyclic_kernel<T, 4, false> : cyclic_kernel<T, 2, false>);
   XC_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024));
   const int slot = kernel_timer_begin(stream);
-  kern<<<(unsigned)blocks, 32 * c.nw, c.smem, stream>>>(a);
+  cudaLaunchAttribute attr{};
+  attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr.val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3((unsigned)blocks);
+  cfg.blockDim = dim3(32u * c.nw);
+  cfg.dynamicSmemBytes = (size_t)c.smem;
+  cfg.stream = stream;
+  cfg.attrs = &attr;
+  cfg.numAttrs = c.n_rb > 1 && !add ? 1 : 0;  // without the zero kernel before it, in stream order
+  XC_CUDA_TRY(cudaLaunchKernelEx(&cfg, kern, a));
   kernel_timer_end(slot, stream);
-  XC_CUDA_TRY(cudaGetLastError());
   return XC_OK;
 }
 
