@@ -216,7 +216,8 @@ def workspace_size(mode, dtype, method, left_shape, n_left, right_shape, n_right
 def _stream_ptr(stream) -> Optional[int]:
     if stream is None:
         import torch
-        return torch.cuda.current_stream().cuda_stream
+        # the handle alone: current_stream() builds a Stream object around it (a few us)
+        return torch._C._cuda_getCurrentRawStream(torch.cuda.current_device())
     return int(stream)
 
 
@@ -244,18 +245,19 @@ def correlate(mode: str, left, right, method: str = "direct", out=None, workspac
     if out is None:
         out = torch.empty((n_out, hl + hr - 1, wl + wr - 1), dtype=left.dtype, device=left.device)
     base, _, tile = method.partition(":")
-    ws_bytes = workspace_size(mode, dtype, base, (hl, wl), n, (hr, wr), m)
+    L, b, ls, rs = lib(), ctypes.c_size_t(), Size2(wl, hl), Size2(wr, hr)
+    mode_i, dtype_i, method_i = MODES[mode], DTYPES[dtype], METHODS[base]
+    check(L.xc_workspace_size(mode_i, dtype_i, method_i, ls, n, rs, m, ctypes.byref(b)))
+    ws_bytes = b.value
     if ws_bytes and (workspace is None or workspace.numel() < ws_bytes):
         workspace = torch.empty(ws_bytes, dtype=torch.uint8, device=left.device)
     wptr = workspace.data_ptr() if (workspace is not None and ws_bytes) else None
     if tile:
-        check(lib().xc_correlate_algo(MODES[mode], DTYPES[dtype], Algo(METHODS[base], int(tile)), left.data_ptr(),
-                                      size2(hl, wl), n, right.data_ptr(), size2(hr, wr), m, out.data_ptr(), wptr,
-                                      ws_bytes, _stream_ptr(stream)))
+        check(L.xc_correlate_algo(mode_i, dtype_i, Algo(method_i, int(tile)), left.data_ptr(), ls, n,
+                                  right.data_ptr(), rs, m, out.data_ptr(), wptr, ws_bytes, _stream_ptr(stream)))
     else:
-        check(lib().xc_correlate(MODES[mode], DTYPES[dtype], METHODS[base], left.data_ptr(), size2(hl, wl), n,
-                                 right.data_ptr(), size2(hr, wr), m, out.data_ptr(), wptr, ws_bytes,
-                                 _stream_ptr(stream)))
+        check(L.xc_correlate(mode_i, dtype_i, method_i, left.data_ptr(), ls, n, right.data_ptr(), rs, m,
+                             out.data_ptr(), wptr, ws_bytes, _stream_ptr(stream)))
     return out
 
 
