@@ -466,17 +466,6 @@ double cyc_fill(const CycPlan& c, int C) {
   return res / 16.0 * (c.win ? (double)C / (32.0 * c.win) : 1.0);
 }
 
-int sm_count() {
-  static const int n = [] {
-    int dev = 0, sms = 0;
-    if (cudaGetDevice(&dev) != cudaSuccess ||
-        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || sms <= 0)
-      return 152;
-    return sms;
-  }();
-  return n;
-}
-
 // Row shifts per lane, right rows per block and warps per CTA: the first shape
 // of the list that gives the launch enough warps, the last one otherwise.
 // Longer blocks load and add less per product (a block adds each of its
@@ -495,7 +484,7 @@ bool cyc_plan(const Geometry& g, long long pairs, CycPlan* best) {
   };
   constexpr Shape shapes[] = {{4, 16}, {4, 8}, {2, 8}, {2, 4}, {2, 2}};
   const int chain = f32 ? 4096 / g.Wr : 1 << 30;
-  const long long enough = (f32 ? 6LL : 32LL) * sm_count();
+  const long long enough = (f32 ? 6LL : 32LL) * sm_count_cached();
   bool found = false;
   for (const Shape& sh : shapes) {
     if (sh.hb > chain || (!f32 && sh.tsy == 4) || (sh.hb > 2 && sh.hb / 2 >= g.Hr)) continue;
@@ -508,7 +497,7 @@ bool cyc_plan(const Geometry& g, long long pairs, CycPlan* best) {
       for (bool windowed : {false, true}) {
         CycPlan t;
         if (!cyc_layout<T>(g, pairs, sh.tsy, sh.hb, nw, windowed, &t)) continue;
-        if (nw == 8 && t.warps < 64LL * sm_count()) continue;
+        if (nw == 8 && t.warps < 64LL * sm_count_cached()) continue;
         if (fits && cyc_fill(t, C) <= cyc_fill(c, C)) continue;
         c = t;
         fits = true;
@@ -556,7 +545,7 @@ xc_status cyc_launch(const T* left, const T* right, T* out, const Geometry& g, c
     const long long n_out = (long long)(pm.n_left - 1) * pm.o_l + (long long)(pm.K - 1) * pm.o_k + 1;
     const long long n = n_out * g.Sy * g.Sx;
     const long long want = (n * (long long)sizeof(T) + 4095) / 4096;  // 16 bytes a thread
-    zero_kernel<T><<<(unsigned)std::min<long long>(8LL * sm_count(), want), 256, 0, stream>>>(out, n);
+    zero_kernel<T><<<(unsigned)std::min<long long>(8LL * sm_count_cached(), want), 256, 0, stream>>>(out, n);
     XC_CUDA_TRY(cudaGetLastError());
   }
   auto kern = c.win ? (c.tsy == 4 ? cyclic_kernel<T, 4, true> : cyclic_kernel<T, 2, true>)

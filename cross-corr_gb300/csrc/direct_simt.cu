@@ -495,17 +495,6 @@ int tile_rows(const Geometry& g, int ty) {
   return std::max(0, hi - lo);
 }
 
-int sm_count_cached() {
-  static const int n = [] {
-    int dev = 0, sms = 0;
-    if (cudaGetDevice(&dev) != cudaSuccess ||
-        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || sms <= 0)
-      return 152;
-    return sms;
-  }();
-  return n;
-}
-
 // Rows per slice for a launch of `blocks` tiles: none (0) while the tiles
 // fill a wave of CTAs (`wave` resident at once); else the longest slices (a
 // power of two, at least 4 rows) that give two waves of non-empty slices,

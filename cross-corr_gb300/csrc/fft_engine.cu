@@ -131,7 +131,8 @@ xc_status run(const Engine& e, const void* left, const void* right, void* out, c
   };
   const auto columns = [&](const Cx<T>* src, void* dst, int H, long long mats) {
     ColFwdArgs<T> a{src, dst, H, nblk, mats * nblk, tw + e.tw_col};
-    return launch(e.ck.forward, div_up(a.units, e.ck.pu), e.ck.threads, e.ck.unit_smem, a, stream);
+    const int blocks = div_up(a.units, e.ck.pu);
+    return launch(e.ck.form(blocks, e.sms).forward, blocks, e.ck.threads, e.ck.unit_smem, a, stream);
   };
 
   if (e.shared) XC_TRY(rows(true, 0, e.n_right));
@@ -166,9 +167,10 @@ xc_status run(const Engine& e, const void* left, const void* right, void* out, c
         a.r_k = e.pm.r_k;
         a.r_off = e.shared ? 0 : k0 * e.pm.r_k;
         a.tw = tw + e.tw_col;
-        const void* fn = e.shared ? e.ck.pairs_pre : e.lpre ? e.ck.pairs_lpre : e.ck.pairs;
-        XC_TRY(launch(fn, div_up((long long)nl * a.n_kg * nblk, e.ck.pu), e.ck.threads,
-                      e.ck.unit_smem * (e.shared || e.lpre ? 1 : 2), a, stream));
+        const long long blocks = ((long long)nl * a.n_kg * nblk + e.ck.pu - 1) / e.ck.pu;
+        const ColFns& fns = e.ck.form(blocks, e.sms);
+        const void* fn = e.shared ? fns.pairs_pre : e.lpre ? fns.pairs_lpre : fns.pairs;
+        XC_TRY(launch(fn, blocks, e.ck.threads, e.ck.unit_smem * (e.shared || e.lpre ? 1 : 2), a, stream));
       }
       {
         RowInvArgs<T> a{};
@@ -314,10 +316,13 @@ xc_status engine_plan(Engine* e, xc_dtype dtype, const Geometry& g, const PairMa
 
   XC_TRY(raise_limit(e->rk.forward, e->rk.smem));
   XC_TRY(raise_limit(e->rk.inverse, e->rk.smem));
-  XC_TRY(raise_limit(e->ck.forward, e->ck.unit_smem));
-  XC_TRY(raise_limit(e->ck.pairs_lpre, e->ck.unit_smem));
-  XC_TRY(raise_limit(e->ck.pairs_pre, e->ck.unit_smem));
-  if (2 * e->ck.unit_smem <= 227 * 1024) XC_TRY(raise_limit(e->ck.pairs, 2 * e->ck.unit_smem));
+  for (const ColFns& f : {e->ck.roomy, e->ck.dense}) {
+    XC_TRY(raise_limit(f.forward, e->ck.unit_smem));
+    XC_TRY(raise_limit(f.pairs_lpre, e->ck.unit_smem));
+    XC_TRY(raise_limit(f.pairs_pre, e->ck.unit_smem));
+    if (2 * e->ck.unit_smem <= 227 * 1024) XC_TRY(raise_limit(f.pairs, 2 * e->ck.unit_smem));
+  }
+  e->sms = sm_count_cached();
   e->tw_col = twiddle_bytes(e->nx, true, dtype);
   e->zeros = e->tw_col + twiddle_bytes(e->ny, false, dtype);
   std::vector<char> host(e->zeros + (size_t)e->nx * (f32 ? 4 : 8), 0);

@@ -966,9 +966,23 @@ struct ColCfg {
   static constexpr int TU = JT * LC;
   static constexpr int PU = TU >= 128 ? 1 : (127 + TU) / TU;
   static constexpr int threads = TU * PU;
-  // 64 registers a thread while no radix exceeds 8, else 128
-  static constexpr int min_ctas = (L::R1 <= 8 ? 1024 : 512) / threads;
   static constexpr int unit = L::rows * LC;        // shared-memory elements of a unit
+  // CTAs per SM the registers are cut for: 64 registers a thread while no
+  // radix exceeds 8, else 128.  FP32 transforms of three passes up to 2048
+  // points have a dense form too, with `bufs` units in shared memory: 96
+  // registers, 80 with radix 12 and one buffer, where shared memory has room
+  // for the warps (column kernel, us, with 128 / 96 / 80 registers: 640 points
+  // x 163 outputs 145 / 124 / 124; 768 x 113 183 / 139 / 117; 1024 x 64 125 /
+  // 113 / 118 and col_forward slower at 80; 1536 x 28 162 / 128 / 137; 2560 x
+  // 10 166 / 164 / 164; FP64 is bound by its pipe in all).  Launches of one
+  // wave keep the 128 registers: one pair of 340x340 17.4 us, 18.2 dense.
+  static constexpr bool has_dense = Sc<S>::NV == 2 && L::R1 > 8 && L::Ra > 1 && N <= 2048;
+  static constexpr int ctas(int bufs, bool dense) {
+    const int most = 227 * 1024 / (bufs * PU * unit * 16 + 1024), roomy = 512 / threads;
+    const int want = (L::R1 <= 12 && bufs == 1 ? 768 : 640) / threads, fit = want < most ? want : most;
+    if (L::R1 <= 8) return 1024 / threads;
+    return !dense || fit < roomy ? roomy : fit;
+  }
 };
 
 // A thread's columns of one row of a block, RQ elements apart.
@@ -1038,8 +1052,8 @@ __device__ __forceinline__ int col_item(int j) {
 
 // Full spectra of the columns, in pass order: element (q TF + j) LC + lane
 // holds output q of the last pass's item j.
-template <typename S, int N>
-__global__ void __launch_bounds__(ColCfg<S, N>::threads, ColCfg<S, N>::min_ctas) col_forward(const ColFwdArgs<typename Sc<S>::real> p) {
+template <typename S, int N, bool DENSE>
+__global__ void __launch_bounds__(ColCfg<S, N>::threads, ColCfg<S, N>::ctas(1, DENSE)) col_forward(const ColFwdArgs<typename Sc<S>::real> p) {
   using L = ColPasses<N>;
   using C = Cp<S>;
   using K = ColCfg<S, N>;
@@ -1071,8 +1085,8 @@ __global__ void __launch_bounds__(ColCfg<S, N>::threads, ColCfg<S, N>::min_ctas)
 // the product with the left spectrum (LPRE: read from global memory;
 // otherwise transformed once per group and kept in shared memory), and the
 // inverse transform, whose rows go out in the output's row order.
-template <typename S, int N, bool LPRE, bool RPRE, bool RAG>
-__global__ void __launch_bounds__(ColCfg<S, N>::threads, ColCfg<S, N>::min_ctas) col_pairs(const ColArgs<typename Sc<S>::real> p) {
+template <typename S, int N, bool LPRE, bool RPRE, bool RAG, bool DENSE>
+__global__ void __launch_bounds__(ColCfg<S, N>::threads, ColCfg<S, N>::ctas(LPRE ? 1 : 2, DENSE)) col_pairs(const ColArgs<typename Sc<S>::real> p) {
   using L = ColPasses<N>;
   using C = Cp<S>;
   using K = ColCfg<S, N>;
@@ -1212,13 +1226,18 @@ struct RowKernels {
   const void* rag_inverse;
   int threads, q, nv, smem;
 };
-struct ColKernels {
+struct ColFns {
   const void* forward;
   const void* pairs;       // left transformed in the kernel
   const void* pairs_lpre;  // left spectra from col_forward
   const void* pairs_pre;   // both
   const void* rag_pairs;   // `pairs` over a ragged batch's records (FP32 only)
+};
+struct ColKernels {
+  ColFns roomy, dense;  // (the same where a length has one form)
   int threads, pu, lgcb, rq, unit_smem;  // shared memory of one buffer
+  // the form for a launch of `blocks` CTAs on `sms` SMs: dense beyond one wave
+  const ColFns& form(long long blocks, int sms) const { return blocks > (long long)sms * (512 / threads) ? dense : roomy; }
 };
 // false: no kernels for this length
 bool row_kernels_f32(int n, RowKernels* k);
@@ -1245,15 +1264,22 @@ RowKernels row_kernels_of() {
   k.smem = RowCfg<N>::smem;
   return k;
 }
+template <typename S, int N, bool DENSE>
+ColFns col_fns_of() {
+  ColFns k{};
+  k.forward = (const void*)&col_forward<S, N, DENSE>;
+  k.pairs = (const void*)&col_pairs<S, N, false, false, false, DENSE>;
+  k.pairs_lpre = (const void*)&col_pairs<S, N, true, false, false, DENSE>;
+  k.pairs_pre = (const void*)&col_pairs<S, N, true, true, false, DENSE>;
+  if constexpr (Sc<S>::NV == 2) k.rag_pairs = (const void*)&col_pairs<S, N, false, false, true, DENSE>;
+  return k;
+}
 template <typename S, int N>
 ColKernels col_kernels_of() {
   using K = ColCfg<S, N>;
   ColKernels k{};
-  k.forward = (const void*)&col_forward<S, N>;
-  k.pairs = (const void*)&col_pairs<S, N, false, false, false>;
-  k.pairs_lpre = (const void*)&col_pairs<S, N, true, false, false>;
-  k.pairs_pre = (const void*)&col_pairs<S, N, true, true, false>;
-  if constexpr (Sc<S>::NV == 2) k.rag_pairs = (const void*)&col_pairs<S, N, false, false, true>;
+  k.roomy = col_fns_of<S, N, false>();
+  k.dense = col_fns_of<S, N, K::has_dense>();
   k.threads = K::threads;
   k.pu = K::PU;
   k.lgcb = K::lgcb;

@@ -29,6 +29,7 @@ struct Engine {
   bool shared = false;     // every right serves several lefts: all spectra are made first
   bool lpre = false;       // left spectra are made first
   int l_chunk = 1, k_chunk = 1, kc = 1;
+  int sms = 0;
   size_t off_al = 0, off_ar = 0, off_fl = 0, off_fr = 0, off_b = 0, bytes = 0;
 };
 

@@ -200,7 +200,8 @@ xc_status ragged_fft_build(RaggedFft* f, const std::vector<FftPair>& pairs, void
       a.items = reinterpret_cast<const RagCol<T>*>(base + kv.second.items_at);
       a.units = reinterpret_cast<const int2*>(base + kv.second.list_at);
       a.n_units = (int)kv.second.list.size();
-      col.push_back({ck.rag_pairs, (unsigned)div_up(a.n_units, ck.pu), ck.threads, 2 * ck.unit_smem, blob(a)});
+      const int blocks = div_up(a.n_units, ck.pu);
+      col.push_back({ck.form(blocks, sm_count_cached()).rag_pairs, (unsigned)blocks, ck.threads, 2 * ck.unit_smem, blob(a)});
     }
     for (auto& kv : ch.inv) {
       RowKernels rk{};

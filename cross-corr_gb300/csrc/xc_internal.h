@@ -42,6 +42,9 @@ inline Geometry make_geometry(xc_size2 left, xc_size2 right) {
 
 xc_status debug_expire_wait(uint32_t polls, cudaStream_t stream);
 
+// SMs of the device in use at the first call (152 without one).
+int sm_count_cached();
+
 // Optional CUDA-event timing of the dense kernels (xc_kernel_timing).
 // kernel_timer_begin returns a slot (or -1 when timing is off) that
 // kernel_timer_end closes after the launch on the same stream.

@@ -271,4 +271,15 @@ bool make_pair_map(xc_mode mode, uint32_t n_left, uint32_t n_right, PairMap* pm,
   return true;
 }
 
+int sm_count_cached() {
+  static const int n = [] {
+    int dev = 0, sms = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess ||
+        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || sms <= 0)
+      return 152;
+    return sms;
+  }();
+  return n;
+}
+
 }  // namespace xc
