@@ -99,6 +99,15 @@ xc_status launch(const void* fn, long long blocks, int threads, int smem, Args& 
   return XC_OK;
 }
 
+// Transforms (or units) of `threads` threads per CTA for a launch of `count`:
+// as few as give every SM one CTA, whole warps, at most `most` (128-thread CTAs
+// put a small problem on a few SMs; n_to_mn 4 + 8, 56x56: 18.0 us with those,
+// 14.6 with this rule and the one for short launches below).
+int per_cta(long long count, int most, int threads, int sms) {
+  const long long even = (count + sms - 1) / sms, warp = div_up(32, threads);
+  return (int)std::min<long long>(most, std::max(even, warp));
+}
+
 template <typename T>
 xc_status run(const Engine& e, const void* left, const void* right, void* out, char* ws, cudaStream_t stream) {
   const Geometry& g = e.g;
@@ -109,12 +118,16 @@ xc_status run(const Engine& e, const void* left, const void* right, void* out, c
   char* fr = ws + e.off_fr;
   Cx<T>* b = reinterpret_cast<Cx<T>*>(ws + e.off_b);
   const int lgcb = e.ck.lgcb, nblk = e.nblk;
-  const int rows_per_cta = 2 * e.rk.nv * e.rk.q;
+  const int row_threads = e.rk.threads / e.rk.q, row_smem = e.rk.smem / e.rk.q;
+  const int unit_threads = e.ck.threads / e.ck.pu, unit_smem = e.ck.unit_smem / e.ck.pu;
+  const auto transforms = [&](long long mats, int H) { return mats * div_up(H, 2 * e.rk.nv); };
   const Scales sc = spectrum_scales(e.nx, e.ny);
 
   // rows of `nr` rights from the r0-th on, and (first) of all lefts.  FP64
   // applies all of the result's scale here, in a product that is there anyway.
   const auto rows = [&](bool lefts, long long r0, long long nr) {
+    const int q = per_cta((lefts ? transforms(e.pm.n_left, g.Hl) : 0) + transforms(nr, g.Hr), e.rk.q, row_threads, e.sms);
+    const int rows_per_cta = 2 * e.rk.nv * q;
     RowFwdArgs<T> a{};
     a.a = RowSide<T>{static_cast<const T*>(left), al, g.Hl, g.Wl, div_up(g.Hl, rows_per_cta),
                      (T)sc.left};
@@ -127,12 +140,13 @@ xc_status run(const Engine& e, const void* left, const void* right, void* out, c
     a.lgcb = lgcb;
     a.tw = tw;
     a.zeros = reinterpret_cast<const T*>(tw + e.zeros);
-    return launch(e.rk.forward, ab + nr * a.b.groups, e.rk.threads, e.rk.smem, a, stream);
+    return launch(e.rk.forward, ab + nr * a.b.groups, q * row_threads, q * row_smem, a, stream);
   };
   const auto columns = [&](const Cx<T>* src, void* dst, int H, long long mats) {
     ColFwdArgs<T> a{src, dst, H, nblk, mats * nblk, tw + e.tw_col};
-    const int blocks = div_up(a.units, e.ck.pu);
-    return launch(e.ck.form(blocks, e.sms).forward, blocks, e.ck.threads, e.ck.unit_smem, a, stream);
+    const int pu = per_cta(a.units, e.ck.pu, unit_threads, e.sms);
+    return launch(e.ck.form(div_up(a.units, e.ck.pu), e.sms).forward, div_up(a.units, pu), pu * unit_threads,
+                  pu * unit_smem, a, stream);
   };
 
   if (e.shared) XC_TRY(rows(true, 0, e.n_right));
@@ -167,19 +181,22 @@ xc_status run(const Engine& e, const void* left, const void* right, void* out, c
         a.r_k = e.pm.r_k;
         a.r_off = e.shared ? 0 : k0 * e.pm.r_k;
         a.tw = tw + e.tw_col;
-        const long long blocks = ((long long)nl * a.n_kg * nblk + e.ck.pu - 1) / e.ck.pu;
-        const ColFns& fns = e.ck.form(blocks, e.sms);
+        const long long units = (long long)nl * a.n_kg * nblk;
+        const int pu = per_cta(units, e.ck.pu, unit_threads, e.sms);
+        const ColFns& fns = e.ck.form((units + e.ck.pu - 1) / e.ck.pu, e.sms);
         const void* fn = e.shared ? fns.pairs_pre : e.lpre ? fns.pairs_lpre : fns.pairs;
-        XC_TRY(launch(fn, blocks, e.ck.threads, e.ck.unit_smem * (e.shared || e.lpre ? 1 : 2), a, stream));
+        XC_TRY(launch(fn, (units + pu - 1) / pu, pu * unit_threads, pu * unit_smem * (e.shared || e.lpre ? 1 : 2), a,
+                      stream));
       }
       {
+        const int q = per_cta(transforms((long long)nl * nk, g.Sy), e.rk.q, row_threads, e.sms);
         RowInvArgs<T> a{};
         a.src = b;
         a.out = static_cast<T*>(out);
         a.Sy = g.Sy;
         a.Sx = g.Sx;
         a.Wr = g.Wr;
-        a.groups = div_up(g.Sy, rows_per_cta);
+        a.groups = div_up(g.Sy, 2 * e.rk.nv * q);
         a.nblk = nblk;
         a.lgcb = lgcb;
         a.l0 = l0;
@@ -190,7 +207,7 @@ xc_status run(const Engine& e, const void* left, const void* right, void* out, c
         a.scale_hi = (T)sc.rest;
         a.scale_lo = (T)(sc.rest - (double)a.scale_hi);
         a.tw = tw;
-        XC_TRY(launch(e.rk.inverse, (long long)nl * nk * a.groups, e.rk.threads, e.rk.smem, a, stream));
+        XC_TRY(launch(e.rk.inverse, (long long)nl * nk * a.groups, q * row_threads, q * row_smem, a, stream));
       }
     }
   }
@@ -261,13 +278,35 @@ xc_status engine_plan(Engine* e, xc_dtype dtype, const Geometry& g, const PairMa
   e->nblk = div_up(e->nx / 2 + 1, cb);
   const size_t row = (size_t)e->nblk * cb * ce;  // bytes of one spectrum row
   const auto rows = [&](int H) { return row * spectrum_rows(H, e->ck.rq); };
-  e->shared = pm.r_l == 0 && pm.n_left > 1;
+  e->sms = sm_count_cached();
+  // FP64 keeps the library transforms unless the launches fill the GPU: a
+  // transform's chain of FP64 instructions is long, and their shorter ones
+  // spread a small problem better.  Over 303 problems of up to 256x256 the
+  // kernels take 0.5 to 2.3 times as long below 1.1 million points of output
+  // (2 million where spectra are shared), beyond it 0.42 to 0.91 times.
+  const bool n_to_m = pm.r_l == 0 && pm.n_left > 1;
+  const long long points = (long long)pm.n_left * pm.K * e->nx * e->ny;
+  if (!f32 && points < (n_to_m ? 2 << 20 : 1100 << 10)) return XC_OK;
+  // Short FP32 launches (one wave of the column kernel) take every pair by
+  // itself, both column transforms included: three kernels instead of four or
+  // five, the SMs have nothing else to do (n_to_m 2 + 2, 56x56: 14.4 us,
+  // 27.3 in five kernels of full CTAs).
+  const long long pair_units = (long long)pm.n_left * pm.K * e->nblk;
+  const bool brief = f32 && 2 * e->ck.unit_smem <= 227 * 1024 &&
+                     pair_units <= (long long)e->sms * (512 / e->ck.threads) * e->ck.pu;
+  e->shared = n_to_m && !brief;
+  e->lpre = false;
   // The left spectra are made first (col_forward) when several partners use
-  // them: transforming the left's columns in every CTA of the column kernel
-  // doubles the serial work before its first product (one_to_many 256x256 x
-  // 64: column kernel 47 us against 32).  One to three partners save the
-  // launch instead, while both blocks' shared memory leaves two CTAs per SM.
-  e->lpre = !e->shared && (pm.K >= 4 || 2 * e->ck.unit_smem > 100 * 1024);
+  // them: transforming the left's columns in the column kernel doubles the
+  // serial work before its first product (one_to_many 256x256 x 64: column
+  // kernel 47 us against 32).  Short launches with few partners save that
+  // kernel instead.  The whole chain, us, left in the column kernel / first:
+  // 640 points 1 partner 17.7 / 25.5, 2: 24.2 / 26.7, 3: 32.0 / 27.4; 1024: 1:
+  // 23.2 / 29.8, 2: 33.2 / 29.3; 2048: 1: 37.8 / 36.9; 4096: 1: 155 / 148.
+  // The other way runs where the workspace has no room for the full spectra
+  // (one pair whose length is rounded up by much, 700x700: 32 us; it fell back
+  // to the library transforms and took 119).
+  const bool lpre = !brief && (pm.K >= 4 || (pm.K > 1 && (!f32 || pm.K * e->ny >= 1920)) || e->ny > 2048);
 
   // Workspace: row spectra of the lefts and of a chunk of rights, full
   // spectra of shared matrices, column-inverted products of a chunk: all
@@ -282,8 +321,8 @@ xc_status engine_plan(Engine* e, xc_dtype dtype, const Geometry& g, const PairMa
     off += align256(bytes);
     return at;
   };
-  if (e->shared || e->lpre) e->off_fl = take(row * e->ny * pm.n_left);
   if (e->shared) {
+    e->off_fl = take(row * e->ny * pm.n_left);
     e->off_fr = take(row * e->ny * n_right);
     const size_t at = off;
     e->off_al = take(rows(g.Hl) * pm.n_left);
@@ -301,15 +340,32 @@ xc_status engine_plan(Engine* e, xc_dtype dtype, const Geometry& g, const PairMa
     off = std::max(a_end, at + align256(b1 * e->l_chunk * e->k_chunk));
     e->kc = 1;
   } else {
-    e->off_al = take(rows(g.Hl) * pm.n_left);
     e->l_chunk = pm.n_left;
-    const size_t per_k = (ar1 + b1) * pm.n_left;  // r_k = n_left rights (one for a single left)
-    if (off + per_k + 512 > ws_bytes) return XC_OK;
-    const long long fit = (long long)((ws_bytes - off - 512) / per_k);
-    e->k_chunk = div_up(pm.K, div_up(pm.K, (int)std::min<long long>(pm.K, fit)));  // even chunks
-    e->off_ar = take(ar1 * pm.n_left * e->k_chunk);
-    e->off_b = take(b1 * pm.n_left * e->k_chunk);
-    e->kc = e->lpre ? 1 : e->k_chunk;
+    const size_t al1 = rows(g.Hl) * pm.n_left, fl1 = row * e->ny * pm.n_left;
+    const auto place = [&](bool first, int most) {
+      for (int c = 1; c <= most; ++c) {  // as few chunks of partners as fit, even ones
+        const int k = div_up(pm.K, c);
+        off = 0;
+        if (first) e->off_fl = take(fl1);
+        else e->off_al = take(al1);
+        e->off_ar = take(ar1 * pm.r_k * k);
+        // the first products replace the lefts' row spectra once those are transformed
+        e->off_b = take(std::max(b1 * pm.n_left * k, first ? al1 : 0));
+        if (first) e->off_al = e->off_b;
+        if (off > ws_bytes) continue;
+        e->lpre = first;
+        e->k_chunk = k;
+        e->kc = first || brief ? 1 : k;
+        return true;
+      }
+      return false;
+    };
+    // the preferred way in one chunk, the other in one, either in several
+    const bool room = 2 * e->ck.unit_smem <= 227 * 1024;  // both blocks' in the column kernel
+    bool placed = false;
+    for (int most : {1, pm.K})
+      for (bool first : {lpre, !lpre}) placed = placed || ((first || room) && place(first, most));
+    if (!placed) return XC_OK;
   }
   e->bytes = off;
   if (e->bytes > ws_bytes) return XC_OK;
@@ -322,7 +378,6 @@ xc_status engine_plan(Engine* e, xc_dtype dtype, const Geometry& g, const PairMa
     XC_TRY(raise_limit(f.pairs_pre, e->ck.unit_smem));
     if (2 * e->ck.unit_smem <= 227 * 1024) XC_TRY(raise_limit(f.pairs, 2 * e->ck.unit_smem));
   }
-  e->sms = sm_count_cached();
   e->tw_col = twiddle_bytes(e->nx, true, dtype);
   e->zeros = e->tw_col + twiddle_bytes(e->ny, false, dtype);
   std::vector<char> host(e->zeros + (size_t)e->nx * (f32 ? 4 : 8), 0);

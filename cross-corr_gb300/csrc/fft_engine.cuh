@@ -594,7 +594,8 @@ struct RowInvArgs {
   const int2* ctas;
 };
 
-// Row kernels: a transform (NV row pairs) on TP threads, Q of them per CTA.
+// Row kernels: a transform (NV row pairs) on TP threads, Q of them per CTA
+// (fewer in short launches, see per_cta).
 template <int N>
 struct RowCfg {
   using L = RowPasses<N>;
@@ -683,7 +684,8 @@ __global__ void __launch_bounds__(RowCfg<N>::threads, RowCfg<N>::min_ctas) row_f
   using L = RowPasses<N>;
   using C = Cp<S>;
   using T = typename Sc<S>::real;
-  constexpr int TP = RowCfg<N>::TP, Q = RowCfg<N>::Q, NV = Sc<S>::NV;
+  constexpr int TP = RowCfg<N>::TP, NV = Sc<S>::NV;
+  const int Q = blockDim.x / TP;  // at most RowCfg<N>::Q
   extern __shared__ __align__(16) unsigned char smem_raw[];
   pdl_launch();
   const auto* __restrict__ tw = static_cast<const typename Sc<S>::Tw*>(p.tw);
@@ -797,7 +799,8 @@ __global__ void __launch_bounds__(RowCfg<N>::threads, RowCfg<N>::min_ctas) row_i
   using L = RowPasses<N>;
   using C = Cp<S>;
   using T = typename Sc<S>::real;
-  constexpr int TP = RowCfg<N>::TP, Q = RowCfg<N>::Q, NV = Sc<S>::NV;
+  constexpr int TP = RowCfg<N>::TP, NV = Sc<S>::NV;
+  const int Q = blockDim.x / TP;  // at most RowCfg<N>::Q
   extern __shared__ __align__(16) unsigned char smem_raw[];
   pdl_launch();
   const auto* __restrict__ tw = static_cast<const typename Sc<S>::Tw*>(p.tw);
@@ -940,7 +943,7 @@ __global__ void __launch_bounds__(RowCfg<N>::threads, RowCfg<N>::min_ctas) row_i
 // ---------------------------------------------------------------------------
 // Column kernels: a unit is one block of CB columns of one matrix (or pair),
 // on TU threads, lanes over the block's columns (NV at a time) first; PU
-// units per CTA.
+// units per CTA (fewer in short launches).
 // ---------------------------------------------------------------------------
 template <typename S, int N>
 struct ColCfg {
@@ -1063,7 +1066,7 @@ __global__ void __launch_bounds__(ColCfg<S, N>::threads, ColCfg<S, N>::ctas(1, D
   const int pu = threadIdx.x / K::TU, t = threadIdx.x - pu * K::TU;
   const int c = t % K::LC, j0 = t / K::LC;
   C* z = reinterpret_cast<C*>(smem_raw) + pu * K::unit + c;
-  const long long u = (long long)blockIdx.x * K::PU + pu;
+  const long long u = (long long)blockIdx.x * (blockDim.x / K::TU) + pu;
   const bool live = u < p.units;
   pdl_wait();
   col_load_passes<S, N, K::RQ>(z, p.src + (live ? u : 0) * spectrum_rows(p.H, K::RQ) * K::CB + c * (Sc<S>::NV * K::RQ), live ? p.H : 0, j0, tw);
@@ -1098,8 +1101,9 @@ __global__ void __launch_bounds__(ColCfg<S, N>::threads, ColCfg<S, N>::ctas(LPRE
   const int pu = threadIdx.x / K::TU, t = threadIdx.x - pu * K::TU;
   const int c = t % K::LC, j0 = t / K::LC;
   C* z = reinterpret_cast<C*>(smem_raw) + pu * K::unit + c;
-  C* zl = z + (LPRE ? 0 : K::PU * K::unit);  // left spectrum
-  const unsigned gu = blockIdx.x * K::PU + pu;
+  const int PU = blockDim.x / K::TU;  // units of this launch's CTAs, at most K::PU
+  C* zl = z + (LPRE ? 0 : PU * K::unit);  // left spectrum
+  const unsigned gu = blockIdx.x * PU + pu;
   unsigned blk;
   int ll = 0, ka = 0, nk, kc = 1, Hl, Hr, Sy, nblk;
   long long l = 0;
@@ -1235,7 +1239,7 @@ struct ColFns {
 };
 struct ColKernels {
   ColFns roomy, dense;  // (the same where a length has one form)
-  int threads, pu, lgcb, rq, unit_smem;  // shared memory of one buffer
+  int threads, pu, lgcb, rq, unit_smem;  // of pu units; shared memory of one buffer
   // the form for a launch of `blocks` CTAs on `sms` SMs: dense beyond one wave
   const ColFns& form(long long blocks, int sms) const { return blocks > (long long)sms * (512 / threads) ? dense : roomy; }
 };

@@ -59,19 +59,17 @@ def test_modes_and_ragged_sizes(mode, n, m, ls, rs, dtype):
     check(mode, n, m, ls, rs, dtype, "normal")
 
 
-@pytest.mark.parametrize("mode,n,m", [("one_to_many", 1, 45), ("n_to_mn", 2, 50), ("n_to_m", 3, 17)])
-def test_several_chunks(mode, n, m):
-    """More partners than one chunk of intermediate spectra holds (a chunk is
-    64 MiB: about 20 partners of these sizes, fewer with two lefts), against
-    the library transforms run stage by stage."""
-    left = torch.from_numpy(seeded((n, 400, 380), 7, "uniform")).cuda()
-    right = torch.from_numpy(seeded((m, 390, 400), 8, "uniform")).cuda()
-    plan = xcorr.FftPlan(mode, "f32", (400, 380), n, (390, 400), m)
+def check_against_stages(mode, n, m, ls, rs, dtype):
+    """The fused result against the library transforms run stage by stage."""
+    npdt = np.float32 if dtype == "f32" else np.float64
+    left = torch.from_numpy(seeded((n,) + ls, 7, "uniform", npdt)).cuda()
+    right = torch.from_numpy(seeded((m,) + rs, 8, "uniform", npdt)).cuda()
+    plan = xcorr.FftPlan(mode, dtype, ls, n, rs, m)
     ws = torch.empty(plan.workspace_bytes, dtype=torch.uint8, device="cuda")
-    shape = (xcorr.output_count(mode, n, m), 789, 779)
-    out = torch.full(shape, float("nan"), device="cuda")
+    shape = (xcorr.output_count(mode, n, m), ls[0] + rs[0] - 1, ls[1] + rs[1] - 1)
+    out = torch.full(shape, float("nan"), dtype=left.dtype, device="cuda")
     plan.execute(left, right, out, ws)
-    ref = torch.empty(shape, device="cuda")
+    ref = torch.empty(shape, dtype=left.dtype, device="cuda")
     s, L = torch.cuda.current_stream().cuda_stream, xcorr.lib()
     xcorr.check(L.xc_fft_forward(plan.handle, left.data_ptr(), right.data_ptr(), ws.data_ptr(), ws.numel(), s))
     xcorr.check(L.xc_fft_multiply(plan.handle, ws.data_ptr(), ws.numel(), s))
@@ -79,7 +77,23 @@ def test_several_chunks(mode, n, m):
     torch.cuda.synchronize()
     plan.close()
     err = (out - ref).abs().amax(dim=(1, 2)) / ref.abs().amax(dim=(1, 2))
-    assert float(err.max()) <= 1e-5  # (a NaN fails: nothing was left unwritten)
+    assert float(err.max()) <= TOL[dtype]  # (a NaN fails: nothing was left unwritten)
+
+
+@pytest.mark.parametrize("mode,n,m", [("one_to_many", 1, 45), ("n_to_mn", 2, 50), ("n_to_m", 3, 17)])
+def test_many_partners(mode, n, m):
+    """More partners than a launch has waves: the column kernels' dense form."""
+    check_against_stages(mode, n, m, (400, 380), (390, 400), "f32")
+
+
+@pytest.mark.parametrize("dtype", ["f32", "f64"])
+@pytest.mark.parametrize("mode,n,m", [("one_to_one", 1, 1), ("one_to_many", 1, 2), ("n_to_mn", 2, 6)])
+@pytest.mark.parametrize("size", [320, 530, 700, 1000, 1100, 1300, 1900])
+def test_few_large_partners(size, mode, n, m, dtype):
+    """Either side of the rule for making the left spectra first, and sizes
+    whose workspace has no room for them (lengths rounded up by much)."""
+    check_against_stages(mode, n, m, (size, size), (size, size), dtype)
+    check_against_stages(mode, n, m, (size, size - 7), (size - 30, size // 2), dtype)
 
 
 def test_beyond_the_kernels_lengths():
