@@ -38,6 +38,8 @@
 //    its row-shift tiles meet, loaded whole before the products (a CTA's loads
 //    overlap another's products).  Results go through a small transpose
 //    buffer, so that each instruction covers 32 consecutive outputs.
+//  * The wider matrix of a pair takes the left's part: correlating the right
+//    with the left gives the same outputs, mirrored.
 //  * With one block of right rows the output is written; with several, it
 //    starts zeroed and each block adds (red.global.add).  The zeros are a
 //    kernel whose dependent launch this one is, so that its CTAs load their
@@ -227,7 +229,10 @@ __global__ void __launch_bounds__(256) zero_kernel(T* out, long long n) {
     reinterpret_cast<float4*>(out + head)[i] = make_float4(0.f, 0.f, 0.f, 0.f);
 }
 
-template <typename T, int TSY, bool WIN>
+// FLIP: `left` holds the pairs' right matrices and `right` the left ones, and
+// the outputs are mirrored.  (A form of its own: the choice of address at run
+// time cost 1 to 4% of the other launches.)
+template <typename T, int TSY, bool WIN, bool FLIP>
 __global__ void __launch_bounds__(256, 2) cyclic_kernel(const CycArgs<T> p) {
   using Tl = Tile<T, TSY>;
   constexpr int TSX = Tl::TSX;
@@ -243,10 +248,11 @@ __global__ void __launch_bounds__(256, 2) cyclic_kernel(const CycArgs<T> p) {
   const int rb = (int)(bid % (unsigned)p.n_rb);
   bid /= (unsigned)p.n_rb;
   const int k = (int)(bid % (unsigned)p.pm.K), l = (int)(bid / (unsigned)p.pm.K);
-  const T* __restrict__ L = p.left + (long long)l * p.Hl * p.Wl;
+  const long long lefts = l, rights = l * p.pm.r_l + k * p.pm.r_k;
+  const T* __restrict__ L = p.left + (FLIP ? rights : lefts) * p.Hl * p.Wl;
   const int b0 = rb * p.hb, hbj = min(p.hb, p.Hr - b0);
-  const T* __restrict__ R = p.right + ((l * p.pm.r_l + k * p.pm.r_k) * p.Hr + b0) * (long long)p.Wr;
-  T* out = p.out + (l * p.pm.o_l + k * p.pm.o_k) * p.Sy * (long long)p.Sx;
+  const T* __restrict__ R = p.right + ((FLIP ? lefts : rights) * p.Hr + b0) * (long long)p.Wr;
+  T* out = p.out + (l * p.pm.o_l + k * p.pm.o_k) * p.Sy * (long long)p.Sx + (FLIP ? p.Sy * (long long)p.Sx - 1 : 0);
 
   // This CTA's tiles u0 .. u1; left row (u - u0) TSY + i of shared memory is
   // row u TSY - (hb - 1) + i of the matrix, which right row i - t of the block
@@ -313,12 +319,14 @@ __global__ void __launch_bounds__(256, 2) cyclic_kernel(const CycArgs<T> p) {
   const int sx = c * TSX + p.Wr - 1;                    // of q = 0, m = 0
   const int P = p.C * TSX;
   // a sum that is NaN is made again from what its shift meets (`redo`)
-  const auto emit = [&](T* dst, T v) {
+  const auto emit = [&](int oy, int ox, T v) {
+    const long long at = (long long)oy * p.Sx + ox;
+    T* dst = FLIP ? out - at : out + at;
     if (p.accumulate) atomicAdd(dst, v);  // result unused: red.global.add
     else *dst = v;
   };
   const auto redo = [&](int oy, int ox) {
-    emit(out + (long long)oy * p.Sx + ox,
+    emit(oy, ox,
          overlap_sum(L, R, p.Hl, p.Wl, hbj, p.Wr, oy - (p.Hr - 1) + b0, ox - (p.Wr - 1)));
   };
   // the warp's buffer, as the sums of segment mm of every lane in `mask`
@@ -335,7 +343,7 @@ __global__ void __launch_bounds__(256, 2) cyclic_kernel(const CycArgs<T> p) {
       for (int t = 0; t < TSY; ++t)
         if (fy + t >= 0 && fy + t < p.Sy) {
           const T v = buf[t * (32 * TSX) + j * 32 + lane];
-          if (v == v) emit(out + (long long)(fy + t) * p.Sx + fx, v);
+          if (v == v) emit(fy + t, fx, v);
           else bad |= 1u << (j * TSY + t);
         }
     }
@@ -381,7 +389,7 @@ __global__ void __launch_bounds__(256, 2) cyclic_kernel(const CycArgs<T> p) {
             const int x = sx - m * P + q;
             if (sy + t >= 0 && sy + t < p.Sy && x >= 0 && x < p.Sx) {
               const T v = a.get(t, q);
-              if (v == v) emit(out + (long long)(sy + t) * p.Sx + x, v);
+              if (v == v) emit(sy + t, x, v);
               else bad |= 1u << (t * TSX + q);
             }
           }
@@ -511,9 +519,18 @@ bool cyc_plan(const Geometry& g, long long pairs, CycPlan* best) {
 }
 
 template <typename T>
-xc_status cyc_launch(const T* left, const T* right, T* out, const Geometry& g, const PairMap& pm, cudaStream_t stream,
+xc_status cyc_launch(const T* left, const T* right, T* out, Geometry g, const PairMap& pm, cudaStream_t stream,
                      bool add, bool* taken) {
   constexpr int TSX = 32 / (int)sizeof(T);
+  // A left narrower than the right changes places with it: few classes wrap
+  // often, and every wrap costs a surplus block and a hand-over (16x16 by
+  // 128x128 27.6 us, 8.1 with places changed; x 24 43.0 and 16.4).
+  const bool flip = g.Wl < g.Wr;
+  if (flip) {
+    std::swap(g.Hl, g.Hr);
+    std::swap(g.Wl, g.Wr);
+    std::swap(left, right);
+  }
   CycPlan c;
   *taken = cyc_plan<T>(g, (long long)pm.n_left * pm.K, &c);
   if (!*taken) return XC_OK;
@@ -548,8 +565,11 @@ xc_status cyc_launch(const T* left, const T* right, T* out, const Geometry& g, c
     zero_kernel<T><<<(unsigned)std::min<long long>(8LL * sm_count_cached(), want), 256, 0, stream>>>(out, n);
     XC_CUDA_TRY(cudaGetLastError());
   }
-  auto kern = c.win ? (c.tsy == 4 ? cyclic_kernel<T, 4, true> : cyclic_kernel<T, 2, true>)
-                    : (c.tsy == 4 ? cyclic_kernel<T, 4, false> : cyclic_kernel<T, 2, false>);
+  const auto pick = [&](auto plain, auto mirrored) { return flip ? mirrored : plain; };
+  auto kern = c.win ? (c.tsy == 4 ? pick(cyclic_kernel<T, 4, true, false>, cyclic_kernel<T, 4, true, true>)
+                                  : pick(cyclic_kernel<T, 2, true, false>, cyclic_kernel<T, 2, true, true>))
+                    : (c.tsy == 4 ? pick(cyclic_kernel<T, 4, false, false>, cyclic_kernel<T, 4, false, true>)
+                                  : pick(cyclic_kernel<T, 2, false, false>, cyclic_kernel<T, 2, false, true>));
   XC_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024));
   const int slot = kernel_timer_begin(stream);
   cudaLaunchAttribute attr{};
