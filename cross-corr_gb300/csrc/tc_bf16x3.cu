@@ -149,13 +149,13 @@ struct TcParams {
   int mats_mode;    // 1: one TMA box per row shift spans P partners; 0: one box per partner spans DY rows
   int n_pgroups;    // ceil(K / P)
   int n_dytiles;    // ceil(Sy / DY)
-  // A work item covers one x-part (shifts [512 xp, 512 xp + 512), in two
-  // halves) and one k-part (right columns [256 kp, 256 kp + 256)) of its
+  // A work item covers one x-part (shifts [2 half_w xp, 2 half_w (xp + 1)), in
+  // two halves) and one k-part (right columns [256 kp, 256 kp + 256)) of its
   // rows; parts of the same outputs add into them like row chunks do.
   int n_parts;      // work items per tile key: n_xparts * n_kparts
   int n_kparts;
   int half_w;       // shifts per half (a multiple of 16, at most 256): half h of x-part xp
-                    // covers [512 xp + h half_w, 512 xp + (h+1) half_w)
+                    // covers [(2 xp + h) half_w, (2 xp + h + 1) half_w)
   int rowsplit;     // 1 (Sx <= 256): issuer h takes every other left row, each over all
                     // shifts (half_w of them) in its own accumulator, instead of a half of
                     // the shifts of every row
@@ -386,7 +386,7 @@ struct TcItem {
 __host__ __device__ __forceinline__ bool tc_piece(const TcParams& p, int part, int lp, int rank, int row0, int n,
                                                   TcItem* w) {
   const int xp = part / p.n_kparts, kp = part % p.n_kparts;
-  w->s0 = 512 * xp;
+  w->s0 = 2 * p.half_w * xp;
   w->kbase = 256 * kp;
   const int chunk_cols = 4 * p.kstep;
   w->nkc = min(p.nkc, (p.Wr - w->kbase + chunk_cols - 1) / chunk_cols);
@@ -1449,7 +1449,7 @@ bool tc_plan(const Geometry& g, const PairMap& pm, bool tf32, TcPlan* t, bool ba
   t->P = P;
   t->DY = kLanes / P;
   t->mats_mode = P >= 8 ? 1 : 0;
-  // x-parts of 512 shifts (two halves), k-parts of 256 right columns
+  // x-parts of up to 512 shifts (two halves), k-parts of 256 right columns
   const TcParts parts = tc_parts(g.Sx, g.Wr, tf32);
   // One accumulator holds every shift: the issuers split the rows instead.
   // BF16 rights of more than one column chunk only up to 208 shifts: with four
@@ -1459,7 +1459,8 @@ bool tc_plan(const Geometry& g, const PairMap& pm, bool tf32, TcPlan* t, bool ba
   // of 120x130 by 120x120 90 and 94; TF32 221 and 187, 170 and 147, 238 and
   // 195, 142 and 124).
   t->rowsplit = g.Sx <= kHalfCols && (tf32 || g.Wr <= 64 || g.Sx <= 208) ? 1 : 0;
-  t->half_w = t->rowsplit ? div_up(g.Sx, 16) * 16 : parts.half_w;
+  t->half_w = t->rowsplit ? div_up(g.Sx, 16) * 16
+              : parts.n_xparts > 1 ? tc_even_half(g.Sx, parts.n_xparts) : parts.half_w;
   t->n_kparts = parts.n_kparts;
   t->n_parts = parts.n_xparts * parts.n_kparts;
   t->es = tf32 ? 4 : 2;                 // bytes per operand element
