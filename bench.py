@@ -376,7 +376,7 @@ def run_ours(args, rank, world, local_rank):
         bound, peak, unit = "fp32", 152 * 128 * 2 * mhz * 1e6 / 1e12, "TFLOP/s"
         peak_note = "nominal FP32 FMA peak (152 SMs x 128 lanes x 2 x max SM clock); no measured SIMT peak exists"
     clocks = clk.summary()
-    kernel_name = "tc_kernel" if method.startswith("tc_") else "direct_kernel"
+    kernel_name = "tc_kernel" if method.startswith("tc_") else "cyclic_kernel"
     line = {
         "metric": METRIC, "value": value, "unit": "correlations/s", "n_gpus": world, "steps": args.steps,
         "warmup": args.warmup, "ms_per_step": ms_max, "higher_is_better": True, "scaling": "weak",
@@ -412,14 +412,12 @@ def run_ours(args, rank, world, local_rank):
         "gpu_launches": gpu_launches(method, args.steps),
     }
     if method == "fft":
-        # the step is two cuFFT transforms around four glue kernels: the
-        # transforms are the library's, timed but not modelled; the glue
-        # kernels' HBM fractions come from their own captures
+        # four fused kernels, none of them dominant: their HBM fractions come
+        # from their own captures
         line["roofline"] = {"bound": "hbm", "achieved": None, "peak": float(peaks.get("hbm_gbs", 6800.0)),
                             "unit": "GB/s", "frac": None, "traffic": None, "kernel": "fft step",
-                            "note": "cuFFT transforms plus pad, conj-multiply and normalise kernels; the glue "
-                                    "kernels' achieved GB/s against this peak are in "
-                                    "profiles/fft_glue_one_to_many_256x64.md"}
+                            "note": "row, column and inverse row kernels; their achieved GB/s against this peak "
+                                    "are in profiles/fft_kernels_one_to_many_256x64.md"}
     if plain is not None:
         line["plain_fp32"] = plain
     if tf32 is not None:
@@ -871,10 +869,10 @@ def reference_gpu_study(torch, xcorr, line, reps=10):
 
 
 def gpu_launches(method, steps):
-    # kernels per xc_correlate call: direct 1; fft 2 pads + multiply + normalise
-    # (+ cuFFT's own); tc: sums; column sums with the means, split planes,
+    # kernels per xc_correlate call: direct: zeros, correlation; fft: rows, left
+    # columns, column products, inverse rows; tc: sums; column sums with the means, split planes,
     # accumulation windows and work list; row scans; correction; tcgen05 kernel
-    per_step = {"direct": 1, "fft": 4, "tc_bf16x3": 5, "tc_tf32x3": 5}.get(method, 1)
+    per_step = {"direct": 2, "fft": 4, "tc_bf16x3": 5, "tc_tf32x3": 5}.get(method, 1)
     return per_step * steps
 
 

@@ -46,7 +46,7 @@
 //    rows meanwhile (one pair of 128x128: 24.6 us, 28.5 after a memset).  hb
 //    bounds an FP32 chain to 4096 products, as the tiled kernel's flushes do.
 //
-// What bounds it: instruction issue (81% of the slots, FMA pipe 73%; a bare
+// What bounds it: instruction issue (83% of the slots, FMA pipe 76%; a bare
 // loop of such bodies reaches 62 of the 75 TFLOP/s of independent FMAs) in
 // FP32, the FP64 pipe in FP64.
 #include <algorithm>

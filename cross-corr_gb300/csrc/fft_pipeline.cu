@@ -1,4 +1,6 @@
-// fft_pipeline.cu -- FFT-based correlation of a whole batch:
+// fft_pipeline.cu -- FFT-based correlation of a whole batch.  Normalised
+// results go to the fused kernels (fft_engine.cu) where those take the problem;
+// else, and for the separate stages and the raw circular result:
 //   pad (device) -> batched in-place R2C of every left and right matrix ->
 //   fused conj-multiply over the mode's pair map -> batched in-place C2R ->
 //   device normalisation (or the raw circular result).

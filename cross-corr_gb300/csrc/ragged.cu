@@ -111,7 +111,7 @@ struct RaggedPlanImpl {
     CopyJob* jobs = nullptr;  // the matrices the variant's plain pairs use, and the first block of each
     int* first = nullptr;
     int n_left = 0, n_jobs = 0, repack_blocks = 0;
-    int tc_pairs = 0;  // pairs of the variant's route (split-BF16 calls)
+    int tc_pairs = 0;  // pairs of the variant's route
     int grid = 0;
     cudaGraph_t graph = nullptr;
     cudaGraphExec_t exec = nullptr;
@@ -416,7 +416,7 @@ std::string cache_path() {
   return std::string(home ? home : "/tmp") + "/.cache/xcorr_gb300_autotune.jsonl";
 }
 
-// Side streams of the split-BF16 routes: XC_RAGGED_TC_STREAMS (1-8), default
+// Side streams of the routes: XC_RAGGED_TC_STREAMS (1-8), default
 // 8 (512-pair batch, 448 pairs routed, 32-row items: 31.8 ms on 6 streams,
 // 30.6 ms on 8; with the lone-call item rule 40.9 / 34.2 / 33.3 ms on 2 / 4 / 8).
 int tc_stream_count() {

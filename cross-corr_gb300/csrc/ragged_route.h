@@ -1,6 +1,7 @@
-// ragged_route.h -- host planning of a ragged plan's split-BF16 routes:
-// which pairs a route sends to the split tensor-core path, and how those
-// calls are dealt out to the side streams.  Header-only, shared by ragged.cu
+// ragged_route.h -- host planning of a ragged plan's routes: which pairs leave
+// the plain kernel, and how those that run as calls of the split tensor-core
+// path (outputs beyond the FFT kernels' lengths) are dealt out to the side
+// streams.  Header-only, shared by ragged.cu
 // and a CPU test harness (tests/ragged_route_check.cpp).
 #pragma once
 
@@ -12,8 +13,8 @@
 namespace xc {
 
 // Routes of an FP32 plan: 0 keeps every pair on the plain kernel; 1-4 send
-// the pairs with at least 2^32, 2^30, 2^28, 2^26 multiply-adds (that the
-// split path takes) to the split path.
+// the pairs with at least 2^32, 2^30, 2^28, 2^26 multiply-adds to the FFT
+// kernels or the split path.
 constexpr int kRaggedRoutes = 5;
 
 inline double route_min_mac(int route) { return route <= 0 ? 0.0 : std::ldexp(1.0, 34 - 2 * route); }

@@ -418,8 +418,8 @@ class RaggedPlan:
 
     def describe(self, variant=-1):
         """Variant `variant` (-1: the chosen one) as a dict: its index, the
-        plan's variant count, the plain kernel's tile shape, and the pairs run
-        on the split-BF16 path (count and multiply-add threshold)."""
+        plan's variant count, the plain kernel's tile shape, and the pairs
+        that leave the plain kernel (count and multiply-add threshold)."""
         v = RaggedVariant()
         check(lib().xc_ragged_describe(self.handle, variant, ctypes.byref(v)))
         return {"index": v.index, "n_variants": v.n_variants, "tile_shape": v.tile_shape, "tc_pairs": v.tc_pairs,

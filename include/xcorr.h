@@ -55,15 +55,16 @@ typedef enum xc_dtype { XC_F32 = 0, XC_F64 = 1 } xc_dtype;
 
 typedef enum xc_method {
   XC_METHOD_AUTO = 0,     /* library choice */
-  XC_METHOD_DIRECT = 1,   /* plain definition-based kernel (FP32 or FP64 FMA, TMA-staged) */
-  XC_METHOD_FFT = 2,      /* cuFFT transforms + fused pad / conj-multiply / normalise kernels */
+  XC_METHOD_DIRECT = 1,   /* plain definition-based kernel (FP32 or FP64 FMA) */
+  XC_METHOD_FFT = 2,      /* fused FFT kernels (outputs up to 4096 a side), else cuFFT + glue kernels */
   XC_METHOD_TC_BF16X3 = 3, /* split-BF16 (3 products) tcgen05 tensor-core implicit GEMM, FP32 only */
   XC_METHOD_TC_TF32X3 = 4  /* the same with split-TF32 operands (kind::tf32): more accurate, half the rate */
 } xc_method;
 
 /* An algorithm: a method and one of its tile configurations.  Tiles: the
- * plain kernel 0 (its default: 8 partners per CTA when there are 4 or more,
- * else one), 1 (8 partners, 32 x 64 shifts; FP64: 4), 2 (one partner,
+ * plain kernel 0 (its default: the cyclic column-class form, or where rows
+ * are too wide for it the tiled form with 8 partners per CTA when there are 4
+ * or more, else one), 1 (tiled, 8 partners, 32 x 64 shifts; FP64: 4), 2 (one partner,
  * 64 x 64 shifts; FP64: 32 x 64), 3 (one partner, 32 x 64 shifts); the FFT
  * path 0; the split tensor-core paths 0 (items of at most 64 left rows) or
  * the item length cap, 4 to 1024.  The reference names algorithm and tile
@@ -131,8 +132,8 @@ xc_status xc_workspace_size(xc_mode mode, xc_dtype dtype, xc_method method, xc_s
  * `left`, `d_right` n_right of size `right`, `d_out` receives the outputs in
  * the mode's order, normalised (FFT results are quadrant-swapped and divided
  * by the transform size on the device).  The FFT method keeps a per-thread
- * cache of cuFFT plans: its first call for a shape creates (allocates) plans;
- * create them explicitly with xc_fft_plan_create to keep allocation out of
+ * cache of plans (twiddle tables, or cuFFT plans): its first call for a shape
+ * creates (allocates) them; create them explicitly with xc_fft_plan_create to keep allocation out of
  * timed or captured regions. */
 xc_status xc_correlate(xc_mode mode, xc_dtype dtype, xc_method method, const void* d_left, xc_size2 left,
                        uint32_t n_left, const void* d_right, xc_size2 right, uint32_t n_right, void* d_out,
@@ -266,17 +267,18 @@ xc_status xc_ragged_plan_create(xc_ragged_plan* plan, xc_dtype dtype, const void
 /* A plan's variants: a tile shape of the plain kernel and, for FP32 plans, a
  * route.  Variant index = tile_shape + (tile shapes) x route.  Route 0 keeps
  * every pair on the plain kernel; routes 1-4 run the pairs with at least
- * 2^32, 2^30, 2^28, 2^26 multiply-adds (that the split path takes) as
- * one_to_one calls of the split-BF16 tensor-core path, on eight side streams
- * captured into the same graph beside the plain kernel's launch (those
- * pairs' outputs then carry the split path's error, up to about 1e-5 of
- * max|out| on zero-mean data).  XC_RAGGED_TC=0 in the environment leaves FP32
+ * 2^32, 2^30, 2^28, 2^26 multiply-adds through the fused FFT kernels, a few
+ * launches for all of them, on side streams captured into the same graph
+ * beside the plain kernel's launch; a pair with an output beyond 4096 a side
+ * runs as a one_to_one call of the split-BF16 tensor-core path instead (its
+ * output then carries that path's error, up to about 1e-5 of max|out| on
+ * zero-mean data).  XC_RAGGED_TC=0 in the environment leaves FP32
  * plans with route 0 only.  Variant 0 runs until another is chosen. */
 typedef struct xc_ragged_variant {
   int32_t index;        /* the variant described */
   int32_t n_variants;   /* variants of this plan */
   int32_t tile_shape;   /* plain-kernel tile shape of the pairs left on the plain kernel */
-  uint32_t tc_pairs;    /* pairs run on the split-BF16 path */
+  uint32_t tc_pairs;    /* pairs that leave the plain kernel */
   uint64_t tc_min_macs; /* ... those with at least this many multiply-adds (0: none) */
 } xc_ragged_variant;
 /* Times every tile shape with route 0, then every route with the best shape,
@@ -287,7 +289,7 @@ typedef struct xc_ragged_variant {
 xc_status xc_ragged_autotune(xc_ragged_plan plan, void* stream, int* chosen_shape, double* best_ms);
 /* Describes variant `variant` (-1: the chosen one). */
 xc_status xc_ragged_describe(xc_ragged_plan plan, int variant, xc_ragged_variant* out);
-/* Chooses a variant (builds its graph now; allocates for the first split-path route). */
+/* Chooses a variant (builds its graph now; allocates for the first route). */
 xc_status xc_ragged_select(xc_ragged_plan plan, int variant);
 /* Replays the chosen variant's graph on `stream`. */
 xc_status xc_ragged_execute(xc_ragged_plan plan, void* stream);
