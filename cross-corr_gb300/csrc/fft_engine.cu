@@ -142,23 +142,21 @@ xc_status run(const Engine& e, const void* left, const void* right, void* out, c
     a.zeros = reinterpret_cast<const T*>(tw + e.zeros);
     return launch(e.rk.forward, ab + nr * a.b.groups, q * row_threads, q * row_smem, a, stream);
   };
-  const auto columns = [&](const Cx<T>* src, void* dst, int H, long long mats) {
-    ColFwdArgs<T> a{src, dst, H, nblk, mats * nblk, tw + e.tw_col};
+  // full spectra of the lefts and of `nr` rights
+  const auto columns = [&](long long nr) {
+    ColFwdArgs<T> a{{al, fl, g.Hl}, {ar, fr, g.Hr}, (long long)e.pm.n_left * nblk, (e.pm.n_left + nr) * nblk, tw + e.tw_col};
     const int pu = per_cta(a.units, e.ck.pu, unit_threads, e.sms);
     return launch(e.ck.form(div_up(a.units, e.ck.pu), e.sms).forward, div_up(a.units, pu), pu * unit_threads,
                   pu * unit_smem, a, stream);
   };
 
   if (e.shared) XC_TRY(rows(true, 0, e.n_right));
-  if (e.shared) {
-    XC_TRY(columns(al, fl, g.Hl, e.pm.n_left));
-    XC_TRY(columns(ar, fr, g.Hr, e.n_right));
-  }
+  if (e.shared) XC_TRY(columns(e.n_right));
   for (int k0 = 0; k0 < e.pm.K; k0 += e.k_chunk) {
     const int k1 = std::min(e.pm.K, k0 + e.k_chunk), nk = k1 - k0;
     if (!e.shared) {
       XC_TRY(rows(k0 == 0, k0 * e.pm.r_k, nk * e.pm.r_k));
-      if (e.lpre && k0 == 0) XC_TRY(columns(al, fl, g.Hl, e.pm.n_left));
+      if (e.lpre && k0 == 0) XC_TRY(columns(0));
     }
     for (int l0 = 0; l0 < e.pm.n_left; l0 += e.l_chunk) {
       const int nl = std::min(e.pm.n_left - l0, e.l_chunk);

@@ -572,11 +572,15 @@ struct ColArgs {
   int n_units;
 };
 template <typename T>
-struct ColFwdArgs {
+struct ColFwdSide {
   const Cx<T>* src;   // row spectra, H rows
   void* dst;          // full spectra: Cp<S> in pass order
-  int H, nblk;
-  long long units;    // matrices x nblk
+  int H;
+};
+template <typename T>
+struct ColFwdArgs {
+  ColFwdSide<T> a, b;       // units [0, a_units) are side a's, the rest side b's
+  long long a_units, units;  // matrices x blocks
   const void* tw;
 };
 template <typename T>
@@ -1067,11 +1071,14 @@ __global__ void __launch_bounds__(ColCfg<S, N>::threads, ColCfg<S, N>::ctas(1, D
   const int c = t % K::LC, j0 = t / K::LC;
   C* z = reinterpret_cast<C*>(smem_raw) + pu * K::unit + c;
   const long long u = (long long)blockIdx.x * (blockDim.x / K::TU) + pu;
-  const bool live = u < p.units;
+  const bool live = u < p.units, first = u < p.a_units;
+  const long long v = !live ? 0 : first ? u : u - p.a_units;
+  const ColFwdSide<typename Sc<S>::real> side = first ? p.a : p.b;
   pdl_wait();
-  col_load_passes<S, N, K::RQ>(z, p.src + (live ? u : 0) * spectrum_rows(p.H, K::RQ) * K::CB + c * (Sc<S>::NV * K::RQ), live ? p.H : 0, j0, tw);
+  col_load_passes<S, N, K::RQ>(z, side.src + v * spectrum_rows(side.H, K::RQ) * K::CB + c * (Sc<S>::NV * K::RQ),
+                                live ? side.H : 0, j0, tw);
   if (!live) return;
-  C* dst = static_cast<C*>(p.dst) + u * N * K::LC + c;
+  C* dst = static_cast<C*>(side.dst) + v * N * K::LC + c;
   for (int j = j0; j < L::TF; j += K::JT) {
     C x[L::R3];
     const C* base = z + col_item<S, N>(j);
