@@ -358,10 +358,14 @@ xc_status engine_plan(Engine* e, xc_dtype dtype, const Geometry& g, const PairMa
       }
       return false;
     };
-    // the preferred way in one chunk, the other in one, either in several
+    // The preferred way in one chunk, the other in one, either in several.
+    // Short launches that need several chunks (lengths rounded up by much)
+    // stay with the library transforms while they are small: n_to_m 4 + 16,
+    // 72x72 (1.6 million points) 23.9 us there, 32 in two chunks; 1 + 24, 16x16
+    // by 128x128 21.7 and 29.4; but 4 + 16, 100x100 (3.2 million) 42.8 and 34.8.
     const bool room = 2 * e->ck.unit_smem <= 227 * 1024;  // both blocks' in the column kernel
     bool placed = false;
-    for (int most : {1, pm.K})
+    for (int most : {1, brief && points < (2 << 20) ? 1 : pm.K})
       for (bool first : {lpre, !lpre}) placed = placed || ((first || room) && place(first, most));
     if (!placed) return XC_OK;
   }
