@@ -386,10 +386,10 @@ xc_status engine_plan(Engine* e, xc_dtype dtype, const Geometry& g, const PairMa
   fill_twiddles(e->nx, true, dtype, host.data());
   fill_twiddles(e->ny, false, dtype, host.data() + e->tw_col);
   XC_CUDA_TRY(cudaMalloc(&e->tw, host.size()));
-  const cudaError_t err = cudaMemcpy(e->tw, host.data(), host.size(), cudaMemcpyHostToDevice);
-  if (err != cudaSuccess) {
+  const xc_status st = upload(e->tw, host.data(), host.size());
+  if (st != XC_OK) {
     engine_release(e);
-    return from_cuda(err, "upload of the twiddle tables");
+    return st;
   }
   e->ready = true;
   return XC_OK;

@@ -202,8 +202,8 @@ xc_status shape_maps(RaggedPlanImpl* P, int shape, const RaggedShape& sh) {
   P->maps_for_shape[2 * shape] = dl;
   XC_CUDA_TRY(cudaMalloc(&dr, sizeof(CUtensorMap) * rm.size()));
   P->maps_for_shape[2 * shape + 1] = dr;
-  XC_CUDA_TRY(cudaMemcpy(dl, lm.data(), sizeof(CUtensorMap) * lm.size(), cudaMemcpyHostToDevice));
-  XC_CUDA_TRY(cudaMemcpy(dr, rm.data(), sizeof(CUtensorMap) * rm.size(), cudaMemcpyHostToDevice));
+  XC_TRY(upload(dl, lm.data(), sizeof(CUtensorMap) * lm.size()));
+  XC_TRY(upload(dr, rm.data(), sizeof(CUtensorMap) * rm.size()));
   return XC_OK;
 }
 
@@ -283,7 +283,7 @@ xc_status build_variant(RaggedPlanImpl* P, int index) {
   for (size_t i = 0; i < tiles.size(); ++i) ht[i] = tiles[i].second;
   if (P->dpairs == nullptr) {
     XC_CUDA_TRY(cudaMalloc(&P->dpairs, sizeof(RaggedPairDev) * hp.size()));
-    XC_CUDA_TRY(cudaMemcpy(P->dpairs, hp.data(), sizeof(RaggedPairDev) * hp.size(), cudaMemcpyHostToDevice));
+    XC_TRY(upload(P->dpairs, hp.data(), sizeof(RaggedPairDev) * hp.size()));
   }
   v.n_tiles = (int)ht.size();
   v.tc_pairs = (int)tc_pairs.size();
@@ -311,11 +311,11 @@ xc_status build_variant(RaggedPlanImpl* P, int index) {
     v.n_jobs = (int)jobs.size();
     v.repack_blocks = (int)blocks;
     XC_CUDA_TRY(cudaMalloc(&v.jobs, sizeof(CopyJob) * jobs.size()));
-    XC_CUDA_TRY(cudaMemcpy(v.jobs, jobs.data(), sizeof(CopyJob) * jobs.size(), cudaMemcpyHostToDevice));
+    XC_TRY(upload(v.jobs, jobs.data(), sizeof(CopyJob) * jobs.size()));
     XC_CUDA_TRY(cudaMalloc(&v.first, sizeof(int) * first.size()));
-    XC_CUDA_TRY(cudaMemcpy(v.first, first.data(), sizeof(int) * first.size(), cudaMemcpyHostToDevice));
+    XC_TRY(upload(v.first, first.data(), sizeof(int) * first.size()));
     XC_CUDA_TRY(cudaMalloc(&v.tiles, sizeof(RaggedTile) * ht.size()));
-    XC_CUDA_TRY(cudaMemcpy(v.tiles, ht.data(), sizeof(RaggedTile) * ht.size(), cudaMemcpyHostToDevice));
+    XC_TRY(upload(v.tiles, ht.data(), sizeof(RaggedTile) * ht.size()));
     XC_TRY(shape_maps(P, shape, sh));
     // persistent grid: every SM filled to the kernel's occupancy
     int dev = 0, sms = 0, per_sm = 0;

@@ -174,10 +174,10 @@ xc_status ragged_fft_build(RaggedFft* f, const std::vector<FftPair>& pairs, void
     put(ch.inv);
   }
   XC_CUDA_TRY(cudaMalloc(&f->tables, image.bytes.size()));
-  const cudaError_t err = cudaMemcpy(f->tables, image.bytes.data(), image.bytes.size(), cudaMemcpyHostToDevice);
-  if (err != cudaSuccess) {
+  const xc_status up = upload(f->tables, image.bytes.data(), image.bytes.size());
+  if (up != XC_OK) {
     ragged_fft_release(f);
-    return from_cuda(err, "upload of the ragged FFT tables");
+    return up;
   }
   const char* base = static_cast<const char*>(f->tables);
   for (Chunk& ch : chunks) {

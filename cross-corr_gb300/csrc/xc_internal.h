@@ -42,6 +42,10 @@ inline Geometry make_geometry(xc_size2 left, xc_size2 right) {
 
 xc_status debug_expire_wait(uint32_t polls, cudaStream_t stream);
 
+// Copies `bytes` from host memory to the device and waits for the copy, so that
+// a kernel on any stream launched afterwards finds it.
+xc_status upload(void* dst, const void* host, size_t bytes);
+
 // SMs of the device in use at the first call (152 without one).
 int sm_count_cached();
 

@@ -271,6 +271,16 @@ bool make_pair_map(xc_mode mode, uint32_t n_left, uint32_t n_right, PairMap* pm,
   return true;
 }
 
+// cudaMemcpy from pageable memory returns once the data is staged; the copy to
+// the device may still be on its way, and only the legacy default stream and
+// the streams that synchronise with it are ordered after it.  A plan's first
+// launches may be on a non-blocking stream.
+xc_status upload(void* dst, const void* host, size_t bytes) {
+  XC_CUDA_TRY(cudaMemcpy(dst, host, bytes, cudaMemcpyHostToDevice));
+  XC_CUDA_TRY(cudaStreamSynchronize(cudaStreamLegacy));
+  return XC_OK;
+}
+
 int sm_count_cached() {
   static const int n = [] {
     int dev = 0, sms = 0;
