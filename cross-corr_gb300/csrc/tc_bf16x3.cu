@@ -251,11 +251,17 @@ __device__ __forceinline__ void pdl_begin() {
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   asm volatile("griddepcontrol.wait;" ::: "memory");
 }
-// Loads of what an earlier kernel may have written.  Not __ldg: the compiler
-// may move a non-coherent load above the wait; volatile assembly stays below.
+// Loads of what an earlier kernel may have written.  Not __ldg, nor through
+// __restrict__ pointers: the compiler may move a non-coherent load above the
+// wait; volatile assembly stays below.
 __device__ __forceinline__ float ld_after(const float* g) {
   float v;
   asm volatile("ld.global.f32 %0, [%1];" : "=f"(v) : "l"(g));
+  return v;
+}
+__device__ __forceinline__ double ld_after(const double* g) {
+  double v;
+  asm volatile("ld.global.f64 %0, [%1];" : "=d"(v) : "l"(g));
   return v;
 }
 __device__ __forceinline__ float4 ld_after(const float4* g) {
@@ -1010,11 +1016,11 @@ struct PrepSide {
 // slice); FP64 partial sums of a slice, block-reduced, added into sums[m]
 // and sq[m] (zeroed before the launch).
 __device__ __forceinline__ void sum_block(const PrepSide& sd_, int b) {
-  const float* __restrict__ src = sd_.src;
+  const float* src = sd_.src;
   const long long area = sd_.area;
   const int slices = sd_.slices;
-  double* __restrict__ sums = sd_.sums;
-  double* __restrict__ sq = sd_.sq;
+  double* sums = sd_.sums;
+  double* sq = sd_.sq;
   __shared__ double red[8], red2[8];
   const int m = b / slices, sl = b % slices;
   const long long per = (area + slices - 1) / slices;
@@ -1081,11 +1087,11 @@ __global__ void __launch_bounds__(256) sum_kernel(const PrepSide a, const PrepSi
 struct MeanSd {
   float mu, sd;
 };
-__device__ __forceinline__ MeanSd mean_sd(const double* __restrict__ sums, const double* __restrict__ sq, int m,
-                                          int n_left, double left_area, double right_area) {
+__device__ __forceinline__ MeanSd mean_sd(const double* sums, const double* sq, int m, int n_left,
+                                          double left_area, double right_area) {
   const double area = m < n_left ? left_area : right_area;
-  const double mean = sums[m] / area;
-  return {(float)mean, (float)sqrt(fmax(0.0, sq[m] / area - mean * mean))};
+  const double mean = ld_after(sums + m) / area;
+  return {(float)mean, (float)sqrt(fmax(0.0, ld_after(sq + m) / area - mean * mean))};
 }
 
 // Accumulation windows: one warp per (left matrix, partner group), lanes
@@ -1129,9 +1135,10 @@ __device__ __forceinline__ void window_block(const WinArgs& wa, long long b) {
 // prefix sums C[y][x] = sum_{i<y} into S[y][x+1]; rowscan_kernel then scans
 // each row.  Centred, these sums are random walks of modest size, so FP32
 // holds them to ~1e-7; the summation is blocked (8-row segments, a carry per
-// 64-row chunk), which keeps every FP32 chain short.  One block per (matrix,
-// 32-column strip); each of its 8 warps loads 8 consecutive rows of a chunk
-// (coalesced, independent loads).
+// chunk of 8 NW rows), which keeps every FP32 chain short.  One block per
+// (matrix, 32-column strip); each of its NW warps (8, or 32 for matrices of
+// more than 256 rows) loads 8 consecutive rows of a chunk (coalesced,
+// independent loads).
 // Split planes of the centred right matrices fl32(R - mu_R), hi/lo with a
 // padded pitch: BF16 (T = __nv_bfloat16) or TF32-rounded FP32 (T = float).
 // Block b covers 1/bpm of matrix b / bpm (its mean computed once, from the
@@ -1143,7 +1150,7 @@ __device__ __forceinline__ void split_block(const PrepSide& sd_, int b, int bpm)
   constexpr int E = 16 / (int)sizeof(T);
   const int H = sd_.H, W = sd_.W, cpr = sd_.pitch / E;  // chunks per row
   const int m = b / bpm, part = b % bpm;
-  const float mv = (float)(sd_.sums[m] / (double)sd_.area);
+  const float mv = (float)(ld_after(sd_.sums + m) / (double)sd_.area);
   const long long per = (long long)H * cpr;
   const long long lo = per * part / bpm, hi = per * (part + 1) / bpm;
   const float* src = sd_.src + (long long)m * H * W;
@@ -1193,9 +1200,9 @@ __device__ __forceinline__ void split_block(const PrepSide& sd_, int b, int bpm)
 
 template <int NW>
 __device__ __forceinline__ void colsum_block(const PrepSide& sd_, int b) {
-  const float* __restrict__ src = sd_.src;
+  const float* src = sd_.src;
   const int H = sd_.H, W = sd_.W;
-  float* __restrict__ C = sd_.sat;
+  float* C = sd_.sat;
   __shared__ float seg[NW][32];
   __shared__ float carry[32];
   const int strips = (W + 31) / 32;
@@ -1207,7 +1214,7 @@ __device__ __forceinline__ void colsum_block(const PrepSide& sd_, int b) {
   float* c = C + (long long)m * (H + 1) * (W + 1) + 1;  // column x of C is column x + 1 of S
   // the mean as the statistics of every other kernel see it: FP64 sum over
   // the area, rounded once
-  const float mv = (float)(sd_.sums[m] / (double)sd_.area);
+  const float mv = (float)(ld_after(sd_.sums + m) / (double)sd_.area);
   if (b % strips == 0 && threadIdx.x == 0) sd_.mu[m] = mv;
   if (w == 0) {
     carry[lane] = 0.0f;
@@ -1284,7 +1291,7 @@ __global__ void __launch_bounds__(256) rowscan_kernel(const PrepSide a, const Pr
   pdl_begin();
   const bool first = blockIdx.x < a_blocks;
   const PrepSide& sd_ = first ? a : b;
-  float* __restrict__ S = sd_.sat;
+  float* S = sd_.sat;
   const long long n_rows = sd_.sat_rows;
   const int W = sd_.W;
   const int lane = threadIdx.x & 31;
@@ -1297,7 +1304,7 @@ __global__ void __launch_bounds__(256) rowscan_kernel(const PrepSide a, const Pr
     // eight 32-column chunks loaded together (the scan is latency-bound)
     float v[8];
 #pragma unroll
-    for (int u = 0; u < 8; ++u) v[u] = c0 + 32 * u + lane < W ? q[c0 + 32 * u + lane] : 0.0f;
+    for (int u = 0; u < 8; ++u) v[u] = c0 + 32 * u + lane < W ? ld_after(q + c0 + 32 * u + lane) : 0.0f;
 #pragma unroll
     for (int u = 0; u < 8; ++u) {
 #pragma unroll
