@@ -344,10 +344,10 @@ void host_forward(const float* P, const float* x, float* y) {
 }
 
 // The algorithm XC_METHOD_AUTO runs: the network's fastest prediction among
-// the supported candidates, else the tuning record; false when neither
-// exists.
+// the supported candidates (*predicted), else the tuning record; false when
+// neither exists.
 bool select_algorithm(xc_mode mode, xc_dtype dtype, xc_size2 left, uint32_t n_left, xc_size2 right,
-                      uint32_t n_right, xc_algo* algo) {
+                      uint32_t n_right, xc_algo* algo, bool* predicted = nullptr) {
   std::lock_guard<std::mutex> lock(g_sel_mutex);
   PairMap pm;
   uint64_t n_out = 1;
@@ -361,6 +361,7 @@ bool select_algorithm(xc_mode mode, xc_dtype dtype, xc_size2 left, uint32_t n_le
       if (method_supported(kAlgos[o].method, dtype, left, right) && (best < 0 || y[o] < y[best])) best = o;
     if (best >= 0) {
       *algo = kAlgos[best];
+      if (predicted != nullptr) *predicted = true;
       return true;
     }
   }
@@ -515,15 +516,17 @@ xc_status xc_correlate(xc_mode mode, xc_dtype dtype, xc_method method, const voi
   if (!make_pair_map(mode, n_left, n_right, &pm, &n_out))
     return fail(XC_ERR_INVALID_ARGUMENT, "invalid matrix counts for the mode");
   xc_algo a{method, 0};
-  if (method == XC_METHOD_AUTO && !select_algorithm(mode, dtype, left, n_left, right, n_right, &a)) {
+  bool predicted = false;
+  if (method == XC_METHOD_AUTO && !select_algorithm(mode, dtype, left, n_left, right, n_right, &a, &predicted)) {
     // no network and no record for this problem: the exhaustive autotune on
     // these buffers decides (and is remembered)
     double ms = 0.0;
     XC_TRY(xc_autotune_algorithm(mode, dtype, d_left, left, n_left, d_right, right, n_right, d_out, stream, &a, &ms));
   }
-  // the plain kernel's own choice of form is the faster one where the
-  // selector's timings (of its tiled forms) favour the plain kernel
-  if (method == XC_METHOD_AUTO && a.method == XC_METHOD_DIRECT) a.tile = 0;
+  // Where the network's predictions (of the tiled forms) favour the plain
+  // kernel, its default form runs: a prediction stands for the method.  A
+  // tuning record was measured on this problem and runs as measured.
+  if (predicted && a.method == XC_METHOD_DIRECT) a.tile = 0;
   if (a.method != XC_METHOD_DIRECT && a.method != XC_METHOD_FFT && a.method != XC_METHOD_TC_BF16X3 &&
       a.method != XC_METHOD_TC_TF32X3)
     return fail(XC_ERR_INVALID_ARGUMENT, "unknown method");

@@ -339,13 +339,15 @@ xc_status xc_selector_load_builtin(void);
  * 0-2 the plain kernel's tiles 1-3, 3 the FFT path, 4-5 split-BF16 with
  * items of at most 32 and 64 left rows, 6 split-TF32. */
 xc_status xc_algorithm(uint32_t index, xc_algo* algo);
-/* The algorithm XC_METHOD_AUTO runs for a problem: the network's fastest
- * prediction among the candidates that support it; without weights, the
- * candidate xc_autotune_algorithm last measured fastest for this problem;
- * with neither, {XC_METHOD_AUTO, 0}: xc_correlate's first call for the
- * problem then runs the exhaustive autotune on its own buffers (allocating
- * temporary workspaces and synchronising its stream) and remembers the
- * result. */
+/* The algorithm XC_METHOD_AUTO chooses for a problem: the network's fastest
+ * prediction among the candidates that support it (where that is one of the
+ * plain kernel's tiles, the call runs the plain kernel's default form, tile
+ * 0, which the network does not know); without weights, the candidate
+ * xc_autotune_algorithm last measured fastest for this problem, which then
+ * runs as measured; with neither, {XC_METHOD_AUTO, 0}: xc_correlate's first
+ * call for the problem then runs the exhaustive autotune on its own buffers
+ * (allocating temporary workspaces and synchronising its stream) and
+ * remembers the result. */
 xc_status xc_select_algorithm(xc_mode mode, xc_dtype dtype, xc_size2 left, uint32_t n_left, xc_size2 right,
                               uint32_t n_right, xc_algo* algo);
 /* The method of xc_select_algorithm's choice. */
