@@ -121,10 +121,11 @@ xc_status run(const Engine& e, const void* left, const void* right, void* out, c
   const int row_threads = e.rk.threads / e.rk.q, row_smem = e.rk.smem / e.rk.q;
   const int unit_threads = e.ck.threads / e.ck.pu, unit_smem = e.ck.unit_smem / e.ck.pu;
   const auto transforms = [&](long long mats, int H) { return mats * div_up(H, 2 * e.rk.nv); };
-  const Scales sc = spectrum_scales(e.nx, e.ny);
+  const Scales sc = spectrum_scales(e.nx, e.ny, sizeof(T) == 8);
 
   // rows of `nr` rights from the r0-th on, and (first) of all lefts.  FP64
-  // applies all of the result's scale here, in a product that is there anyway.
+  // applies all of the result's scale here, in a product that is there anyway:
+  // its range ends 900 binades further down than FP32's.
   const auto rows = [&](bool lefts, long long r0, long long nr) {
     const int q = per_cta((lefts ? transforms(e.pm.n_left, g.Hl) : 0) + transforms(nr, g.Hr), e.rk.q, row_threads, e.sms);
     const int rows_per_cta = 2 * e.rk.nv * q;
@@ -214,12 +215,15 @@ xc_status run(const Engine& e, const void* left, const void* right, void* out, c
 
 }  // namespace
 
-Scales spectrum_scales(int nx, int ny) {
+Scales spectrum_scales(int nx, int ny, bool early) {
   Scales s;
   int e = 0;
-  s.rest = 1.0 / std::frexp((double)nx * (double)ny, &e);  // nx ny = m 2^e, 1/2 <= m < 1
+  const double m = std::frexp((double)nx * (double)ny, &e);  // nx ny = m 2^e, 1/2 <= m < 1
+  const int end = early ? 0 : e / 2;
+  e -= end;
   s.left = std::ldexp(1.0, -(e / 2));
   s.right = std::ldexp(1.0, -(e - e / 2));
+  s.rest = std::ldexp(1.0 / m, -end);
   return s;
 }
 

@@ -34,13 +34,20 @@ struct Engine {
 };
 
 // 1 / (nx ny), the scale of an unnormalised pair of transforms, as powers of
-// two on the left and right spectra (half the exponent each, as a unitary
-// transform has, so that neither spectrum nor product leaves the type's range
-// before the result does) and a rest in (1, 2] at the end.
+// two on the left and right spectra and the rest at the end.  `early` puts all
+// of the power on the spectra, half each, as unitary transforms have it:
+// nothing leaves the type's range above before the result does (ragged
+// batches, whose pairs would else run on the split path, which has no scale).
+// Otherwise half of it stays for the end: the product of the spectra then lies
+// sqrt(nx ny) above its unitary size, so that what it loses below the smallest
+// normal number is below the result's own last place, as with transforms that
+// are scaled at the end.  (FP32, 256x256 by 256x256, both of 2^-66: error
+// 2.4e-5 of the result with all of the power on the spectra.)  Above, results
+// up to 2^127 / sqrt(nx ny) are finite, 2^127 / (nx ny) with all of it at the end.
 struct Scales {
   double left, right, rest;
 };
-Scales spectrum_scales(int nx, int ny);
+Scales spectrum_scales(int nx, int ny, bool early);
 // Smallest length >= n that the kernels have; 0 when n is beyond the largest.
 int length_for(int n);
 // Twiddle tables of a length's row or column passes: a complex value of the

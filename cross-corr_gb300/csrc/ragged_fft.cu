@@ -146,7 +146,7 @@ xc_status ragged_fft_build(RaggedFft* f, const std::vector<FftPair>& pairs, void
       Cx<T>* ar = reinterpret_cast<Cx<T>*>(ws + p.ar);
       Cx<T>* b = reinterpret_cast<Cx<T>*>(ws + p.b);
       ws += p.bytes;
-      const Scales sc = spectrum_scales(p.nx, p.ny);
+      const Scales sc = spectrum_scales(p.nx, p.ny, true);
       const int rows = 2 * p.rk.nv * p.rk.q;
       Group<RagRow<T>>& gf = ch.fwd[p.nx];
       for (int side = 0; side < 2; ++side) {
