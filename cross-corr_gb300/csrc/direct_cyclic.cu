@@ -39,7 +39,8 @@
 //    overlap another's products).  Results go through a small transpose
 //    buffer, so that each instruction covers 32 consecutive outputs.
 //  * The wider matrix of a pair takes the left's part: correlating the right
-//    with the left gives the same outputs, mirrored.
+//    with the left gives the same outputs, mirrored.  (But for rights of a few
+//    rows, see cyc_launch; a lane then wraps more than once.)
 //  * With one block of right rows the output is written; with several, it
 //    starts zeroed and each block adds (red.global.add).  The zeros are a
 //    kernel whose dependent launch this one is, so that its CTAs load their
@@ -50,6 +51,7 @@
 // loop of such bodies reaches 62 of the 75 TFLOP/s of independent FMAs) in
 // FP32, the FP64 pipe in FP64.
 #include <algorithm>
+#include <type_traits>
 
 #include "xc_common.cuh"
 #include "xc_internal.h"
@@ -482,20 +484,29 @@ double cyc_fill(const CycPlan& c, int C) {
 //   n_to_m 3x6, 201x183 by 75x59   4, 16: 167 (4 warps per CTA) and 196 (8); 4, 8: 173; 2, 8: 199
 //   one pair of 128x128        4, 8: 41; 2, 8: 29; 2, 4: 27; 2, 2: 29
 //   n_to_mn 8 + 32, 64x64 FP64   2, 16: 1281; 2, 8: 1199; 2, 4: 1027; 2, 2: 1021
+//   one pair of 1x300, FP32    1, 1: 10.8; 2, 2: 17.2 (the tiled kernel 10.7)
+//   n_to_m 4x8, 16x300 by 1x300 FP64   1, 1: 121; 2, 2: 312 (309)
+//   n_to_m 8x9, 314x403 by 1x1, FP32   1, 1: 60.6; 2, 2: 52.6
 // FP64 wants more warps (its pipe is the bound, and an uneven share of the SMs
-// shows), FP32 chains stay within 4096 products as in the tiled kernel.
+// shows), FP32 chains stay within 4096 products as in the tiled kernel.  Rights
+// of one row take 1 shift and 1 row, which multiplies nothing else; in FP32 with
+// a single column block of a wider left, where outputs and not products cost,
+// only launches that 2 shifts do not fill.
 template <typename T>
 bool cyc_plan(const Geometry& g, long long pairs, CycPlan* best) {
   constexpr bool f32 = sizeof(T) == 4;
+  constexpr int TSX = 32 / (int)sizeof(T);
   struct Shape {
     int tsy, hb;
   };
-  constexpr Shape shapes[] = {{4, 16}, {4, 8}, {2, 8}, {2, 4}, {2, 2}};
+  constexpr Shape shapes[] = {{4, 16}, {4, 8}, {2, 8}, {2, 4}, {2, 2}, {1, 1}};
   const int chain = f32 ? 4096 / g.Wr : 1 << 30;
+  if (chain < 2) return false;  // rows too wide for a chain of two
   const long long enough = (f32 ? 6LL : 32LL) * sm_count_cached();
   bool found = false;
   for (const Shape& sh : shapes) {
     if (sh.hb > chain || (!f32 && sh.tsy == 4) || (sh.hb > 2 && sh.hb / 2 >= g.Hr)) continue;
+    if (g.Hr > 1 ? sh.hb == 1 : sh.hb == 2 && (!f32 || g.Wr > TSX || g.Wl <= TSX)) continue;
     CycPlan c;
     // CTAs of eight warps share more of their left rows; four-warp ones spread
     // a short launch more evenly.  The form that fills more warp slots.
@@ -524,8 +535,18 @@ xc_status cyc_launch(const T* left, const T* right, T* out, Geometry g, const Pa
   constexpr int TSX = 32 / (int)sizeof(T);
   // A left narrower than the right changes places with it: few classes wrap
   // often, and every wrap costs a surplus block and a hand-over (16x16 by
-  // 128x128 27.6 us, 8.1 with places changed; x 24 43.0 and 16.4).
-  const bool flip = g.Wl < g.Wr;
+  // 128x128 27.6 us, 8.1 with places changed; x 24 43.0 and 16.4).  Not where
+  // the right has one to three rows and the left many: in the left's part those
+  // few rows meet a few right rows each, most of a block's products are of
+  // zeros.  There the wraps cost less once the lanes (a left row's classes, over
+  // all pairs) fill the GPU: 1000x1 by 1x8 x 64 50.4 us, 6.6 in its place; 300x4 by
+  // 2x40 x 64 21.3 and 16.9; 238x160 by 1x227, 105 pairs, 352 and 152; but one
+  // pair of 300x1 by 1x40 5.2 and 8.2, 20x60 by 1x300 x 64 17.8 and 24.9.
+  const int C = div_up(g.Wl, TSX);
+  const long long lanes = (long long)pm.n_left * pm.K * g.Hl * C;
+  const bool columns = g.Hl > g.Hr && ((g.Hr == 1 && C == 1 && g.Wr <= 8) ||
+                                       (g.Hr <= 3 && g.Hl >= 64 && lanes >= (g.Hr == 1 && C == 1 ? 9000 : 16000)));
+  const bool flip = g.Wl < g.Wr && !columns;
   if (flip) {
     std::swap(g.Hl, g.Hr);
     std::swap(g.Wl, g.Wr);
@@ -545,7 +566,7 @@ xc_status cyc_launch(const T* left, const T* right, T* out, Geometry g, const Pa
   a.Sy = g.Sy;
   a.Sx = g.Sx;
   a.pm = pm;
-  a.C = div_up(g.Wl, TSX);
+  a.C = flip ? div_up(g.Wl, TSX) : C;
   a.NB = div_up(g.Wr, TSX);
   a.hb = c.hb;
   a.n_rb = c.n_rb;
@@ -565,11 +586,17 @@ xc_status cyc_launch(const T* left, const T* right, T* out, Geometry g, const Pa
     zero_kernel<T><<<(unsigned)std::min<long long>(8LL * sm_count_cached(), want), 256, 0, stream>>>(out, n);
     XC_CUDA_TRY(cudaGetLastError());
   }
-  const auto pick = [&](auto plain, auto mirrored) { return flip ? mirrored : plain; };
-  auto kern = c.win ? (c.tsy == 4 ? pick(cyclic_kernel<T, 4, true, false>, cyclic_kernel<T, 4, true, true>)
-                                  : pick(cyclic_kernel<T, 2, true, false>, cyclic_kernel<T, 2, true, true>))
-                    : (c.tsy == 4 ? pick(cyclic_kernel<T, 4, false, false>, cyclic_kernel<T, 4, false, true>)
-                                  : pick(cyclic_kernel<T, 2, false, false>, cyclic_kernel<T, 2, false, true>));
+  const auto pick = [&](auto tsy) -> void (*)(const CycArgs<T>) {
+    constexpr int Y = decltype(tsy)::value;
+    if (c.win) return flip ? cyclic_kernel<T, Y, true, true> : cyclic_kernel<T, Y, true, false>;
+    return flip ? cyclic_kernel<T, Y, false, true> : cyclic_kernel<T, Y, false, false>;
+  };
+  void (*kern)(const CycArgs<T>) = nullptr;
+  if constexpr (sizeof(T) == 4) {
+    if (c.tsy == 4) kern = pick(std::integral_constant<int, 4>());
+  }
+  if (c.tsy == 2) kern = pick(std::integral_constant<int, 2>());
+  if (c.tsy == 1) kern = pick(std::integral_constant<int, 1>());
   XC_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024));
   const int slot = kernel_timer_begin(stream);
   cudaLaunchAttribute attr{};

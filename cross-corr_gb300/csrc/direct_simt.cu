@@ -648,11 +648,16 @@ RaggedShape shape_of() {
 xc_status direct_launch(xc_dtype dtype, const void* left, const void* right, void* out, const Geometry& g,
                         const PairMap& pm, cudaStream_t stream, int force_loader, DirectAccumulate acc, int tile) {
   // tile 0: cyclic column classes (direct_cyclic.cu), faster than every tile
-  // of this file from 16x16 to 1024x1024 lefts and 8x8 to 512x512 rights, thin
-  // matrices most (FP32 1.03-43 times the default tile, FP64 1.04-6.8); rows
-  // too wide for it take 8 partners per CTA when there are 4 or more (3 for
-  // FP64), else one.  1: 8 (FP64: 4) partners, 32 x 64 shifts; 2: one partner, 64 x 64
-  // shifts (FP64: 32 x 64); 3: one partner, 32 x 64 shifts
+  // of this file from 16x16 to 1024x1024 lefts and 8x8 to 512x512 rights (FP32
+  // 1.03-43 times the default tile, FP64 1.04-6.8).  Of 5500 thin problems (one
+  // matrix of 1 to 8 rows, mostly) 32 are slower by over 4%, the geometric mean
+  // is 4.7 times faster.  The 32 are mostly rights of 1 to 3 rows, up to 1.4
+  // times slower (FP64 one_to_many 16x300 by 3x3 x 64 30.6 us, 25.8 tiled; one
+  // FP32 pair of 1x1000 by 2x40 6.9 and 5.8), and stay with it: the tiles spread
+  // a non-finite value to shifts that do not meet it.  Rows too wide for it
+  // take 8 partners per CTA when there are 4 or more (3 for FP64), else one.
+  // 1: 8 (FP64: 4) partners, 32 x 64 shifts; 2: one partner, 64 x 64 shifts
+  // (FP64: 32 x 64); 3: one partner, 32 x 64 shifts
   if (tile < 0 || tile > 3) return fail(XC_ERR_INVALID_ARGUMENT, "plain kernel tiles are 0-3");
   if (tile == 0 && force_loader < 0 && acc != DirectAccumulate::kNever) {
     bool taken = false;
