@@ -811,6 +811,12 @@ xc_status xc_fft_plan_pad_size(xc_fft_plan plan, xc_size2* pad) {
   return XC_OK;
 }
 
+xc_status xc_fft_plan_describe(xc_fft_plan plan, xc_fft_form* form) {
+  if (plan == nullptr || form == nullptr) return fail(XC_ERR_INVALID_ARGUMENT, "NULL argument");
+  fft_plan_describe(plan->impl, form);
+  return XC_OK;
+}
+
 xc_status xc_fft_execute(xc_fft_plan plan, const void* d_left, const void* d_right, void* d_out, int normalize,
                          void* d_workspace, size_t workspace_bytes, void* stream) {
   if (plan == nullptr || d_left == nullptr || d_right == nullptr || d_out == nullptr)

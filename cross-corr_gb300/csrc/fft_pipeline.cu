@@ -138,6 +138,20 @@ size_t fft_plan_workspace(const FftPlanImpl* p) { return p->ws_inputs + p->ws_pr
 
 xc_size2 fft_plan_pad(const FftPlanImpl* p) { return xc_size2{(uint32_t)p->px, (uint32_t)p->py}; }
 
+void fft_plan_describe(const FftPlanImpl* p, xc_fft_form* form) {
+  *form = xc_fft_form{};
+  const fe::Engine& e = p->engine;
+  if (!e.ready) return;
+  form->fused = 1;
+  form->size_y = e.ny;
+  form->size_x = e.nx;
+  form->spectra = e.shared ? 2 : e.lpre ? 1 : 0;
+  form->lefts = e.l_chunk;
+  form->partners = e.k_chunk;
+  form->group = e.kc;
+  form->units = e.l_chunk * div_up(e.k_chunk, e.kc) * e.nblk;
+}
+
 namespace {
 struct WsView {
   char* inputs;

@@ -132,6 +132,7 @@ xc_status fft_plan_create(FftPlanImpl** plan, xc_mode mode, xc_dtype dtype, xc_s
                           xc_size2 right, uint32_t n_right, xc_size2 pad, bool stages);
 size_t fft_plan_workspace(const FftPlanImpl* plan);
 xc_size2 fft_plan_pad(const FftPlanImpl* plan);
+void fft_plan_describe(const FftPlanImpl* plan, xc_fft_form* form);
 xc_status fft_plan_execute(FftPlanImpl* plan, const void* left, const void* right, void* out, int normalize,
                            void* workspace, size_t ws_bytes, cudaStream_t stream);
 xc_status fft_plan_forward(FftPlanImpl* plan, const void* left, const void* right, void* workspace, size_t ws_bytes,

@@ -35,7 +35,8 @@ EXPORTED = [
     "xc_debug_expire_wait", "xc_kernel_timing", "xc_kernel_timing_read", "xc_output_count", "xc_output_size",
     "xc_workspace_size", "xc_correlate", "xc_correlate_host", "xc_correlate_host_async", "xc_host_wait",
     "xc_release_thread_cache", "xc_correlate_tc_noalloc",
-    "xc_fft_plan_create", "xc_fft_plan_workspace_size", "xc_fft_plan_pad_size", "xc_fft_execute",
+    "xc_fft_plan_create", "xc_fft_plan_workspace_size", "xc_fft_plan_pad_size",
+    "xc_fft_plan_describe", "xc_fft_execute",
     "xc_fft_forward", "xc_fft_multiply", "xc_fft_inverse", "xc_fft_plan_destroy",
     "xc_run_ccn_shuffle_f32", "xc_run_ccn_shuffle_f64",
     "xc_run_ccn_shuffle_multimat_right_f32", "xc_run_ccn_shuffle_multimat_right_f64",
@@ -93,6 +94,11 @@ class PairDesc(ctypes.Structure):
     _fields_ = [("left", ctypes.c_uint32), ("right", ctypes.c_uint32), ("out_offset", ctypes.c_uint64)]
 
 
+class FftForm(ctypes.Structure):
+    _fields_ = [(f, ctypes.c_int32) for f in ("fused", "size_y", "size_x", "spectra", "lefts", "partners", "group",
+                                              "units")]
+
+
 class RaggedVariant(ctypes.Structure):
     _fields_ = [("index", ctypes.c_int32), ("n_variants", ctypes.c_int32), ("tile_shape", ctypes.c_int32),
                 ("tc_pairs", ctypes.c_uint32), ("tc_min_macs", ctypes.c_uint64)]
@@ -136,6 +142,7 @@ def lib():
         L.xc_fft_plan_create.argtypes = [c.POINTER(vp), i, i, Size2, u32, Size2, u32, Size2]
         L.xc_fft_plan_workspace_size.argtypes = [vp, c.POINTER(sz)]
         L.xc_fft_plan_pad_size.argtypes = [vp, c.POINTER(Size2)]
+        L.xc_fft_plan_describe.argtypes = [vp, c.POINTER(FftForm)]
         L.xc_fft_execute.argtypes = [vp, vp, vp, vp, i, vp, sz, vp]
         L.xc_fft_forward.argtypes = [vp, vp, vp, vp, sz, vp]
         L.xc_fft_multiply.argtypes = [vp, vp, sz, vp]
@@ -329,7 +336,7 @@ class kernel_timing:
 
 
 class FftPlan:
-    """Explicit FFT plan (xc_fft_plan_create); owns its cuFFT plans."""
+    """Explicit FFT plan (xc_fft_plan_create); owns its tables and cuFFT plans."""
 
     def __init__(self, mode, dtype, left_shape, n_left, right_shape, n_right, pad=(0, 0)):
         self.handle = ctypes.c_void_p()
@@ -341,6 +348,12 @@ class FftPlan:
         p = Size2()
         check(lib().xc_fft_plan_pad_size(self.handle, ctypes.byref(p)))
         self.pad = (int(p.y), int(p.x))
+
+    def describe(self):
+        """How normalised execution runs (xc_fft_plan_describe), as a dict."""
+        f = FftForm()
+        check(lib().xc_fft_plan_describe(self.handle, ctypes.byref(f)))
+        return {name: getattr(f, name) for name, _ in FftForm._fields_}
 
     def execute(self, left, right, out, workspace, normalize=True, stream=None):
         check(lib().xc_fft_execute(self.handle, left.data_ptr(), right.data_ptr(), out.data_ptr(), int(normalize),

@@ -221,12 +221,27 @@ xc_status xc_correlate_tc_noalloc(xc_mode mode, const float* d_left, xc_size2 le
 /* src/n_to_m.hpp:700-745, src/fft_helpers.hpp:193-261).                    */
 /* ------------------------------------------------------------------------ */
 typedef struct xc_fft_plan_s* xc_fft_plan;
-/* `pad` = transform size; {0,0} selects the reference's 2H x 2W for equal
- * sizes and the smallest 2^a3^b5^c7^d size >= H+Hr-1 otherwise. */
+/* `pad` = size of the library transforms, which the separate stages and
+ * normalize == 0 run, and of their workspace; {0,0} selects the reference's
+ * 2H x 2W for equal sizes and the smallest 2^a3^b5^c7^d size >= H+Hr-1
+ * otherwise.  Normalised execution by the fused kernels has lengths of its own
+ * (xc_fft_plan_describe). */
 xc_status xc_fft_plan_create(xc_fft_plan* plan, xc_mode mode, xc_dtype dtype, xc_size2 left, uint32_t n_left,
                              xc_size2 right, uint32_t n_right, xc_size2 pad);
 xc_status xc_fft_plan_workspace_size(xc_fft_plan plan, size_t* bytes);
 xc_status xc_fft_plan_pad_size(xc_fft_plan plan, xc_size2* pad);
+/* How a plan's normalised execution runs. */
+typedef struct xc_fft_form {
+  int32_t fused;      /* 1: the fused kernels; 0: the library transforms, and zeros below */
+  int32_t size_y;     /* the fused kernels' transform lengths */
+  int32_t size_x;
+  int32_t spectra;    /* made before the products: 0 none, 1 the lefts', 2 both sides' */
+  int32_t lefts;      /* left matrices and partners of each per product launch */
+  int32_t partners;
+  int32_t group;      /* partners of a left that one block column's threads take in turn */
+  int32_t units;      /* such groups x block columns in a product launch */
+} xc_fft_form;
+xc_status xc_fft_plan_describe(xc_fft_plan plan, xc_fft_form* form);
 /* normalize != 0: normalised (Hl+Hr-1)x(Wl+Wr-1) outputs.  normalize == 0:
  * the raw, unnormalised pad.y x pad.x circular correlations the reference's
  * fft_* algorithms store without -n (src/fft_alg.hpp:13-20). */
