@@ -357,7 +357,15 @@ xc_status engine_plan(Engine* e, xc_dtype dtype, const Geometry& g, const PairMa
         if (off > ws_bytes) continue;
         e->lpre = first;
         e->k_chunk = k;
-        e->kc = first || brief ? 1 : k;
+        // Without left spectra made first a unit transforms its left block once
+        // for a group of partners: all of them where the units nearly fill a
+        // wave of CTAs (0.8 of it), else as many as leave two waves.  One group
+        // of all partners left the SMs idle: one_to_many 232x26 x 98, 9 units,
+        // 509 us, 25 one by one (library transforms 71); FP64 75x319 by 263x9 x
+        // 68, 97 units, 5978 us, 1123 in groups of five (2182).
+        const long long units = (long long)pm.n_left * e->nblk, wave = (long long)e->sms * (512 / e->ck.threads) * e->ck.pu;
+        const bool filled = 10 * units >= 8 * wave;
+        e->kc = first || brief ? 1 : filled ? k : (int)std::max<long long>(1, std::min<long long>(k, k * units / (2 * wave)));
         return true;
       }
       return false;

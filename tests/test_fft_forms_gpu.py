@@ -104,3 +104,18 @@ def test_fp32_lengths(length, columns):
 def test_chunks(dtype, mode, n, m, ls, rs, spectra, lefts, partners):
     form = check(mode, n, m, ls, rs, dtype)
     assert (form["spectra"], form["lefts"], form["partners"]) == (spectra, lefts, partners)
+
+
+@pytest.mark.parametrize("dtype,mode,n,m,ls,rs", [
+    ("f32", "one_to_many", 1, 98, (232, 26), (232, 26)), ("f32", "one_to_many", 1, 20, (9, 235), (335, 21)),
+    ("f64", "one_to_many", 1, 10, (13, 396), (377, 22)), ("f64", "n_to_mn", 5, 30, (13, 22), (433, 72)),
+    ("f32", "n_to_mn", 6, 12, (212, 212), (212, 212)), ("f32", "one_to_many", 1, 3000, (9, 9), (8, 8)),
+])
+def test_groups_of_partners_fill_the_gpu(dtype, mode, n, m, ls, rs):
+    """Where no spectra are made first (here: no room for them), a group of
+    partners shares a left block's transform: no longer groups than leave one
+    unit, of at most 128 threads, to every two SMs."""
+    form = check(mode, n, m, ls, rs, dtype)
+    assert form["spectra"] == 0
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    assert form["group"] == 1 or form["units"] >= sms // 2
