@@ -46,6 +46,11 @@
 //    kernel whose dependent launch this one is, so that its CTAs load their
 //    rows meanwhile (one pair of 128x128: 24.6 us, 28.5 after a memset).  hb
 //    bounds an FP32 chain to 4096 products, as the tiled kernel's flushes do.
+//    The order in which blocks add is not fixed, so results of more than two
+//    blocks differ between runs in their last places.  CTAs that walk over all
+//    blocks of their tiles instead, in order, repeat bit for bit, but their
+//    loads differ by what their tiles meet: one_to_many 256x256 x 64 10.3 ms
+//    against 9.9, x 16 3.0 against 2.6, 300x300 by 40x40 x 64 588 us against 499.
 //
 // What bounds it: instruction issue (83% of the slots, FMA pipe 76%; a bare
 // loop of such bodies reaches 62 of the 75 TFLOP/s of independent FMAs) in
@@ -201,6 +206,10 @@ __device__ __forceinline__ void stage_rows(char* dst, int pitch, const T* __rest
 // dy, column x + dx.  For outputs whose sum came out as NaN: the zero columns
 // and rows around the matrices make NaN of an infinity, and of a NaN, that the
 // shift does not meet.  A sum that is NaN stays one, so the loop ends there.
+// One lane walks one output's overlap, at many times a product's cost in the
+// kernel's body: one NaN in the left of one_to_many 256x256 x 64 makes 9.8 ms
+// 18.5, one value of a hundred 25.1 (the tiled kernel, which spreads it, 14.0);
+// one infinity costs nothing (9.7: only sums that are NaN are made again).
 template <typename T>
 __device__ __forceinline__ T overlap_sum(const T* __restrict__ L, const T* __restrict__ R, int Hl, int Wl, int rows,
                                          int Wr, int dy, int dx) {

@@ -30,7 +30,8 @@
 // spectra's loads 14%, the stores 12%, the twiddles' loads 10%, the rows' 1%
 // (each left out in turn, before the twiddles were halved and half of the left
 // spectra loaded ahead).
-// FP64 is bound by its pipe (85% busy; 1.0 TFLOP/s measured).
+// FP64 is bound by its pipe (82 to 84% busy in col_pairs and row_inverse, 69 to
+// 77% in the forward kernels, whose launches are short; 1.0 TFLOP/s measured).
 #pragma once
 
 #include <cstdint>

@@ -621,9 +621,10 @@ __global__ void __launch_bounds__(kThreads, 1)
     // [256 h, 256 h + 256)) and commits to the shared consumed barriers.
     // With at most 256 shifts (RS) one MMA covers what the two halves
     // took two for: issuer h then issues the MMAs of every other left row
-    // over all shifts, which halves their number (each costs an issuer about
-    // 79 cycles however narrow: n_to_m 8 x 32 of 64x64, kernel 103 us with
-    // halves, 92 with rows).
+    // over all shifts, which halves their number (n_to_m 8 x 32 of 64x64,
+    // kernel 103 us with halves, 92 with rows; at about 79 cycles each the
+    // remaining MMAs are 13 of these, the rest is each row's chain of barriers,
+    // builds, stages and drains).
     const int h = warp == 1 ? 0 : 1;
     uint32_t* ktab = ktab_all + h * (kMaxKSteps + 1);
     {

@@ -67,7 +67,13 @@ typedef enum xc_method {
  * or more, else one), 1 (tiled, 8 partners, 32 x 64 shifts; FP64: 4), 2 (one partner,
  * 64 x 64 shifts; FP64: 32 x 64), 3 (one partner, 32 x 64 shifts); the FFT
  * path 0; the split tensor-core paths 0 (items of at most 64 left rows) or
- * the item length cap, 4 to 1024.  The reference names algorithm and tile
+ * the item length cap, 4 to 1024.  Repeatability: the plain kernel's default
+ * form adds blocks of 2 to 16 right rows into an output in no fixed order, so
+ * two runs may differ in their last places where the right (of the pair, the
+ * narrower matrix) has more than two blocks; tiles 1-3 repeat bit for bit
+ * where their tiles fill a wave of CTAs and add slices of rows where not; the
+ * split paths add row chunks in no fixed order; the FFT path repeats.  The
+ * reference names algorithm and tile
  * arguments by hand (src/main.cpp:361-411, the JSON tile arguments of each
  * plug-in). */
 typedef struct xc_algo {
