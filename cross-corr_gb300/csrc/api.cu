@@ -394,7 +394,7 @@ xc_status run_algo(xc_mode mode, xc_dtype dtype, xc_algo a, const void* d_left, 
   const Geometry g = make_geometry(left, right);
   switch (a.method) {
     case XC_METHOD_DIRECT:
-      return direct_launch(dtype, d_left, d_right, d_out, g, pm, stream, -1, DirectAccumulate::kAuto, a.tile);
+      return direct_launch(dtype, d_left, d_right, d_out, g, pm, stream, DirectAccumulate::kAuto, a.tile);
     case XC_METHOD_FFT: {
       FftPlanImpl* plan = nullptr;
       XC_TRY(cached_plan(mode, dtype, left, n_left, right, n_right, &plan));
@@ -1114,7 +1114,7 @@ xc_status run_mode(xc_mode mode, const T* left, const T* right, T* out, xc_size2
   if (!make_pair_map(mode, nl, nr, &pm, &n_out)) return fail(XC_ERR_INVALID_ARGUMENT, "invalid matrix counts");
   if (left == nullptr || right == nullptr || out == nullptr) return fail(XC_ERR_INVALID_ARGUMENT, "NULL pointer");
   return direct_launch(sizeof(T) == 4 ? XC_F32 : XC_F64, left, right, out, make_geometry(ms, ms), pm,
-                       as_stream(stream), -1, acc);
+                       as_stream(stream), acc);
 }
 
 }  // namespace

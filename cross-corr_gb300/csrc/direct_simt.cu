@@ -524,8 +524,7 @@ int pick_slice_rows(const Geometry& g, long long blocks, int tiles_sy, long long
 
 template <typename C>
 xc_status launch_uniform(const typename C::type* left, const typename C::type* right, typename C::type* out,
-                         const Geometry& g, const PairMap& pm, cudaStream_t stream, int force_loader,
-                         DirectAccumulate acc_mode) {
+                         const Geometry& g, const PairMap& pm, cudaStream_t stream, DirectAccumulate acc_mode) {
   using T = typename C::type;
   DirectArgs<T> p;
   std::memset(&p, 0, sizeof(p));
@@ -553,10 +552,8 @@ xc_status launch_uniform(const typename C::type* left, const typename C::type* r
   int per_sm = 0;
   XC_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, C::SMEM_BYTES));
   XC_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, C::NT, C::SMEM_BYTES));
-  const int slice_rows = acc_mode == DirectAccumulate::kNever
-                             ? 0
-                             : pick_slice_rows<C>(g, tiles, u.tiles_sy, (long long)u.tiles_sx * pm.n_left * u.kgroups,
-                                                  std::max(1, per_sm) * sm_count_cached());
+  const int slice_rows = pick_slice_rows<C>(g, tiles, u.tiles_sy, (long long)u.tiles_sx * pm.n_left * u.kgroups,
+                                            std::max(1, per_sm) * sm_count_cached());
   u.n_slices = 1;
   u.rows_per_slice = 1 << 30;
   if (slice_rows > 0) {
@@ -577,10 +574,8 @@ xc_status launch_uniform(const typename C::type* left, const typename C::type* r
 
   // TMA needs 16-byte aligned bases and row/matrix pitches.
   const size_t es = sizeof(T);
-  const bool tma_ok = ((uintptr_t)left % 16 == 0) && ((uintptr_t)right % 16 == 0) && ((size_t)g.Wl * es % 16 == 0) &&
-                      ((size_t)g.Wr * es % 16 == 0);
-  const bool use_tma = force_loader < 0 ? tma_ok : (force_loader == 1);
-  if (use_tma && !tma_ok) return fail(XC_ERR_INVALID_ARGUMENT, "TMA loader requested for unaligned pitches");
+  const bool use_tma = ((uintptr_t)left % 16 == 0) && ((uintptr_t)right % 16 == 0) && ((size_t)g.Wl * es % 16 == 0) &&
+                       ((size_t)g.Wr * es % 16 == 0);
 
   CUtensorMap lmap, rmap;
   std::memset(&lmap, 0, sizeof(lmap));
@@ -646,7 +641,7 @@ RaggedShape shape_of() {
 }  // namespace
 
 xc_status direct_launch(xc_dtype dtype, const void* left, const void* right, void* out, const Geometry& g,
-                        const PairMap& pm, cudaStream_t stream, int force_loader, DirectAccumulate acc, int tile) {
+                        const PairMap& pm, cudaStream_t stream, DirectAccumulate acc, int tile) {
   // tile 0: cyclic column classes (direct_cyclic.cu), faster than every tile
   // of this file from 16x16 to 1024x1024 lefts and 8x8 to 512x512 rights (FP32
   // 1.03-43 times the default tile, FP64 1.04-6.8).  Of 5500 thin problems (one
@@ -659,7 +654,7 @@ xc_status direct_launch(xc_dtype dtype, const void* left, const void* right, voi
   // 1: 8 (FP64: 4) partners, 32 x 64 shifts; 2: one partner, 64 x 64 shifts
   // (FP64: 32 x 64); 3: one partner, 32 x 64 shifts
   if (tile < 0 || tile > 3) return fail(XC_ERR_INVALID_ARGUMENT, "plain kernel tiles are 0-3");
-  if (tile == 0 && force_loader < 0 && acc != DirectAccumulate::kNever) {
+  if (tile == 0) {
     bool taken = false;
     XC_TRY(direct_cyclic(dtype, left, right, out, g, pm, stream, acc == DirectAccumulate::kCaller, &taken));
     if (taken) return XC_OK;
@@ -669,16 +664,16 @@ xc_status direct_launch(xc_dtype dtype, const void* left, const void* right, voi
     const float* l = (const float*)left;
     const float* r = (const float*)right;
     float* o = (float*)out;
-    if (t == 1) return launch_uniform<CfgF32Multi>(l, r, o, g, pm, stream, force_loader, acc);
-    if (t == 2) return launch_uniform<CfgF32Single>(l, r, o, g, pm, stream, force_loader, acc);
-    return launch_uniform<CfgF32Small>(l, r, o, g, pm, stream, force_loader, acc);
+    if (t == 1) return launch_uniform<CfgF32Multi>(l, r, o, g, pm, stream, acc);
+    if (t == 2) return launch_uniform<CfgF32Single>(l, r, o, g, pm, stream, acc);
+    return launch_uniform<CfgF32Small>(l, r, o, g, pm, stream, acc);
   }
   const int t = tile != 0 ? tile : (pm.K >= 3 ? 1 : 2);
   const double* l = (const double*)left;
   const double* r = (const double*)right;
   double* o = (double*)out;
-  if (t == 1) return launch_uniform<CfgF64Multi>(l, r, o, g, pm, stream, force_loader, acc);
-  return launch_uniform<CfgF64Single>(l, r, o, g, pm, stream, force_loader, acc);
+  if (t == 1) return launch_uniform<CfgF64Multi>(l, r, o, g, pm, stream, acc);
+  return launch_uniform<CfgF64Single>(l, r, o, g, pm, stream, acc);
 }
 
 // Tile shapes a ragged plan may pick from (the autotuner's candidates).

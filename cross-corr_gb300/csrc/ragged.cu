@@ -681,7 +681,7 @@ xc_status correlate_pairs(xc_dtype dtype, const void* d_left, const xc_matrix_de
     const xc_matrix_desc& R = rights[pd.right];
     const Geometry g = make_geometry(xc_size2{L.cols, L.rows}, xc_size2{R.cols, R.rows});
     XC_TRY(direct_launch(dtype, (const char*)d_left + L.offset * es, (const char*)d_right + R.offset * es,
-                         (char*)d_out + pd.out_offset * es, g, pm, stream, -1));
+                         (char*)d_out + pd.out_offset * es, g, pm, stream));
   }
   return XC_OK;
 }

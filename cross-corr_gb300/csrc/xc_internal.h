@@ -59,15 +59,15 @@ xc_status kernel_timing_read(double* total_ms, uint32_t* launches);
 
 // Plain definition-based correlation (direct_simt.cu).  How results reach
 // the output:
-//  kAuto   - the output is written; under-filled launches split each tile's
-//            rows over several CTAs, which zero the output first and add;
+//  kAuto   - the output is written; where several CTAs share an output (blocks
+//            of right rows of the cyclic form, slices of a tile's rows in
+//            under-filled launches of the tiled one) it is zeroed first and they add;
 //  kCaller - always added into the output, which the caller zeroed (the
 //            reference's work-distribution launchers, src/one_to_one.hpp:276-277);
-//  kNever  - written, never split (studies and tests of the unsplit kernel).
-enum class DirectAccumulate { kAuto = 0, kCaller = 1, kNever = 2 };
+enum class DirectAccumulate { kAuto = 0, kCaller = 1 };
 xc_status direct_launch(xc_dtype dtype, const void* left, const void* right, void* out, const Geometry& g,
-                        const PairMap& pm, cudaStream_t stream, int force_loader /* -1 auto, 0 cp.async, 1 TMA */,
-                        DirectAccumulate acc = DirectAccumulate::kAuto, int tile = 0);
+                        const PairMap& pm, cudaStream_t stream, DirectAccumulate acc = DirectAccumulate::kAuto,
+                        int tile = 0);
 
 // The same by cyclic column classes (direct_cyclic.cu); `add`: into an output
 // the caller zeroed.  *taken is false, and nothing is launched, when the rows
