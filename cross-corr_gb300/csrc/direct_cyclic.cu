@@ -550,10 +550,11 @@ xc_status cyc_launch(const T* left, const T* right, T* out, Geometry g, const Pa
   // zeros.  There the wraps cost less once the lanes (a left row's classes, over
   // all pairs) fill the GPU: 1000x1 by 1x8 x 64 50.4 us, 6.6 in its place; 300x4 by
   // 2x40 x 64 21.3 and 16.9; 238x160 by 1x227, 105 pairs, 352 and 152; but one
-  // pair of 300x1 by 1x40 5.2 and 8.2, 20x60 by 1x300 x 64 17.8 and 24.9.
+  // pair of 300x1 by 1x40 5.2 and 8.2, of 300x2 by 1x8 4.8 and 5.2, 20x60 by 1x300
+  // x 64 17.8 and 24.9.
   const int C = div_up(g.Wl, TSX);
   const long long lanes = (long long)pm.n_left * pm.K * g.Hl * C;
-  const bool columns = g.Hl > g.Hr && ((g.Hr == 1 && C == 1 && g.Wr <= 8) ||
+  const bool columns = g.Hl > g.Hr && ((g.Hr == 1 && C == 1 && g.Wr <= 8 && (g.Hl < 64 || lanes >= 2000)) ||
                                        (g.Hr <= 3 && g.Hl >= 64 && lanes >= (g.Hr == 1 && C == 1 ? 9000 : 16000)));
   const bool flip = g.Wl < g.Wr && !columns;
   if (flip) {
